@@ -30,8 +30,9 @@ using staged::RepLuts2;
 using staged::build_luts2;
 using staged::Super;
 using lanes::LaneAt;
-using lanes::iq1m_block_sums;
+using lanes::iq1_block_sums;
 using lanes::iq3_block_sums;
+using lanes::kTernary;
 using lanes::sub_codes;
 
 constexpr int kWarps = 16, kThreads = kWarps * kWarp;
@@ -39,6 +40,9 @@ constexpr int kMaxSlots = 4;
 constexpr uint32_t kTaskRows = 32;  // rows a fused task has at most, a lane each (its tokens' loads are shared by them)
 constexpr uint32_t kMaxEntries = 1024;  // entries a launch takes (their pointers and live list sit in shared memory)
 constexpr uint32_t kSmemLimit = 226u * 1024u;
+
+// the codebooks' bytes, from the start of dynamic shared memory
+template <uint32_t T> constexpr uint32_t kLutBytes = kTernary<T> ? lanes::kTernaryBytes : ((uint32_t) Rep<T>::bytes + 127u) & ~127u;
 
 __device__ uint32_t g_status;
 
@@ -81,7 +85,9 @@ __global__ void __launch_bounds__(kThreads, 1) lane_ring_kernel(const Args a) {
     for (uint32_t s = 0; s < S; s++) bar_init(&full[warp][s], 1);
     bar_init_fence();
   }
-  const RepLuts2<T> luts = build_luts2<T>(smem, kThreads);
+  RepLuts2<T> luts{};
+  if constexpr (kTernary<T>) lanes::build_ternary(smem, kThreads);  // (complete at the list's first barrier below)
+  else luts = build_luts2<T>(smem, kThreads);
   // (a dependent launch: the tables and activations read from here on may be the output of the kernels ahead; the
   // codebooks above are not)
   pdl_wait();
@@ -167,29 +173,31 @@ __global__ void __launch_bounds__(kThreads, 1) lane_ring_kernel(const Args a) {
   if (lane == 0)
     for (uint32_t q = 0; q < S; q++) issue(q);
 
-  // the lane's blocks: block sub + L k is sub-block jj[k] of the superblock sboff[k] bytes into a row
-  uint32_t sboff[NB];
-#pragma unroll
-  for (int k = 0; k < NB; k++) sboff[k] = ((sub + (uint32_t) L * k) >> 3) * SB;
+  // the lane's blocks: block sub + L k is sub-block sub % 8 of the superblock sb0 + k kSbStep bytes into a row
+  const uint32_t sb0 = (sub >> 3) * SB;
+  constexpr uint32_t kSbStep = (L / 8) * SB;
   // (a row is a multiple of 4 bytes and the lane's superblocks lie an even count apart: one alignment for all)
   const uint32_t par = (SB % 4) ? ((sub >> 3) & 1u) * 2u : 0u;
   const LaneAt at{sub & 7u, 8u * (sub & 7u) + par, 16u - 8u * par};
 
   // one row's chain: the lane's blocks in order
-  auto row_chain = [&](auto live_tag, uint32_t ra, const int (&xq)[NT][NB][8], const float (&xd)[NT][NB], float* acc) {
+  constexpr int kXC = kTernary<T> ? NB : 1;
+  auto row_chain = [&](auto live_tag, uint32_t ra, const int (&xq)[NT][NB][8], const float (&xd)[NT][NB], const int (&xc)[NT][kXC][2],
+                       float* acc) {
     constexpr int NTL = decltype(live_tag)::value;
+    ra += sb0;
 #pragma unroll
     for (int k = 0; k < NB; k++) {
       if (EXACT || (uint32_t) k < nbl) {
-        if constexpr (T == QTYPE_IQ3_XXS || T == QTYPE_IQ1_M) {
+        if constexpr (T == QTYPE_IQ3_XXS || kTernary<T>) {
           float bs[NTL];
-          if constexpr (T == QTYPE_IQ3_XXS) iq3_block_sums<NTL, NT, NB>(ra + sboff[k], at, luts, xq, k, bs);
-          else iq1m_block_sums<NTL, NT, NB>(ra + sboff[k], at, luts, xq, k, bs);
+          if constexpr (T == QTYPE_IQ3_XXS) iq3_block_sums<NTL, NT, NB>(ra + k * kSbStep, at, luts, xq, k, bs);
+          else iq1_block_sums<T, NTL, NT, NB>(ra + k * kSbStep, at, smem, lane % lanes::kTernaryCopies * 4u, xq, xc, k, bs);
 #pragma unroll
           for (int t = 0; t < NTL; t++) acc[t] = __fmaf_rn(xd[t][k], bs[t], acc[t]);
         } else {
           LaneCodes c;
-          sub_codes<T>(ra + sboff[k], at, c, luts);
+          sub_codes<T>(ra + k * kSbStep, at, c, luts);
 #pragma unroll
           for (int t = 0; t < NTL; t++) acc[t] = __fmaf_rn(xd[t][k], lane_block_sum<T>(c, xq[t][k]), acc[t]);
         }
@@ -206,15 +214,15 @@ __global__ void __launch_bounds__(kThreads, 1) lane_ring_kernel(const Args a) {
   // fused: a row's gate and up sums are kept by the lane whose index is the row's place in the task (hg, hu); the
   // task's rows get their activation together at its end, a lane a row
   auto do_slot = [&](auto live_tag, uint32_t sa, uint32_t row0, uint32_t place0, float* const (&orow)[NT],
-                     const int (&xq)[NT][NB][8], const float (&xd)[NT][NB], float* hg, float* hu) {
+                     const int (&xq)[NT][NB][8], const float (&xd)[NT][NB], const int (&xc)[NT][kXC][2], float* hg, float* hu) {
     constexpr int NTL = decltype(live_tag)::value;
-    const uint32_t half_bytes = RC * row_bytes;  // fused: the up rows follow the gate rows
+    [[maybe_unused]] const uint32_t half_bytes = RC * row_bytes;  // fused: the up rows follow the gate rows
     if constexpr (FUSED && L == 16) {
       for (uint32_t p = 0; p < RC; p++) {  // lanes 0 .. 15 the gate row, 16 .. 31 the up row
         float acc[NTL];
 #pragma unroll
         for (int t = 0; t < NTL; t++) acc[t] = 0.0f;
-        row_chain(live_tag, sa + grp * half_bytes + p * row_bytes, xq, xd, acc);
+        row_chain(live_tag, sa + grp * half_bytes + p * row_bytes, xq, xd, xc, acc);
 #pragma unroll
         for (int t = 0; t < NTL; t++) {
           const float v = tree(acc[t]);  // (lanes 0 .. 15: the gate row's sum, 16 .. 31: the up row's)
@@ -227,8 +235,8 @@ __global__ void __launch_bounds__(kThreads, 1) lane_ring_kernel(const Args a) {
         float ag[NTL], au[NTL];
 #pragma unroll
         for (int t = 0; t < NTL; t++) ag[t] = 0.0f, au[t] = 0.0f;
-        row_chain(live_tag, sa + p * row_bytes, xq, xd, ag);
-        row_chain(live_tag, sa + half_bytes + p * row_bytes, xq, xd, au);
+        row_chain(live_tag, sa + p * row_bytes, xq, xd, xc, ag);
+        row_chain(live_tag, sa + half_bytes + p * row_bytes, xq, xd, xc, au);
 #pragma unroll
         for (int t = 0; t < NTL; t++) {
           const float g = tree(ag[t]), u = tree(au[t]);
@@ -241,7 +249,7 @@ __global__ void __launch_bounds__(kThreads, 1) lane_ring_kernel(const Args a) {
         float acc[NTL];
 #pragma unroll
         for (int t = 0; t < NTL; t++) acc[t] = 0.0f;
-        row_chain(live_tag, sa + (p + grp) * row_bytes, xq, xd, acc);
+        row_chain(live_tag, sa + (p + grp) * row_bytes, xq, xd, xc, acc);
 #pragma unroll
         for (int t = 0; t < NTL; t++) {
           const float v = tree(acc[t]);
@@ -264,6 +272,7 @@ __global__ void __launch_bounds__(kThreads, 1) lane_ring_kernel(const Args a) {
     // the task's tokens: the lane's blocks of their int8 rows, their scales, the routed weights
     int xq[NT][NB][8];
     float xd[NT][NB], scale[NT];
+    int xc[NT][kXC][2];  // (IQ1: minus the chunks' sums)
     float* orow[NT];  // where each token's results go: looked up now, used when the task's rows are done
     const int8_t* const in_q = a.q + parity * a.ep.half_q;
     const float* const in_d = (const float*) ((const uint8_t*) a.d + parity * a.ep.half_d);
@@ -286,6 +295,7 @@ __global__ void __launch_bounds__(kThreads, 1) lane_ring_kernel(const Args a) {
         xq[t][k][0] = lo.x, xq[t][k][1] = lo.y, xq[t][k][2] = lo.z, xq[t][k][3] = lo.w;
         xq[t][k][4] = hi.x, xq[t][k][5] = hi.y, xq[t][k][6] = hi.z, xq[t][k][7] = hi.w;
         xd[t][k] = dv;
+        if constexpr (kTernary<T>) lanes::chunk_sums(xq[t][k], xc[t][k]);
       }
     }
     float hg[NT], hu[NT];
@@ -299,8 +309,8 @@ __global__ void __launch_bounds__(kThreads, 1) lane_ring_kernel(const Args a) {
         break;
       }
       const uint32_t sa = smem_addr(ring + slot * a.slot_bytes);
-      if (NT > 1 && live == (uint32_t) NT) do_slot(I2{}, sa, task_row0 + ss * RC, ss * RC, orow, xq, xd, hg, hu);
-      else do_slot(I1{}, sa, task_row0 + ss * RC, ss * RC, orow, xq, xd, hg, hu);
+      if (NT > 1 && live == (uint32_t) NT) do_slot(I2{}, sa, task_row0 + ss * RC, ss * RC, orow, xq, xd, xc, hg, hu);
+      else do_slot(I1{}, sa, task_row0 + ss * RC, ss * RC, orow, xq, xd, xc, hg, hu);
       __syncwarp();  // every lane is done reading the slot: refill it
       if (lane == 0) {
         fence_async_smem();
@@ -350,8 +360,8 @@ int launch(const Request& r, cudaStream_t s) {
   constexpr uint32_t M = FUSED ? 2 : 1, RU = FUSED ? 1 : kWarp / L;
   const uint32_t row_bytes = r.cols / 256 * Super<T>::bytes;
   Args a{};
-  a.list_off = (uint32_t) ((Rep<T>::bytes + 127) & ~127);
-  a.ptr_off = a.list_off + kMaxEntries * (8 / NT) * 2;
+  a.list_off = kLutBytes<T>;
+  a.ptr_off = (a.list_off + r.n_entries * ((r.max_cnt + NT - 1) / NT) * 2u + 7u) & ~7u;  // (an entry has at most max_cnt / NT groups)
   a.ring_off = (a.ptr_off + r.n_entries * (M * 8 + 8) + 127u) & ~127u;  // (pointers, then (count, first row))
   if (a.ring_off + 16u >= kSmemLimit) return 0;
   // a slot: the fewest rows (a multiple of the rows a pass takes) whose bytes are a multiple of 16 and reach about 3 KB
@@ -397,8 +407,13 @@ int by_shape(const Request& r, cudaStream_t s) {
   const uint32_t per = nblk / 32;
   if (per == 4) return launch<T, FUSED, 32, 4, 2, true>(r, s);
   if (per < 4) return launch<T, FUSED, 32, 4, 2, false>(r, s);
-  if (per <= 8) return launch<T, FUSED, 32, 8, 1, false>(r, s);
-  return 0;
+  switch (per) {  // (exact: no test a block, the blocks' loads scheduled together)
+    case 5: return launch<T, FUSED, 32, 5, 1, true>(r, s);
+    case 6: return launch<T, FUSED, 32, 6, 1, true>(r, s);
+    case 7: return launch<T, FUSED, 32, 7, 1, true>(r, s);
+    case 8: return launch<T, FUSED, 32, 8, 1, true>(r, s);
+    default: return 0;
+  }
 }
 
 }  // namespace

@@ -123,6 +123,40 @@ def test_group_tok_and_gate_up(lib, dev, oracle, name, cols):
     assert same_bits(y1.cpu().numpy()[10, :rows], want_g[10, :rows])
 
 
+@pytest.mark.parametrize("name", ["IQ1_S", "IQ1_M", "IQ2_XXS", "IQ3_XXS"])
+@pytest.mark.parametrize("cols", [512, 1024, 2048, 3072, 4096, 5120, 6144, 7168, 8192])
+def test_lane_ring_row_widths(lib, dev, oracle, name, cols):
+    """the warp-ring kernel's row widths: every number of blocks a lane holds, one token and two a decode, activations
+    at the codes' limits (all 127, alternating +-127) among them"""
+    tid = TYPES[name]
+    rows, n_mat = 64, 3
+    rng = synth.rng_for(29, tid, cols)
+    gate = [synth.random_tensor(tid, rows, cols, rng) for _ in range(n_mat)]
+    up = [synth.random_tensor(tid, rows, cols, rng) for _ in range(n_mat)]
+    cnt, xrow, total = [3, 0, 2], [0, 3, 3], 5
+    x = rng.standard_normal((total, cols)).astype(np.float32)
+    x[1], x[3] = 2.5, np.where(np.arange(cols) % 2, -1.0, 1.0)
+    scale = rng.uniform(0.05, 0.5, size=total).astype(np.float32)
+    wq, wd = oracle.q8_round(x)
+    q, d, sd = to_dev(wq, dev), to_dev(wd, dev), to_dev(scale, dev)
+    _p, tg, cd, xd_ = _tables(dev, gate, cnt, xrow)
+    _u, tu, _, _ = _tables(dev, up, cnt, xrow)
+    y = torch.full((total, rows), -9.0, dtype=torch.float32, device=dev)
+    h = torch.full((total, rows), -9.0, dtype=torch.float32, device=dev)
+    lib.q8_status()
+    assert lib.q8_group_tok(tid, ptr(tu), ptr(cd), ptr(xd_), None, n_mat, 8, rows, cols, ptr(q), ptr(d), ptr(y), rows, None)
+    assert lib.q8_gate_up(tid, ptr(tg), ptr(tu), ptr(cd), ptr(xd_), None, None, n_mat, 8, rows, cols, ptr(q), ptr(d), ptr(sd), 1.5,
+                          ptr(h), rows, None)
+    sync()
+    for m in range(n_mat):
+        r = slice(xrow[m], xrow[m] + cnt[m])
+        if cnt[m]:
+            g, u = (oracle.q8_rows(tid, w[m], rows, cols, wq[r], wd[r]) for w in (gate, up))
+            assert same_bits(y.cpu().numpy()[r], u)
+            assert same_bits(h.cpu().numpy()[r], oracle.swiglu_lane(g, u, 1.5, scale[r]))
+    assert lib.q8_status() == 0
+
+
 @pytest.mark.parametrize("name", ["Q4_0", "Q8_0"])
 @pytest.mark.parametrize("cols", [2048, 4096])
 def test_q8_run_plain_blocks(lib, dev, oracle, name, cols):
