@@ -4,6 +4,7 @@
 // loads, so x traffic from L1 is 1 / kRows of the naive count.
 #include "decode.cuh"
 #include "dispatch.cuh"
+#include "mv_pair_api.h"
 #include "mv_staged_api.h"
 #include "osmos_b200/mv.h"
 
@@ -126,6 +127,7 @@ bool strided(const void* w, uint32_t rows, uint32_t cols, const float* x, uint32
   if ((n_tok > 1 && (xs < cols || ys < rows)) || xs % kChunk) return false;
   if (g_use_staged && n_tok <= MV_MAX_TOKENS) {  // the staged kernel when it takes the shape: the same bits
     const mvs::Request r{w, x, y, rows, cols, xs, ys, n_tok};
+    if (const int st = mvp::try_launch(T, r, s)) return st > 0;
     if (const int st = mvs::try_launch(T, r, s)) return st > 0;
     // long rows: as many tokens a pass as the staged kernel holds x for (a token's sums do not depend on its batch),
     // a pass it still does not take on the generic kernel
@@ -158,6 +160,7 @@ bool group(const void* const* w, uint32_t n, uint32_t rows, uint32_t cols, const
   if (g_use_staged) {  // the staged kernel when it takes the shape: the same bits
     mvs::Request r{nullptr, x, y, rows, cols, cols, rows, 1};
     r.wt = w, r.n_entries = n, r.x_mat = x_mat, r.x_div = x_div;
+    if (const int st = mvp::try_launch(T, r, s)) return st > 0;
     if (const int st = mvs::try_launch(T, r, s)) return st > 0;
   }
   MvArgs a{};
@@ -173,6 +176,7 @@ bool group_tok(const void* const* w, const int32_t* cnt, const int32_t* xrow, ui
   if (g_use_staged) {  // the staged kernel when it takes the shape: the same bits
     mvs::Request r{nullptr, x, y, rows, cols, xs, ys, max_cnt};
     r.wt = w, r.n_entries = n, r.cnt = cnt, r.xrow = xrow;
+    if (const int st = mvp::try_launch(T, r, s)) return st > 0;
     if (const int st = mvs::try_launch(T, r, s)) return st > 0;
   }
   MvArgs a{};
@@ -195,7 +199,7 @@ extern "C" bool mv_strided(uint32_t type, const void* w, uint32_t rows, uint32_t
 }
 
 extern "C" void mv_set_staged(int on) { g_use_staged = on != 0; }
-extern "C" uint32_t mv_status(void) { return mvs::read_status(); }
+extern "C" uint32_t mv_status(void) { return mvs::read_status() | mvp::read_status(); }
 
 extern "C" bool mv_run(uint32_t type, const void* w, uint32_t rows, uint32_t cols, const float* x, uint32_t n_tok,
                        float* y, void* stream) {

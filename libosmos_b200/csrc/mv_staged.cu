@@ -8,6 +8,9 @@
 // block holds 16 x (slots - 1) copies in flight. Plain 32-value blocks are decoded with one byte-permute and one fmaf a
 // value (see scaled4); the other types go through the same decode8 as the generic kernel.
 //
+// (mv_pair.cu serves Q4_K, Q5_K and Q6_K, the grouped forms of Q4_0, Q8_0, IQ4_XS and MXFP4, and most of their dense ones:
+// its by_shape has the rule.)
+//
 // Two kernels. One token and rows of at most 2048 values (the decode step's usual shape): every lane keeps its 64
 // values of x in registers for the whole launch, so shared memory serves only the weights (mv_regx_kernel). Else x
 // lies in shared memory and is read a chunk at a time (mv_staged_kernel; up to eight tokens, each its own chain of
@@ -148,35 +151,6 @@ template <> struct LanePlan<QTYPE_Q8_0> {
     const uint32_t r0 = lds32(base + al), r1 = lds32(base + al + 4), r2 = lds32(base + al + 8);
     d = half_value(lds16(base + doff)), neg = mul_rn(d, -32896.0f);
     m[0] = __funnelshift_r(r0, r1, sh) ^ 0x80808080u, m[1] = __funnelshift_r(r1, r2, sh) ^ 0x80808080u;
-  }
-};
-
-template <> struct LanePlan<QTYPE_Q4_K> {
-  // lane l's chunk of a 144-byte block: group l / 4 (its 6-bit scale and min among the 12 packed bytes), values
-  // 8 (l % 4) .. of the group - the low (even group) or high nibbles of 8 bytes; everything but the bytes themselves
-  // is worked out once. A row starts on 16 bytes and a block is 144 long, so every read is aligned.
-  static constexpr uint32_t kStretch = 144;
-  uint32_t qoff, s4, b8, upper;
-  __device__ __forceinline__ explicit LanePlan(uint32_t l) {
-    const uint32_t grp = l >> 2;
-    qoff = 16u + (grp >> 1) * 32u + (l & 3u) * 8u, s4 = 4u * (grp & 1u), b8 = 8u * (grp & 3u), upper = grp >> 2;
-  }
-  __device__ __forceinline__ void values(uint32_t row, const uint8_t*, uint32_t it, float* v, const Grids&) const {
-    const uint32_t base = row + it * kStretch;
-    const uint32_t hd = lds32(base);
-    const uint32_t a0 = (lds32(base + 4) >> b8) & 0xFFu, a1 = (lds32(base + 8) >> b8) & 0xFFu, a2 = (lds32(base + 12) >> b8) & 0xFFu;
-    const uint32_t sc = upper ? (a2 & 0x0Fu) | ((a0 >> 6) << 4) : a0 & 63u;
-    const uint32_t mn = upper ? (a2 >> 4) | ((a1 >> 6) << 4) : a1 & 63u;
-    // d sc has at most 17 significant bits and a code 4: the product is exact, so one fmaf against the biased code
-    // gives the bits of mul_rn(d sc, n); then the min is taken off, rounded once - decode8's value
-    const float ds = mul_rn(half_value(hd & 0xFFFFu), (float) sc), dm = mul_rn(half_value(hd >> 16), (float) mn);
-    const float c = mul_rn(ds, -32768.0f);
-    const uint2 q = lds64(base + qoff);
-    const uint32_t m0 = (q.x >> s4) & 0x0F0F0F0Fu, m1 = (q.y >> s4) & 0x0F0F0F0Fu;
-    v[0] = __fsub_rn(__fmaf_rn(ds, biased<0>(m0), c), dm), v[1] = __fsub_rn(__fmaf_rn(ds, biased<1>(m0), c), dm);
-    v[2] = __fsub_rn(__fmaf_rn(ds, biased<2>(m0), c), dm), v[3] = __fsub_rn(__fmaf_rn(ds, biased<3>(m0), c), dm);
-    v[4] = __fsub_rn(__fmaf_rn(ds, biased<0>(m1), c), dm), v[5] = __fsub_rn(__fmaf_rn(ds, biased<1>(m1), c), dm);
-    v[6] = __fsub_rn(__fmaf_rn(ds, biased<2>(m1), c), dm), v[7] = __fsub_rn(__fmaf_rn(ds, biased<3>(m1), c), dm);
   }
 };
 
@@ -498,6 +472,10 @@ uint32_t slots_for(uint32_t rw, uint32_t x_tokens, uint32_t cols) {
   return n > (uint32_t) kMaxSlots ? (uint32_t) kMaxSlots : n;
 }
 
+// what mv_pair.cu takes: every shape of the first three types, the grouped forms of all seven
+template <uint32_t T> constexpr bool kPaired = (T == QTYPE_Q4_K || T == QTYPE_Q5_K || T == QTYPE_Q6_K);
+template <uint32_t T> constexpr bool kPairedGroups = kPaired<T> || T == QTYPE_Q4_0 || T == QTYPE_Q8_0 || T == QTYPE_IQ4_XS || T == QTYPE_MXFP4;
+
 template <uint32_t T>
 int by_shape(const Request& r, cudaStream_t s) {
   const Device* dev = device_info();
@@ -550,13 +528,17 @@ int try_launch(uint32_t type, const Request& r, void* stream) {
   if (!r.rows || !r.n_tok || r.n_tok > 8 || r.cols % 8) return 0;
   if (r.wt) {  // grouped: every entry's x row starts on 16 bytes when the first does and the strides are whole words of 16
     if (((uintptr_t) r.x & 15u) || r.xs % 4 || r.x_mat % 4) return 0;
-#define CASE(T) return grouped<T>(r, (cudaStream_t) stream);
+#define CASE(T)                                                            \
+  if constexpr (!kPairedGroups<T>) return grouped<T>(r, (cudaStream_t) stream); \
+  else return 0;
     OSMOS_SWITCH_QUANT(type, CASE, return 0)
 #undef CASE
   }
   if (((uintptr_t) r.w | (uintptr_t) r.x) & 15u) return 0;
   if (r.n_tok > 1 && r.xs % 4) return 0;
-#define CASE(T) return by_shape<T>(r, (cudaStream_t) stream);
+#define CASE(T)                                                       \
+  if constexpr (!kPaired<T>) return by_shape<T>(r, (cudaStream_t) stream); \
+  else return 0;
   OSMOS_SWITCH_QUANT(type, CASE, return 0)
 #undef CASE
 }
@@ -565,7 +547,7 @@ uint32_t max_tokens(uint32_t type, uint32_t cols) {
   if (!cols || cols % 256) return 0;
 #define CASE(T)                                                                          \
   {                                                                                      \
-    if ((cols / Fmt<T>::values * Fmt<T>::bytes) % 16u) return 0;                          \
+    if (kPaired<T> || (cols / Fmt<T>::values * Fmt<T>::bytes) % 16u) return 0;            \
     uint32_t n = 8;                                                                      \
     while (n && slots_for<T>(1, n, cols) < 2) n--;                                       \
     return n;                                                                            \

@@ -118,6 +118,67 @@ def test_mv_staged_row_pairs(lib, dev, oracle, name):
     assert lib.mv_status() == 0
 
 
+PAIRED = ["Q4_0", "Q8_0", "Q4_K", "Q5_K", "Q6_K", "IQ4_XS", "MXFP4"]  # (the types of the kernel that runs two lanes a thread)
+
+
+@pytest.mark.parametrize("name", PAIRED)
+@pytest.mark.parametrize("cols,rows", [(256, 1), (256, 7), (768, 66), (2048, 35), (2304, 5), (4352, 33), (9472, 6), (768, 8 * 16 * 160 + 5)])
+def test_mv_paired_lanes(lib, dev, oracle, name, cols, rows):
+    """rows that start anywhere in a 16-byte piece (the matrix's last bytes among them), one and several segments of a row,
+    tokens in one pass and in two, one and two rows a thread; every token count, strided x and y"""
+    tid = TYPES[name]
+    xs, ys = cols + 8, (rows + 7) // 8 * 8 + 8
+    rng = synth.rng_for(15, tid, rows, cols)
+    w = synth.random_tensor(tid, rows, cols, rng)
+    x = rng.standard_normal((8, xs)).astype(np.float32)
+    want = oracle.mv_rows(tid, w, rows, cols, np.ascontiguousarray(x[:, :cols]))
+    wd, xd = to_dev(w, dev), to_dev(x, dev)
+    lib.mv_status()
+    for n in range(1, 9):
+        y = torch.full((8, ys), -3.0, dtype=torch.float32, device=dev)
+        assert lib.mv_strided(tid, ptr(wd), rows, cols, ptr(xd), xs, n, ptr(y), ys, None)
+        sync()
+        got = y.cpu().numpy()
+        assert same_bits(got[:n, :rows], want[:n]) and (got[:n, rows:] == -3.0).all() and (got[n:] == -3.0).all()
+    assert lib.mv_status() == 0
+
+
+@pytest.mark.parametrize("name", PAIRED)
+@pytest.mark.parametrize("cols,rows", [(768, 37), (2560, 130)])
+def test_mv_paired_lanes_grouped(lib, dev, oracle, name, cols, rows):
+    """an entry's matrix, count and rows out of the tables: every count, one past max_cnt, none; and one row a matrix"""
+    tid = TYPES[name]
+    cnt = [8, 0, 1, 3, 9, 5, 2, 7, 4, 6]
+    rng = synth.rng_for(16, tid, rows, cols)
+    mats = [synth.random_tensor(tid, rows, cols, rng) for _ in cnt]
+    step = (mats[0].size + 15) // 16 * 16
+    pool = np.zeros(step * len(cnt), np.uint8)
+    for m, w in enumerate(mats):
+        pool[m * step:m * step + w.size] = w.reshape(-1)
+    total = sum(cnt)
+    xrow = np.cumsum([0] + cnt[:-1]).astype(np.int32)
+    x = rng.standard_normal((total, cols)).astype(np.float32)
+    pd, xd = to_dev(pool, dev), to_dev(x, dev)
+    table = pointer_table(pd, [m * step for m in range(len(cnt))], dev)
+    cd, rd = to_dev(np.array(cnt, np.int32), dev), to_dev(xrow, dev)
+    lib.mv_status()
+    for max_cnt in (8, 3, 1):
+        y = torch.full((total, rows), -3.0, dtype=torch.float32, device=dev)
+        assert lib.mv_group_tok(tid, ptr(table), ptr(cd), ptr(rd), len(cnt), max_cnt, rows, cols, ptr(xd), cols, ptr(y), rows, None)
+        sync()
+        got, want = y.cpu().numpy(), np.full((total, rows), -3.0, np.float32)
+        for m, c in enumerate(cnt):
+            r = slice(int(xrow[m]), int(xrow[m]) + min(c, max_cnt))
+            if c:
+                want[r] = oracle.mv_rows(tid, mats[m], rows, cols, x[r])
+        assert same_bits(got, want)
+    y = torch.full((len(cnt), rows), -3.0, dtype=torch.float32, device=dev)
+    assert lib.mv_group(tid, ptr(table), len(cnt), rows, cols, ptr(xd), cols, 2, ptr(y), None)
+    sync()
+    assert same_bits(y.cpu().numpy(), np.concatenate([oracle.mv_rows(tid, w, rows, cols, x[m // 2:m // 2 + 1]) for m, w in enumerate(mats)]))
+    assert lib.mv_status() == 0
+
+
 @pytest.mark.parametrize("name", ["Q4_0", "IQ3_XXS", "Q4_K", "MXFP4"])
 def test_mv_strided_many_tokens(lib, dev, oracle, name):
     tid = TYPES[name]
