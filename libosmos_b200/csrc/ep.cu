@@ -188,9 +188,11 @@ struct StepArgs {
   float rscale;
 };
 
-// A block a home token. Its last warp routes it (route.cuh) while the eight before it round its row to int8
-// (q8_round.cuh); every result goes straight to its token-major place in every rank's buffer. The last block to finish
-// releases this rank's dispatch flag everywhere and advances the step counter.
+// A block a home token and 2048 values of its row (blockIdx.y: a thread eight values, so a long row's loads all leave at
+// once - one block a token took a trip to memory every 2048 values). The first block's last warp routes the token
+// (route.cuh) while eight warps round the values to int8 (q8_round.cuh); every result goes straight to its token-major
+// place in every rank's buffer. The last block to finish releases this rank's dispatch flag everywhere and advances the
+// step counter.
 constexpr int kRoundWarps = 8, kStepThreads = (kRoundWarps + 1) * kWarp;
 template <int R, int ROUTER>
 __global__ void __launch_bounds__(kStepThreads) route_round_push_kernel(const StepArgs a, const float* __restrict__ x,
@@ -200,36 +202,37 @@ __global__ void __launch_bounds__(kStepThreads) route_round_push_kernel(const St
   const uint32_t step = a.sync[0] + 1u, half = step & 1u;
   const uint32_t tl = blockIdx.x, t = a.rank * a.tokens + tl, lane = threadIdx.x % kWarp;
   if (threadIdx.x >= kRoundWarps * kWarp) {
-    route::Pick p;
-    if constexpr (ROUTER == EP_ROUTER_SOFTMAX) p = route::softmax_topk<R>(logits + (uint64_t) tl * a.n_exp, a.n_exp, a.k, lane);
-    else if constexpr (ROUTER == EP_ROUTER_SIGMOID)
-      p = route::scored_topk<R, route::kSigmoid>(logits + (uint64_t) tl * a.n_exp, a.bias, a.n_exp, a.k, a.rscale, lane);
-    else p = route::scored_topk<R, route::kSqrtSoftplus>(logits + (uint64_t) tl * a.n_exp, a.bias, a.n_exp, a.k, a.rscale, lane);
-    if (lane < a.k)
-      for (uint32_t r = 0; r < a.n_ranks; r++) {
-        ((int32_t*) (a.peers.base[r] + a.lay.ids[half]))[t * a.k + lane] = (int32_t) p.id;
-        ((float*) (a.peers.base[r] + a.lay.weights[half]))[t * a.k + lane] = p.w;
-      }
+    if (blockIdx.y == 0) {
+      route::Pick p;
+      if constexpr (ROUTER == EP_ROUTER_SOFTMAX) p = route::softmax_topk<R>(logits + (uint64_t) tl * a.n_exp, a.n_exp, a.k, lane);
+      else if constexpr (ROUTER == EP_ROUTER_SIGMOID)
+        p = route::scored_topk<R, route::kSigmoid>(logits + (uint64_t) tl * a.n_exp, a.bias, a.n_exp, a.k, a.rscale, lane);
+      else p = route::scored_topk<R, route::kSqrtSoftplus>(logits + (uint64_t) tl * a.n_exp, a.bias, a.n_exp, a.k, a.rscale, lane);
+      if (lane < a.k)
+        for (uint32_t r = 0; r < a.n_ranks; r++) {
+          ((int32_t*) (a.peers.base[r] + a.lay.ids[half]))[t * a.k + lane] = (int32_t) p.id;
+          ((float*) (a.peers.base[r] + a.lay.weights[half]))[t * a.k + lane] = p.w;
+        }
+    }
   } else {
-    const uint32_t per = a.dim / 8;
-    for (uint32_t c0 = 0; c0 < per; c0 += kRoundWarps * kWarp) {  // (whole warps: per is a multiple of 4)
-      const uint32_t c = c0 + threadIdx.x;
-      const bool live = c < per;
-      float v[8], scale;
-      load8(x + (uint64_t) tl * a.dim + (uint64_t) (live ? c : 0) * 8, v);
-      const uint2 codes = round_block8<false>(v, &scale);
-      if (!live) continue;
+    const uint32_t per = a.dim / 8, c = blockIdx.y * (kRoundWarps * kWarp) + threadIdx.x;
+    const bool live = c < per;  // (a 32-value block's four lanes alike: per is a multiple of 4)
+    float v[8], scale;
+    load8(x + (uint64_t) tl * a.dim + (uint64_t) (live ? c : 0) * 8, v);
+    const uint2 codes = round_block8<false>(v, &scale);
+    if (live)
       for (uint32_t r = 0; r < a.n_ranks; r++) {
         *(uint2*) (a.peers.base[r] + a.lay.q[half] + (uint64_t) t * a.dim + (uint64_t) c * 8) = codes;
         if (c % 4 == 0) ((float*) (a.peers.base[r] + a.lay.d[half]))[(uint64_t) t * (a.dim / 32) + c / 4] = scale;
       }
-    }
   }
   publish_step(a.peers, a.lay.flags_dispatch, a.rank, a.n_ranks, step, a.sync + 1, a.sync);
 }
 
-// A block a home token: a bounded wait on every rank's combine flag, the token's picks ordered by expert id (k is
-// small: one thread sorts by insertion), then every thread its columns, the rows added in that order from 0.
+// A block a home token and 1024 of its columns (blockIdx.y; a thread four): a bounded wait on every rank's combine flag,
+// the token's picks ordered by expert id, then the rows added in that order from 0, eight rows' loads in flight at a
+// time. (With one block a token a 7168-column row was seven rounds of k dependent trips to L2: one token 21 us alone.)
+constexpr uint32_t kCombineRows = 8;
 __global__ void __launch_bounds__(kThreads) combine_wait_kernel(const StepArgs a, const float* __restrict__ add,
                                                                 float* __restrict__ out) {
   __shared__ uint32_t order[32];
@@ -249,18 +252,23 @@ __global__ void __launch_bounds__(kThreads) combine_wait_kernel(const StepArgs a
   }
   __syncthreads();
   const float4* recv = (const float4*) (mine + a.lay.recv[half]) + (uint64_t) tl * k * (a.dim / 4);
-  for (uint32_t c = threadIdx.x; c < a.dim / 4; c += kThreads) {
-    float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    for (uint32_t j = 0; j < k; j++) {
-      const float4 v = recv[(uint64_t) order[j] * (a.dim / 4) + c];
-      s.x = __fadd_rn(s.x, v.x), s.y = __fadd_rn(s.y, v.y), s.z = __fadd_rn(s.z, v.z), s.w = __fadd_rn(s.w, v.w);
-    }
-    if (add) {
-      const float4 v = ((const float4*) add)[(uint64_t) tl * (a.dim / 4) + c];
-      s.x = __fadd_rn(s.x, v.x), s.y = __fadd_rn(s.y, v.y), s.z = __fadd_rn(s.z, v.z), s.w = __fadd_rn(s.w, v.w);
-    }
-    ((float4*) out)[(uint64_t) tl * (a.dim / 4) + c] = s;
+  const uint32_t c = blockIdx.y * kThreads + threadIdx.x;
+  if (c >= a.dim / 4) return;
+  float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f), last = s;
+  if (add) last = ((const float4*) add)[(uint64_t) tl * (a.dim / 4) + c];
+  for (uint32_t j0 = 0; j0 < k; j0 += kCombineRows) {
+    float4 v[kCombineRows];
+#pragma unroll
+    for (uint32_t j = 0; j < kCombineRows; j++)
+      if (j0 + j < k) v[j] = recv[(uint64_t) order[j0 + j] * (a.dim / 4) + c];
+#pragma unroll
+    for (uint32_t j = 0; j < kCombineRows; j++)
+      if (j0 + j < k)
+        s.x = __fadd_rn(s.x, v[j].x), s.y = __fadd_rn(s.y, v[j].y), s.z = __fadd_rn(s.z, v[j].z), s.w = __fadd_rn(s.w, v[j].w);
   }
+  if (add)
+    s.x = __fadd_rn(s.x, last.x), s.y = __fadd_rn(s.y, last.y), s.z = __fadd_rn(s.z, last.z), s.w = __fadd_rn(s.w, last.w);
+  ((float4*) out)[(uint64_t) tl * (a.dim / 4) + c] = s;
 }
 
 StepArgs step_args(const EpPlan* p) {
@@ -330,7 +338,7 @@ extern "C" bool ep_plan_ok(const EpPlan* p) {
 extern "C" bool ep_route_round_push(const EpPlan* p, const float* x, const float* logits, void* stream) {
   if (!p || !x || !logits) return false;
   const StepArgs a = step_args(p);
-  const dim3 grid(a.tokens), block(kStepThreads);
+  const dim3 grid(a.tokens, blocks_for(a.dim / 8, kRoundWarps * kWarp)), block(kStepThreads);
   const cudaStream_t s = stream_of(stream);
 #define ROUTE(R, KIND) launch_dependent(route_round_push_kernel<R, KIND>, grid, block, 0, s, a, x, logits) == cudaSuccess
 #define BY_REGS(KIND)                     \
@@ -388,7 +396,7 @@ extern "C" bool ep_down_push(const EpPlan* p, void* stream) {
 extern "C" bool ep_combine_wait(const EpPlan* p, const float* add, float* out, void* stream) {
   if (!p || !out || (((uintptr_t) out | (uintptr_t) add) & 15u)) return false;
   const StepArgs a = step_args(p);
-  return launch_dependent(combine_wait_kernel, dim3(a.tokens), dim3(kThreads), 0, stream_of(stream), a, add, out) == cudaSuccess;
+  return launch_dependent(combine_wait_kernel, dim3(a.tokens, blocks_for(a.dim / 4, kThreads)), dim3(kThreads), 0, stream_of(stream), a, add, out) == cudaSuccess;
 }
 
 extern "C" bool ep_last_picks(const EpPlan* p, int32_t* ids, float* weights) {
