@@ -37,6 +37,7 @@
 #include "fp4_tc_api.h"
 #include "mm_tc_api.h"
 #include "osmos_b200/mm.h"
+#include "packed.cuh"
 #include "tma.cuh"
 
 namespace osmos {
@@ -108,51 +109,143 @@ __device__ __forceinline__ uint32_t half2_bits(float lo, float hi) {
 template <uint32_t T> constexpr uint32_t kRawK = (T == QTYPE_Q8_0) ? 128u : 256u;
 template <uint32_t T> constexpr uint32_t kRawBytes = kRawK<T> / Fmt<T>::values * Fmt<T>::bytes;
 template <uint32_t T> constexpr uint32_t kRawSlot = ((kRawBytes<T> + 30u + 15u) & ~15u) | 16u;
-template <uint32_t T> constexpr bool kFastChunk = (T == QTYPE_Q4_K || T == QTYPE_Q4_0 || T == QTYPE_Q8_0);
+template <uint32_t T> constexpr bool kFastChunk = (T == QTYPE_Q8_0 || T == QTYPE_Q6_K);
+
+// the eight bytes at shared address `at` (any alignment) out of the three aligned words around them (the third may lie
+// past the last byte asked for: a row's slot in the raw buffer has the room)
+__device__ __forceinline__ uint2 lds_8_bytes(uint32_t at) {
+  const uint32_t al = at & ~3u, sh = (at & 3u) * 8u;
+  const uint32_t r0 = lds32(al), r1 = lds32(al + 4), r2 = lds32(al + 8);
+  return make_uint2(__funnelshift_r(r0, r1, sh), __funnelshift_r(r1, r2, sh));
+}
+// byte J of `bytes` - 0x80 + 2 n with n < 64 - as the F32 64 + n: bits 16 .. 23 of 0x42000000
+template <int J> __device__ __forceinline__ float biased64(uint32_t bytes) {
+  return __uint_as_float(__byte_perm(bytes, 0x42000000u, 0x7044 | (J << 8)));
+}
 
 template <uint32_t T>
 __device__ __forceinline__ uint4 fast_chunk(const uint8_t* blk, uint32_t k) {
   uint4 out;
-  if constexpr (T == QTYPE_Q4_K) {
-    // chunk k of the 256-value block: group k / 4 (its 6-bit scale and min out of the 12 packed bytes), values
-    // 8 (k % 4) .. of the group: the low (even group) or high nibbles of 8 bytes
-    const uint32_t* wp = (const uint32_t*) blk;
-    const uint32_t grp = k >> 2, b8 = 8u * (grp & 3u);
-    const uint32_t hd = wp[0], a0 = (wp[1] >> b8) & 0xFFu, a1 = (wp[2] >> b8) & 0xFFu, a2 = (wp[3] >> b8) & 0xFFu;
-    const uint32_t sc = grp < 4 ? a0 & 63u : (a2 & 0x0Fu) | ((a0 >> 6) << 4);
-    const uint32_t mn = grp < 4 ? a1 & 63u : (a2 >> 4) | ((a1 >> 6) << 4);
-    const float ds = mul_rn(half_value(hd & 0xFFFFu), (float) sc), dm = mul_rn(half_value(hd >> 16), (float) mn);
-    const float c = mul_rn(ds, -32768.0f);
-    const uint32_t* q = wp + 4 + (grp >> 1) * 8 + (k & 3u) * 2;
-    const uint32_t s4 = 4u * (grp & 1u), m0 = (q[0] >> s4) & 0x0F0F0F0Fu, m1 = (q[1] >> s4) & 0x0F0F0F0Fu;
-    out.x = half2_bits(__fsub_rn(__fmaf_rn(ds, biased<0>(m0), c), dm), __fsub_rn(__fmaf_rn(ds, biased<1>(m0), c), dm));
-    out.y = half2_bits(__fsub_rn(__fmaf_rn(ds, biased<2>(m0), c), dm), __fsub_rn(__fmaf_rn(ds, biased<3>(m0), c), dm));
-    out.z = half2_bits(__fsub_rn(__fmaf_rn(ds, biased<0>(m1), c), dm), __fsub_rn(__fmaf_rn(ds, biased<1>(m1), c), dm));
-    out.w = half2_bits(__fsub_rn(__fmaf_rn(ds, biased<2>(m1), c), dm), __fsub_rn(__fmaf_rn(ds, biased<3>(m1), c), dm));
-  } else {
-    // a 32-value block with one f16 scale (2-byte aligned: read by halves): chunk k's 8 codes
+  if constexpr (T == QTYPE_Q6_K) {
+    // chunk k: sub-block j = k / 4; a half of the block has 64 bytes of low nibbles and 32 of top bit pairs
+    const uint32_t at = smem_addr(blk), j = k >> 2, kk = k & 3u, h = j >> 2, r = j & 3u;
+    const uint2 q = lds_8_bytes(at + 64u * h + 32u * (r & 1u) + 8u * kk), t = lds_8_bytes(at + 128u + 32u * h + 8u * kk);
+    const int sc = (int) (int8_t) lds8(at + 192u + 2u * j + (kk >> 1));
+    const float ds = mul_rn(half_value(lds16(at + 208u)), (float) sc);
+    const uint32_t s4 = 4u * (r >> 1), s2 = 2u * r;
+    // 64 + n made by a byte permute, less 96: the code n - 32, exactly; times d s, rounded once, as decode8's
+    const uint32_t u0 = kTops | ((q.x >> s4) & kLow4) << 1 | ((t.x >> s2) & kLow2) << 5;
+    const uint32_t u1 = kTops | ((q.y >> s4) & kLow4) << 1 | ((t.y >> s2) & kLow2) << 5;
+    auto value = [&](float b) -> float { return mul_rn(ds, __fadd_rn(b, -96.0f)); };
+    out.x = half2_bits(value(biased64<0>(u0)), value(biased64<1>(u0))), out.y = half2_bits(value(biased64<2>(u0)), value(biased64<3>(u0)));
+    out.z = half2_bits(value(biased64<0>(u1)), value(biased64<1>(u1))), out.w = half2_bits(value(biased64<2>(u1)), value(biased64<3>(u1)));
+  } else {  // Q8_0: d q, the signed byte as q + 128; a block's f16 scale, then its bytes (2-byte aligned: read by halves)
     const uint16_t* hp = (const uint16_t*) blk;
-    const float d = half_value(hp[0]);
-    uint32_t m0, m1;
-    float c;
-    if constexpr (T == QTYPE_Q4_0) {  // d (n - 8): bytes 8 (k % 2) .., low (k < 2) or high nibbles
-      const uint16_t* q = hp + 1 + 4 * (k & 1u);
-      const uint32_t s4 = 4u * (k >> 1);
-      m0 = (((uint32_t) q[0] | (uint32_t) q[1] << 16) >> s4) & 0x0F0F0F0Fu;
-      m1 = (((uint32_t) q[2] | (uint32_t) q[3] << 16) >> s4) & 0x0F0F0F0Fu;
-      c = mul_rn(d, -32776.0f);
-    } else {  // Q8_0: d q, the signed byte as q + 128
-      const uint16_t* q = hp + 1 + 4 * k;
-      m0 = ((uint32_t) q[0] | (uint32_t) q[1] << 16) ^ 0x80808080u;
-      m1 = ((uint32_t) q[2] | (uint32_t) q[3] << 16) ^ 0x80808080u;
-      c = mul_rn(d, -32896.0f);
-    }
+    const float d = half_value(hp[0]), c = mul_rn(d, -32896.0f);
+    const uint16_t* q = hp + 1 + 4 * k;
+    const uint32_t m0 = ((uint32_t) q[0] | (uint32_t) q[1] << 16) ^ 0x80808080u, m1 = ((uint32_t) q[2] | (uint32_t) q[3] << 16) ^ 0x80808080u;
     out.x = half2_bits(__fmaf_rn(d, biased<0>(m0), c), __fmaf_rn(d, biased<1>(m0), c));
     out.y = half2_bits(__fmaf_rn(d, biased<2>(m0), c), __fmaf_rn(d, biased<3>(m0), c));
     out.z = half2_bits(__fmaf_rn(d, biased<0>(m1), c), __fmaf_rn(d, biased<1>(m1), c));
     out.w = half2_bits(__fmaf_rn(d, biased<2>(m1), c), __fmaf_rn(d, biased<3>(m1), c));
   }
   return out;
+}
+
+// ---- two chunks at once: the low and the high nibbles of the same eight bytes --------------------------------------
+// Of a 64-value K step a row has four such pairs: of the 32-value blocks pair i is chunks i % 2 and two on of block i / 2, of
+// Q4_K and Q5_K (groups 2 g and 2 g + 1 share 32 bytes) chunk i of either group. The bytes are read and unpacked once, the
+// F32 steps of the two run side by side in packed instructions.
+template <uint32_t T> constexpr bool kPairChunk = (T == QTYPE_MXFP4 || T == QTYPE_Q4_0 || T == QTYPE_Q4_K || T == QTYPE_Q5_K);
+template <uint32_t T> constexpr bool kPairOfGroups = (T == QTYPE_Q4_K || T == QTYPE_Q5_K);
+
+__device__ __forceinline__ void store_pairs(const uint64_t (&v)[8], uint4& lo, uint4& hi) {
+  float a[8], b[8];
+#pragma unroll
+  for (int j = 0; j < 8; j++) unpack2(v[j], a[j], b[j]);
+  lo = make_uint4(half2_bits(a[0], a[1]), half2_bits(a[2], a[3]), half2_bits(a[4], a[5]), half2_bits(a[6], a[7]));
+  hi = make_uint4(half2_bits(b[0], b[1]), half2_bits(b[2], b[3]), half2_bits(b[4], b[5]), half2_bits(b[6], b[7]));
+}
+
+// an E2M1 code's bits as an F16's sign, exponent's low two bits and mantissa's top one are its value times 2^-14 (a
+// subnormal code is a subnormal F16): `top` holds such upper bytes of four values, times f
+__device__ __forceinline__ uint2 e2m1_halves(uint32_t top, __half2 f) {
+  const uint32_t p0 = __byte_perm(top, 0, 0x1404), p1 = __byte_perm(top, 0, 0x3424);
+  const __half2 h0 = __hmul2_rn(*(const __half2*) &p0, f), h1 = __hmul2_rn(*(const __half2*) &p1, f);
+  return make_uint2(*(const uint32_t*) &h0, *(const uint32_t*) &h1);
+}
+__device__ __forceinline__ void scale_halves(uint4& v, uint32_t f2) {
+  const __half2 f = *(const __half2*) &f2;
+  uint32_t* w = (uint32_t*) &v;
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const __half2 h = __hmul2_rn(*(const __half2*) &w[i], f);
+    w[i] = *(const uint32_t*) &h;
+  }
+}
+
+// pair i of the step whose block (of the 32-value types: whose pair's block) starts at shared address `at`; g: the step's
+// place in a 256-value block. Q4_K and Q5_K: `at` on a word. Read first, decoded after: a thread's several pairs are all
+// read before the first is decoded and stored, so that their shared-memory latencies run together.
+struct PairBytes {
+  uint2 q, f;            // the eight bytes; Q5_K's fifth bits
+  uint32_t h[4];         // the block's head: Q4_K / Q5_K its first four words, else the scale
+};
+template <uint32_t T>
+__device__ __forceinline__ void load_pair(uint32_t at, uint32_t g, uint32_t i, PairBytes& b) {
+  if constexpr (T == QTYPE_MXFP4) {
+    b.h[0] = lds8(at), b.q = lds_8_bytes(at + 1u + 8u * (i & 1u));
+  } else if constexpr (T == QTYPE_Q4_0) {
+    b.h[0] = lds16(at), b.q = lds_8_bytes(at + 2u + 8u * (i & 1u));
+  } else {
+    const uint32_t qa = at + (T == QTYPE_Q5_K ? 48u : 16u) + 32u * g + 8u * i;
+#pragma unroll
+    for (int k = 0; k < 4; k++) b.h[k] = lds32(at + 4u * k);
+    b.q = make_uint2(lds32(qa), lds32(qa + 4u));
+    if constexpr (T == QTYPE_Q5_K) b.f = make_uint2(lds32(at + 16u + 8u * i), lds32(at + 20u + 8u * i));
+  }
+}
+template <uint32_t T>
+__device__ __forceinline__ void pair_chunks(const PairBytes& p, uint32_t g, uint4& lo, uint4& hi) {
+  const uint2 q = p.q;
+  if constexpr (T == QTYPE_MXFP4) {
+    // times 2^(e - 127): the f16 product by 2^(e - 113) is exact or rounds once, as the F32 value's conversion does - past
+    // F16 infinite, below it zero. 2^(e - 113) is an F16 for e <= 128; below e = 99 every value is under half of F16's
+    // least (6 2^-29), so the factor may be zero; above 128 the rest of the power goes in two more exact products.
+    const uint32_t e = p.h[0], f = e >= 99u ? (min(e, 128u) - 98u) << 10 : 0u, f2 = f | f << 16;
+    const __half2 fh = *(const __half2*) &f2;
+    const uint2 l0 = e2m1_halves(((q.x << 1) & 0x0E0E0E0Eu) | ((q.x << 4) & kTops), fh), l1 = e2m1_halves(((q.y << 1) & 0x0E0E0E0Eu) | ((q.y << 4) & kTops), fh);
+    const uint2 h0 = e2m1_halves(((q.x >> 3) & 0x0E0E0E0Eu) | (q.x & kTops), fh), h1 = e2m1_halves(((q.y >> 3) & 0x0E0E0E0Eu) | (q.y & kTops), fh);
+    lo = make_uint4(l0.x, l0.y, l1.x, l1.y), hi = make_uint4(h0.x, h0.y, h1.x, h1.y);
+    if (e > 128u) {
+      const uint32_t a = (min(e, 143u) - 113u) << 10, b = (min(max(e, 143u), 158u) - 128u) << 10;  // 2^(e - 128) up to 2^15; the rest up to 2^15
+      scale_halves(lo, a | a << 16), scale_halves(hi, a | a << 16), scale_halves(lo, b | b << 16), scale_halves(hi, b | b << 16);
+    }
+  } else if constexpr (T == QTYPE_Q4_0) {
+    const float d = half_value(p.h[0]);
+    const uint64_t dd = pack2(d, d);
+    uint64_t v[8];
+    code_pairs(make_uint2(q.x & kLow4, q.y & kLow4), make_uint2((q.x >> 4) & kLow4, (q.y >> 4) & kLow4), -32776.0f, v);
+#pragma unroll
+    for (int j = 0; j < 8; j++) v[j] = mul2(dd, v[j]);
+    store_pairs(v, lo, hi);
+  } else {  // Q4_K, Q5_K
+    uint32_t sc, mn;
+    k_scales(p.h[1], p.h[2], p.h[3], 16u * (g & 1u), g >= 2u, sc, mn);
+    const float d = half_value(p.h[0] & 0xFFFFu), m = -half_value(p.h[0] >> 16);
+    const uint64_t ds = mul2(pack2(d, d), pack2(byte_value<0>(sc), byte_value<1>(sc)));
+    const uint64_t dm = mul2(pack2(m, m), pack2(byte_value<0>(mn), byte_value<1>(mn)));  // (minus the minimum)
+    uint2 a = make_uint2(q.x & kLow4, q.y & kLow4), b = make_uint2((q.x >> 4) & kLow4, (q.y >> 4) & kLow4);
+    if constexpr (T == QTYPE_Q5_K) {  // the fifth bits: bits 2 g and 2 g + 1 of the 32 bytes at 16
+      const uint32_t f0 = p.f.x >> (2u * g), f1 = p.f.y >> (2u * g);
+      a.x |= (f0 & kOnes) << 4, a.y |= (f1 & kOnes) << 4, b.x |= (f0 << 3) & 0x10101010u, b.y |= (f1 << 3) & 0x10101010u;
+    }
+    uint64_t v[8];
+    code_pairs(a, b, -32768.0f, v);
+#pragma unroll
+    for (int j = 0; j < 8; j++) v[j] = add2(mul2(ds, v[j]), dm);
+    store_pairs(v, lo, hi);
+  }
 }
 
 struct Args {
@@ -242,39 +335,55 @@ __global__ void __launch_bounds__(kThreads, 1) mm_tc_kernel(const Args a, const 
     uint8_t* raw = smem + a.raw_off;
     const uint8_t* w_end = w + (uint64_t) a.rows * row_bytes;
     const uint32_t kblocks = (a.cols + kKb - 1) / kKb;
+    // this thread's pieces: where their rows start, worked out once (a 64-bit product a row), and their place in a buffer
+    constexpr int kFetch = (int) ((kM * kPieces + kProdThreads - 1) / kProdThreads);
+    const uint8_t* fetch_row[kFetch];
+    uint32_t fetch_at[kFetch];  // (a piece past the rows' last: none)
+#pragma unroll
+    for (int j = 0; j < kFetch; j++) {
+      const uint32_t i = pt + (uint32_t) j * kProdThreads, r = i / kPieces, piece = i - r * kPieces;
+      fetch_row[j] = i < (uint32_t) kM * kPieces ? w + wrow(r) * row_bytes : nullptr;
+      fetch_at[j] = r * kSlot + piece * 16u;
+    }
     auto fetch_raw = [&](uint32_t kb) {  // the rows' bytes of K block kb into buffer kb % 2
-      uint8_t* buf = raw + (kb & 1u) * (kM * kSlot);
-      for (uint32_t i = pt; i < (uint32_t) kM * kPieces; i += kProdThreads) {
-        const uint32_t r = i / kPieces, piece = i - r * kPieces;
-        const uint32_t row = wrow(r);
-        const uint8_t* src = (const uint8_t*) ((uintptr_t) (w + row * row_bytes + (uint64_t) kb * kKbBytes) & ~(uintptr_t) 15) + piece * 16u;
-        const uint32_t have = src >= w_end ? 0u : (w_end - src < 16 ? (uint32_t) (w_end - src) : 16u);  // (zero fill past the tensor)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(buf + r * kSlot + piece * 16u)), "l"(src), "r"(have)
-                     : "memory");
+      const uint32_t buf = smem_addr(raw) + (kb & 1u) * (kM * kSlot);
+#pragma unroll
+      for (int j = 0; j < kFetch; j++) {
+        if (!fetch_row[j]) continue;
+        const uint8_t* src = (const uint8_t*) ((uintptr_t) (fetch_row[j] + (uint64_t) (kb * kKbBytes)) & ~(uintptr_t) 15) + fetch_at[j] % kSlot;
+        const int64_t left = w_end - src;
+        const uint32_t have = left >= 16 ? 16u : left > 0 ? (uint32_t) left : 0u;  // (zero fill past the tensor)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(buf + fetch_at[j]), "l"(src), "r"(have) : "memory");
       }
       asm volatile("cp.async.commit_group;" ::: "memory");
     };
     // this thread's chunks of a step: chunk kc of rows 64 apart (eight neighbouring threads take one K piece of eight
     // neighbouring rows - eight different 16-byte bank columns of the operand tile, and of the raw buffer, whose row
     // slots are an odd number of 16-byte pieces); what does not change from step to step is worked out here
-    constexpr int kMine = kM * (kStep / 8) / kTeamThreads;
-    static_assert(kMine * kTeamThreads == kM * (kStep / 8) && kTeamThreads % 64 == 0, "every producer thread the same number of chunks");
+    constexpr uint32_t kChunks = kPairChunk<T> ? kStep / 16 : kStep / 8;  // a row's of a step: pairs, or chunks
+    constexpr int kMine = kM * (int) kChunks / kTeamThreads;
+    static_assert(kMine * kTeamThreads == kM * (int) kChunks && kTeamThreads % (8 * kChunks) == 0, "every producer thread the same number of chunks");
     const uint32_t team = pt / kTeamThreads, tt = pt % kTeamThreads;  // the thread's team and its place in it
-    const uint32_t kc = (tt >> 3) & 7u;
+    const uint32_t kc = (tt >> 3) % kChunks;
+    // (a pair's first chunk; its second is two on in a 32-value block, four on where the pair is two groups of 32)
+    const uint32_t kc0 = !kPairChunk<T> || kPairOfGroups<T> ? kc : 4u * (kc >> 1) + (kc & 1u);
+    constexpr uint32_t kSecond = (kPairOfGroups<T> ? 2u : 1u) * kSubTile;
     uint32_t slot_at[kMine], dst_at[kMine], base15[kMine];
 #pragma unroll
     for (int u = 0; u < kMine; u++) {
-      const uint32_t task = tt + (uint32_t) u * kTeamThreads, r = (task >> 6) * 8u + (task & 7u);
+      const uint32_t task = tt + (uint32_t) u * kTeamThreads, r = task / (8 * kChunks) * 8u + (task & 7u);
       const uint32_t row = wrow(r);  // (a row past the matrix repeats the last one)
-      slot_at[u] = r * kSlot, dst_at[u] = (kc >> 1) * kSubTile + (r >> 3) * 256 + (kc & 1u) * 128 + (r & 7u) * 16;
+      slot_at[u] = r * kSlot, dst_at[u] = (kc0 >> 1) * kSubTile + (r >> 3) * 256 + (kc0 & 1u) * 128 + (r & 7u) * 16;
       base15[u] = (uint32_t) ((uintptr_t) (w + row * row_bytes) & 15u);
     }
     bool dead = false;  // a wait ran out: no more work, but the producers' own barrier is still kept
     fetch_raw(0);
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     static_assert((kKb / kStep) % kGroups == 0, "every team has steps in every K block");
-    for (uint32_t it = team; it < steps; it += kGroups) {
-      const uint32_t stage = it % S, use = it / S, kb = it / (kKb / kStep), sub = it % (kKb / kStep);
+    uint32_t stage = team % S, use = team / S;  // step it's stage and how often it has been used before
+    for (uint32_t it = team; it < steps; it += kGroups, stage += kGroups) {
+      if (stage >= S) stage -= S, use++;  // (a ring is two stages at least)
+      const uint32_t kb = it / (kKb / kStep), sub = it % (kKb / kStep);
       const bool first = sub == team;  // the team's first step of K block kb
       if (first) {  // this thread's pieces of block kb have landed; after the barrier everyone's have, and block
         asm volatile("cp.async.wait_group 0;" ::: "memory");  // kb - 1's buffer is free for kb + 1
@@ -286,24 +395,53 @@ __global__ void __launch_bounds__(kThreads, 1) mm_tc_kernel(const Args a, const 
       // A: the chunk decoded to 8 halves, 16 bytes, to sub-tile kc / 2 of the stage
       uint8_t* sa = smem + stage * a.stage_bytes;
       const uint8_t* buf = raw + (kb & 1u) * (kM * kSlot);
-      const uint32_t cl = sub * (kStep / kChunk) + kc;  // the chunk's index in its K block
-      const uint32_t in_blk = (cl / Fmt<T>::chunks) * Fmt<T>::bytes, k_in = cl % Fmt<T>::chunks;
       const uint32_t kb15 = (kb * kKbBytes) & 15u;
+      if constexpr (kPairChunk<T>) {
+        const uint32_t in_blk = kPairOfGroups<T> ? 0u : (sub * (kStep / 32) + (kc >> 1)) * Fmt<T>::bytes;
+        uint32_t at[kMine];
+        bool whole = true;  // (of Q4_K and Q5_K: the thread's blocks start on words, as they do in a matrix that does)
 #pragma unroll
-      for (int u = 0; u < kMine; u++) {
-        const uint8_t* blk = buf + slot_at[u] + ((base15[u] + kb15) & 15u) + in_blk;
-        uint4 out;
-        bool done = false;
-        if constexpr (kFastChunk<T>) {
-          if (T != QTYPE_Q4_K || ((uintptr_t) blk & 3u) == 0) out = fast_chunk<T>(blk, k_in), done = true;
+        for (int u = 0; u < kMine; u++) {
+          at[u] = smem_addr(buf) + slot_at[u] + ((base15[u] + kb15) & 15u) + in_blk;
+          if (kPairOfGroups<T> && (at[u] & 3u)) whole = false;
         }
-        if (!done) {
-          float v[kChunk];
-          decode8<T>(blk, (int) k_in, v, g);
-          out.x = half2_bits(v[0], v[1]), out.y = half2_bits(v[2], v[3]);
-          out.z = half2_bits(v[4], v[5]), out.w = half2_bits(v[6], v[7]);
+        uint4 lo[kMine], hi[kMine];
+        if (whole) {
+          PairBytes raw_pair[kMine];
+#pragma unroll
+          for (int u = 0; u < kMine; u++) load_pair<T>(at[u], sub, kc, raw_pair[u]);
+#pragma unroll
+          for (int u = 0; u < kMine; u++) pair_chunks<T>(raw_pair[u], sub, lo[u], hi[u]);
+        } else if constexpr (kPairOfGroups<T>) {
+#pragma unroll
+          for (int u = 0; u < kMine; u++) {
+            const uint8_t* blk = buf + (at[u] - smem_addr(buf));
+            float v[kChunk];
+            decode8<T>(blk, (int) (8u * sub + kc), v, g);
+            lo[u] = make_uint4(half2_bits(v[0], v[1]), half2_bits(v[2], v[3]), half2_bits(v[4], v[5]), half2_bits(v[6], v[7]));
+            decode8<T>(blk, (int) (8u * sub + 4u + kc), v, g);
+            hi[u] = make_uint4(half2_bits(v[0], v[1]), half2_bits(v[2], v[3]), half2_bits(v[4], v[5]), half2_bits(v[6], v[7]));
+          }
         }
-        *(uint4*) (sa + dst_at[u]) = out;
+#pragma unroll
+        for (int u = 0; u < kMine; u++) *(uint4*) (sa + dst_at[u]) = lo[u], *(uint4*) (sa + dst_at[u] + kSecond) = hi[u];
+      } else {
+        const uint32_t cl = sub * (kStep / kChunk) + kc;  // the chunk's index in its K block
+        const uint32_t in_blk = (cl / Fmt<T>::chunks) * Fmt<T>::bytes, k_in = cl % Fmt<T>::chunks;
+#pragma unroll
+        for (int u = 0; u < kMine; u++) {
+          const uint8_t* blk = buf + slot_at[u] + ((base15[u] + kb15) & 15u) + in_blk;
+          uint4 out;
+          if constexpr (kFastChunk<T>) {
+            out = fast_chunk<T>(blk, k_in);
+          } else {
+            float v[kChunk];
+            decode8<T>(blk, (int) k_in, v, g);
+            out.x = half2_bits(v[0], v[1]), out.y = half2_bits(v[2], v[3]);
+            out.z = half2_bits(v[4], v[5]), out.w = half2_bits(v[6], v[7]);
+          }
+          *(uint4*) (sa + dst_at[u]) = out;
+        }
       }
       fence_async_smem();  // these writes before the tensor core's reads
       __syncwarp();
@@ -322,8 +460,9 @@ __global__ void __launch_bounds__(kThreads, 1) mm_tc_kernel(const Args a, const 
       // MMA reads (tiles past the last are filled with zeros); the stage's barrier counts the bytes.
       if (lt < (uint32_t) kWarp) {
         const uint32_t ops = n_acc * kSubs;
-        for (uint32_t it = 0; it < steps; it++) {
-          const uint32_t stage = it % S, use = it / S;
+        uint32_t stage = 0, use = 0;
+        for (uint32_t it = 0; it < steps; it++, stage++) {
+          if (stage == S) stage = 0, use++;
           if (use > 0 && !bar_wait(&sh.empty[stage], (use - 1) & 1u)) {
             sh.fail = 1;
             break;
@@ -340,30 +479,36 @@ __global__ void __launch_bounds__(kThreads, 1) mm_tc_kernel(const Args a, const 
           }
         }
       }
-    } else
-    for (uint32_t it = 0; it < steps; it++) {
-      const uint32_t stage = it % S, use = it / S;
-      if (use > 0 && !bar_wait(&sh.empty[stage], (use - 1) & 1u)) {
-        sh.fail = 1;
-        break;
+    } else {
+      // (eight neighbouring threads: one K piece of eight neighbouring tokens - eight different 16-byte bank columns of the
+      // operand tile, so a store takes no more passes than its bytes need.) A thread's pieces are one K piece of every
+      // sixteenth token: a tile of x16 on, 512 bytes on in the operand, to the next accumulator's part every 128 tokens.
+      const uint32_t kc = (lt >> 3) & 7u, n0 = (lt >> 6) * 8u + (lt & 7u);
+      static_assert(kLoaderThreads == 128 && MM_TILE == 16, "a round of pieces is sixteen tokens");
+      const __half* src0 = x16 + mm_x16_at(c0 + n0, kc * 8, a.xts);
+      const uint64_t step_halves = mm_x16_at(0, kStep, a.xts), tile_halves = mm_x16_at(MM_TILE, 0, a.xts);
+      const uint32_t dst0 = (kc >> 1) * kSubTile + (n0 >> 3) * 256 + (kc & 1u) * 128 + (n0 & 7u) * 16;
+      uint32_t stage = 0, use = 0;
+      for (uint32_t it = 0; it < steps; it++, stage++, src0 += step_halves) {
+        if (stage == S) stage = 0, use++;
+        if (use > 0 && !bar_wait(&sh.empty[stage], (use - 1) & 1u)) {
+          sh.fail = 1;
+          break;
+        }
+        const uint32_t sb = smem_addr(smem + stage * a.stage_bytes + kStageA) + dst0;
+        const __half* src = src0;
+        for (uint32_t n = 0; n < n_valid16; n += 16, src += tile_halves)
+          cp_async16(sb + (n / kN) * (kSubs * kSubTile) + (n % kN) * 32, src);
+        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_addr(&sh.full_b[stage])) : "memory");
       }
-      const uint32_t sb = smem_addr(smem + stage * a.stage_bytes + kStageA);
-      const uint32_t pieces = n_valid16 * (kStep / 8);
-      for (uint32_t i = lt; i < pieces; i += kLoaderThreads) {
-        // (eight neighbouring threads: one K piece of eight neighbouring tokens - eight different 16-byte bank
-        // columns of the operand tile, so a store takes no more passes than its bytes need)
-        const uint32_t kc = (i >> 3) & 7u, n = (i >> 6) * 8u + (i & 7u), acc = n / kN, nn = n % kN;
-        cp_async16(sb + (acc * kSubs + (kc >> 1)) * kSubTile + (nn >> 3) * 256 + (kc & 1u) * 128 + (nn & 7u) * 16,
-                   x16 + mm_x16_at(c0 + n, it * kStep + kc * 8, a.xts));
-      }
-      asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_addr(&sh.full_b[stage])) : "memory");
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
   } else if (warp == (uint32_t) kIssuerWarp) {
     // ================= issuer =================
     bool ok = true;
-    for (uint32_t it = 0; it < steps && !sh.fail; it++) {
-      const uint32_t stage = it % S, use = it / S;
+    uint32_t stage = 0, use = 0;
+    for (uint32_t it = 0; it < steps && !sh.fail; it++, stage++) {
+      if (stage == S) stage = 0, use++;
       if (!bar_wait(&sh.full_a[stage], use & 1u) || !bar_wait(&sh.full_b[stage], use & 1u)) {
         sh.fail = 1, ok = false;
         break;
@@ -402,10 +547,10 @@ __global__ void __launch_bounds__(kThreads, 1) mm_tc_kernel(const Args a, const 
     const uint32_t parts = EPI == kGatedMean ? 1u : ((uint32_t) (kThreads / kWarp) - quarter + 3u) / 4u;  // the quarter's warps
     const uint32_t row = 32u * quarter + lane;  // this thread's weight row of the tile = its TMEM lane
     const uint32_t lane_base = tmem + ((32u * quarter) << 16);
-    if (!bar_wait(&sh.done, 0)) {
+    if (!bar_wait_long(&sh.done, 0)) {
       // (the K loop's own waits are 0.2 s each and can queue up: look again while nobody has given up)
       bool landed = false;
-      for (uint32_t tries = 0; tries < 25u && !sh.fail && !landed; tries++) landed = bar_wait(&sh.done, 0);
+      for (uint32_t tries = 0; tries < 25u && !sh.fail && !landed; tries++) landed = bar_wait_long(&sh.done, 0);
       if (!landed) sh.fail = 1;
     }
     // (nobody else writes the word once the last product has landed or been given up: after this barrier every

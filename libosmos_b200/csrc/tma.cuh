@@ -81,6 +81,23 @@ __device__ __forceinline__ bool bar_wait(uint64_t* bar, uint32_t parity) {
     else if (global_ns() - t0 > kWaitLimitNs) return false;
   }
 }
+// the same for a wait that is expected to be long (an epilogue's, through a whole K loop): the look itself may suspend the
+// warp for up to 10 us at a time - it still returns when the phase completes - so that waiting costs no issue slots
+__device__ __forceinline__ bool bar_wait_long(uint64_t* bar, uint32_t parity) {
+  const uint32_t a = smem_addr(bar);
+  uint64_t t0 = 0;
+  for (uint32_t spin = 0;; spin++) {
+    uint32_t done;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 10000;\n selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(done)
+        : "r"(a), "r"(parity)
+        : "memory");
+    if (done) return true;
+    if (spin == 0) t0 = global_ns();
+    else if (global_ns() - t0 > kWaitLimitNs) return false;
+  }
+}
 // global -> this block's shared memory, completion counted on `bar`; both addresses 16-byte aligned, bytes a multiple of 16
 __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_addr(dst)),

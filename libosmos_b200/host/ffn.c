@@ -218,18 +218,18 @@ bool q4x_moe_scratch_bind(const Q4xMoeLayer *l, uint32_t max_tok, void *mem, uin
   return true;
 }
 
-/* one expert tensor over the tables' runs of tile counts, a launch a run (hip_layers.c:317-329) */
+/* one expert tensor over all the tables' entries in one launch: every run of tile counts holds at most 128 tokens an entry,
+   one block's, so a launch a run (hip_layers.c:317-329) would give the same blocks with a thin last wave a run */
 static bool experts(uint32_t type, const void *const *ptr, const Q4xMoeScratch *s, const Q4xExpertBounds *bd, uint32_t rows,
                     uint32_t cols, const uint32_t *xo, float *y, const uint32_t *yo, void *stream)
 {
   bool ok = true;
-  for (int r = 0; ok && r < Q4X_TILE_RUNS; r++)
-    if (bd->count[r])
-    {
-      const uint32_t at = bd->first[r];
-      ok = mm_group(type, ptr + at, s->cnt + at, bd->count[r], (uint32_t)MM_TILE << r, rows, cols, s->xe16, xo + at, cols, y,
-                    yo + at, rows, stream);
-    }
+  for (uint32_t at = 0; ok && at < bd->entries; at += MV_MAX_GROUP)
+  {
+    const uint32_t left = bd->entries - at, n = left < MV_MAX_GROUP ? left : MV_MAX_GROUP;
+    ok = mm_group(type, ptr + at, s->cnt + at, n, (uint32_t)MM_TILE << (Q4X_TILE_RUNS - 1), rows, cols, s->xe16, xo + at, cols, y,
+                  yo + at, rows, stream);
+  }
   return ok;
 }
 
