@@ -41,8 +41,9 @@ constexpr uint32_t kTaskRows = 32;  // rows a fused task has at most, a lane eac
 constexpr uint32_t kMaxEntries = 1024;  // entries a launch takes (their pointers and live list sit in shared memory)
 constexpr uint32_t kSmemLimit = 226u * 1024u;
 
-// the codebooks' bytes, from the start of dynamic shared memory
-template <uint32_t T> constexpr uint32_t kLutBytes = kTernary<T> ? lanes::kTernaryBytes : ((uint32_t) Rep<T>::bytes + 127u) & ~127u;
+// the codebooks' bytes, from the start of dynamic shared memory (COPIES: of the IQ1 types' table)
+template <uint32_t T, int COPIES> constexpr uint32_t kLutBytes = kTernary<T> ? lanes::kTernaryBytes<COPIES> : ((uint32_t) Rep<T>::bytes + 127u) & ~127u;
+static_assert(lanes::kTernaryBytes<4> == (uint32_t) Rep<QTYPE_IQ1_M>::bytes, "four copies take what two of the byte grid did: no shape is lost");
 
 __device__ uint32_t g_status;
 
@@ -64,7 +65,7 @@ struct Args {
 
 // L: lanes a row; NB: blocks a lane holds at most (EXACT: exactly - no test a block, so the blocks' loads can be
 // scheduled together); NT: tokens a task carries
-template <uint32_t T, bool FUSED, int L, int NB, int NT, bool EXACT>
+template <uint32_t T, bool FUSED, int L, int NB, int NT, bool EXACT, int COPIES>
 __global__ void __launch_bounds__(kThreads, 1) lane_ring_kernel(const Args a) {
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ __align__(8) uint64_t full[kWarps][kMaxSlots];
@@ -86,7 +87,7 @@ __global__ void __launch_bounds__(kThreads, 1) lane_ring_kernel(const Args a) {
     bar_init_fence();
   }
   RepLuts2<T> luts{};
-  if constexpr (kTernary<T>) lanes::build_ternary(smem, kThreads);  // (complete at the list's first barrier below)
+  if constexpr (kTernary<T>) lanes::build_ternary<COPIES>(smem, kThreads);  // (complete at the list's first barrier below)
   else luts = build_luts2<T>(smem, kThreads);
   // (a dependent launch: the tables and activations read from here on may be the output of the kernels ahead; the
   // codebooks above are not)
@@ -192,7 +193,7 @@ __global__ void __launch_bounds__(kThreads, 1) lane_ring_kernel(const Args a) {
         if constexpr (T == QTYPE_IQ3_XXS || kTernary<T>) {
           float bs[NTL];
           if constexpr (T == QTYPE_IQ3_XXS) iq3_block_sums<NTL, NT, NB>(ra + k * kSbStep, at, luts, xq, k, bs);
-          else iq1_block_sums<T, NTL, NT, NB>(ra + k * kSbStep, at, smem, lane % lanes::kTernaryCopies * 4u, xq, xc, k, bs);
+          else iq1_block_sums<T, COPIES, NTL, NT, NB>(ra + k * kSbStep, at, smem, lane % COPIES * 4u, xq, xc, k, bs);
 #pragma unroll
           for (int t = 0; t < NTL; t++) acc[t] = __fmaf_rn(xd[t][k], bs[t], acc[t]);
         } else {
@@ -353,15 +354,15 @@ const Device* device_info() {
   return &devs[d];
 }
 
-template <uint32_t T, bool FUSED, int L, int NB, int NT, bool EXACT>
-int launch(const Request& r, cudaStream_t s) {
+template <uint32_t T, bool FUSED, int L, int NB, int NT, bool EXACT, int COPIES>
+int launch_with(const Request& r, cudaStream_t s) {
   const Device* dev = device_info();
   if (!dev) return 0;
   constexpr uint32_t M = FUSED ? 2 : 1, RU = FUSED ? 1 : kWarp / L;
   const uint32_t row_bytes = r.cols / 256 * Super<T>::bytes;
   Args a{};
-  a.list_off = kLutBytes<T>;
-  a.ptr_off = (a.list_off + r.n_entries * ((r.max_cnt + NT - 1) / NT) * 2u + 7u) & ~7u;  // (an entry has at most max_cnt / NT groups)
+  a.list_off = kLutBytes<T, COPIES>;
+  a.ptr_off = a.list_off + kMaxEntries * (8 / NT) * 2;
   a.ring_off = (a.ptr_off + r.n_entries * (M * 8 + 8) + 127u) & ~127u;  // (pointers, then (count, first row))
   if (a.ring_off + 16u >= kSmemLimit) return 0;
   // a slot: the fewest rows (a multiple of the rows a pass takes) whose bytes are a multiple of 16 and reach about 3 KB
@@ -387,9 +388,17 @@ int launch(const Request& r, cudaStream_t s) {
   const uint32_t total = a.ring_off + kWarps * slots * slot_bytes + 16u;
   if (r.dry) return 1;
   static bool sized[64] = {};  // (per template instance and device: the attribute belongs to a device's context)
-  auto kernel = lane_ring_kernel<T, FUSED, L, NB, NT, EXACT>;
+  auto kernel = lane_ring_kernel<T, FUSED, L, NB, NT, EXACT, COPIES>;
   if (!allow_dynamic_smem(kernel, (int) kSmemLimit, sized)) return 0;
   return launch_dependent(kernel, dim3((uint32_t) dev->sms), dim3(kThreads), total, s, a) == cudaSuccess ? 1 : -1;
+}
+
+// the IQ1 types with eight copies of their table where two slots a warp still fit beside it, else with four
+template <uint32_t T, bool FUSED, int L, int NB, int NT, bool EXACT>
+int launch(const Request& r, cudaStream_t s) {
+  if constexpr (kTernary<T>)
+    if (const int st = launch_with<T, FUSED, L, NB, NT, EXACT, 8>(r, s)) return st;
+  return launch_with<T, FUSED, L, NB, NT, EXACT, 4>(r, s);
 }
 
 template <uint32_t T, bool FUSED>

@@ -87,13 +87,14 @@ __device__ __forceinline__ void iq3_block_sums(uint32_t sb, const LaneAt& at, co
 
 // ---- IQ1_S, IQ1_M: the ternary codebook in shared memory as nibbles -------------------------------------------------
 // An entry's eight values t (-1, 0, 1) as t + 1 in eight nibbles: byte b has value b low and value 4 + b high. One 4-byte
-// word where the byte grid has eight, so eight copies (64 KB) stand where two of the byte grid's would: a warp's 32 random
-// lookups, four lanes a copy, meet about three deep in a bank instead of six (two copies of 8-byte entries).
-constexpr uint32_t kTernaryCopies = 8, kTernaryBytes = 2048u * kTernaryCopies * 4u;
+// word where the byte grid has eight: in eight copies (64 KB) a warp's 32 random lookups, four lanes a copy, meet about three
+// deep in a bank, where two copies of 8-byte entries (32 KB) met six. Four copies take those 32 KB, for the row widths whose
+// ring needs the room.
+template <int COPIES> constexpr uint32_t kTernaryBytes = 2048u * COPIES * 4u;
 template <uint32_t T> constexpr bool kTernary = (T == QTYPE_IQ1_S || T == QTYPE_IQ1_M);
 
 // every thread of the block calls it; the table is complete at the block's next barrier
-__device__ inline void build_ternary(uint8_t* smem, int threads) {
+template <int COPIES> __device__ inline void build_ternary(uint8_t* smem, int threads) {
   constexpr int U = 4;
   for (int i0 = threadIdx.x; i0 < 2048; i0 += threads * U) {
     uint64_t g[U];
@@ -103,8 +104,9 @@ __device__ inline void build_ternary(uint8_t* smem, int threads) {
     for (int u = 0; u < U; u++)
       if (i0 + u * threads < 2048) {
         const uint32_t w = __vadd4((uint32_t) g[u], kOnes) | __vadd4((uint32_t) (g[u] >> 32), kOnes) << 4;
-        uint4* to = (uint4*) (smem + (uint32_t) (i0 + u * threads) * (kTernaryCopies * 4u));
-        to[0] = make_uint4(w, w, w, w), to[1] = make_uint4(w, w, w, w);
+        uint4* to = (uint4*) (smem + (uint32_t) (i0 + u * threads) * (COPIES * 4u));
+#pragma unroll
+        for (int c = 0; c < COPIES / 4; c++) to[c] = make_uint4(w, w, w, w);
       }
   }
 }
@@ -125,7 +127,7 @@ __device__ __forceinline__ void chunk_sums(const int (&x)[8], int (&out)[2]) {
 // a task (xc). The sum starts at 0x4B400000, so that it ends as the F32 12582912 + 2 S (|2 S| < 2^22): one subtraction
 // instead of an integer conversion. Half of 2 S goes into the scale, (2 s + 1) / 16: d (2 s + 1) has 15 significant bits,
 // so every product before the last is exact in any order and the last rounds the same number.
-template <uint32_t T, int NTL, int NT, int NB>
+template <uint32_t T, int COPIES, int NTL, int NT, int NB>
 __device__ __forceinline__ void iq1_block_sums(uint32_t sb, const LaneAt& at, const uint8_t* table, uint32_t copy,
                                                const int (&xq)[NT][NB][8], const int (&xc)[NT][NB][2], int k, float* out) {
   const uint32_t j = at.j;
@@ -155,8 +157,9 @@ __device__ __forceinline__ void iq1_block_sums(uint32_t sb, const LaneAt& at, co
 #pragma unroll
   for (int c = 0; c < 4; c++) {
     constexpr int kTop = T == QTYPE_IQ1_M ? 4 : 3;  // bits a chunk has in qh
-    const uint32_t q = c == 0 ? qs << 5 : qs >> (8 * c - 5), h = qh << (13 - kTop * c);  // (index x 32 bytes an entry)
-    w[c] = *(const uint32_t*) (table + ((h & 0xE000u) | ((q & 0x1FE0u) | copy)));
+    constexpr int kSh = COPIES == 8 ? 5 : 4;  // (an entry's copies are 32 or 16 bytes)
+    const uint32_t q = c == 0 ? qs << kSh : qs >> (8 * c - kSh), h = qh << (8 + kSh - kTop * c);
+    w[c] = *(const uint32_t*) (table + ((h & (7u << (8 + kSh))) | ((q & (0xFFu << kSh)) | copy)));
   }
   int acc[NTL][2];
 #pragma unroll

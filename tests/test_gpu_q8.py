@@ -124,7 +124,7 @@ def test_group_tok_and_gate_up(lib, dev, oracle, name, cols):
 
 
 @pytest.mark.parametrize("name", ["IQ1_S", "IQ1_M", "IQ2_XXS", "IQ3_XXS"])
-@pytest.mark.parametrize("cols", [512, 1024, 2048, 3072, 4096, 5120, 6144, 7168, 8192])
+@pytest.mark.parametrize("cols", [512, 1024, 1536, 2048, 4096, 5120, 6144, 7168, 8192])
 def test_lane_ring_row_widths(lib, dev, oracle, name, cols):
     """the warp-ring kernel's row widths: every number of blocks a lane holds, one token and two a decode, activations
     at the codes' limits (all 127, alternating +-127) among them"""
