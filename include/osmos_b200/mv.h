@@ -63,11 +63,12 @@ bool mv_fp4(const void *w, uint32_t rows, uint32_t cols, const float *x, uint32_
 bool mv_fp4_tok(const void *const *w, const int32_t *cnt, const int32_t *xrow, uint32_t n, uint32_t rows,
                 uint32_t cols, const float *x, uint32_t xs, float *y, uint32_t ys, void *stream);
 
-/* Not in the reference. mv_run / mv_strided have two kernels that give the same bits: one that stages whole rows
-   through shared memory with bulk copies (16-byte aligned w and x, rows whose bytes are a multiple of 16, x and a
-   ring of rows fitting shared memory) and a generic one for every other shape. mv_set_staged(0) forces the generic
-   kernel (the tests compare the two). mv_status() reads and clears the staged kernel's record on the current device
-   (it synchronizes): bit 0 = a bulk copy never landed within the kernel's wait limit, whose rows were not written. */
+/* Not in the reference. The matvecs have kernels that stage rows through shared memory with bulk copies (16-byte aligned w
+   and x, columns in 256s; for all but seven types rows whose bytes are a multiple of 16, x and a ring of rows fitting
+   shared memory) and a generic one for every other shape: the same bits. mv_set_staged(0) forces the generic kernel (the
+   tests compare them). mv_status() reads and clears the staged kernels' record on the current device (it synchronizes):
+   bit 0 = a bulk copy never landed within the kernel's wait limit, whose rows were not written; bit 1 = a grouped matrix
+   did not start on 16 bytes though its rows are whole 16-byte pieces, and was left alone. */
 void mv_set_staged(int on);
 uint32_t mv_status(void);
 

@@ -11,8 +11,11 @@
 // read of x whose neighbouring lanes ask for the same piece takes two passes of shared memory, one whose halves do takes
 // four, like 32 different pieces (measured: 2.0 against 4.0 cycles a warp).
 //
-// Bound by: instruction issue and shared-memory passes, about 4 instructions a value at one token (a byte permute, half
-// of an add, half of a multiply, half of an fmaf, and a quarter of the unpacking); HBM for the wider types.
+// Bound by instruction issue and shared-memory passes: about 5 instructions a value at one token (a byte permute, half of an
+// add, half of a multiply, half of an fmaf, the unpacking), and from three tokens on x's reads. Measured, against a lane a
+// thread (mv_staged.cu): 49152 x 2048 at one token Q6_K 41.1 -> 29.5 us (2.8 TB/s), Q5_K 45.1 -> 33.4, Q4_K 39.6 -> 29.9, IQ4_XS
+// 42.1 -> 27.7; at eight tokens 80-85 -> 64-69; Q4_K 2048 x 7168 at five 22.6 -> 12.0; 1536 x 4096 MXFP4 matrices of 64 experts
+// at 64 picks 239 -> 111 us.
 //
 // A warp owns a ring of slots; a slot holds the same run of up to 8 256-value stretches of its 2 RT rows, a bulk copy a
 // row of the 16-byte pieces around the row's bytes - so a row may start anywhere (Q6_K's 210-byte blocks: rows are
@@ -356,6 +359,27 @@ struct Warp {  // one warp's view of a block's work on one matrix and one pass o
   }
 };
 
+// a block's share of a matrix that does not start on 16 bytes: mv.cu's sums straight from global memory, a row a warp, a token
+// at a time
+template <uint32_t T>
+__device__ __noinline__ void rows_in_place(const uint8_t* mat, uint32_t row_bytes, const Args& a, const float* x, float* y, uint32_t live) {
+  const uint32_t lane = threadIdx.x % kWarp, warp = threadIdx.x / kWarp, lo = (uint32_t) ((uint64_t) blockIdx.x * a.rows / gridDim.x),
+                 hi = (uint32_t) ((uint64_t) (blockIdx.x + 1) * a.rows / gridDim.x);
+  for (uint32_t r = lo + warp; r < hi; r += kWarps)
+    for (uint32_t t = 0; t < live; t++) {
+      float s = 0.0f;
+      for (uint32_t c = lane; c < a.cols / kChunk; c += kWarp) {
+        float v[kChunk];
+        decode8<T>(mat + (uint64_t) r * row_bytes + (c / Fmt<T>::chunks) * Fmt<T>::bytes, (int) (c % Fmt<T>::chunks), v, Grids{});
+        const float* xc = x + (uint64_t) t * a.xs + c * kChunk;
+#pragma unroll
+        for (int j = 0; j < kChunk; j++) s = __fmaf_rn(v[j], xc[j], s);
+      }
+      s = xor_tree<kWarp>(s);
+      if (lane == 0) y[(uint64_t) t * a.ys + r] = s;
+    }
+}
+
 template <uint32_t T, int RT, bool GROUP>
 __global__ void __launch_bounds__(kThreads, 1) mv_pair_kernel(const Args a) {
   extern __shared__ __align__(128) uint8_t smem[];
@@ -391,8 +415,13 @@ __global__ void __launch_bounds__(kThreads, 1) mv_pair_kernel(const Args a) {
       xin = a.x + (uint64_t) (m / a.x_div) * a.x_mat, yout = a.y + (uint64_t) m * a.rows, live = 1;
     }
     me.mat = a.wt[m];
-    if ((uintptr_t) me.mat & 15u) {  // such a matrix cannot be copied in bulk: reported, its rows left alone
-      if (tid == 0) atomicOr(a.status, 2u);
+    if ((uintptr_t) me.mat & 15u) {  // such a matrix cannot be copied in bulk:
+      if (me.row_bytes % 16u == 0) {  // reported, its rows left alone
+        if (tid == 0) atomicOr(a.status, 2u);
+        return;
+      }
+      // where an expert's bytes need not be whole 16-byte pieces, its matrix need not start on one: read where it lies
+      rows_in_place<T>(me.mat, me.row_bytes, a, xin, yout, live);
       return;
     }
   }

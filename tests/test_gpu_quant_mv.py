@@ -179,6 +179,29 @@ def test_mv_paired_lanes_grouped(lib, dev, oracle, name, cols, rows):
     assert lib.mv_status() == 0
 
 
+@pytest.mark.parametrize("name,cols,off", [("Q6_K", 768, 2), ("Q6_K", 256, 10), ("MXFP4", 768, 8), ("MXFP4", 256, 3), ("IQ4_XS", 768, 8)])
+def test_mv_grouped_matrices_anywhere(lib, dev, oracle, name, cols, off):
+    """matrices whose rows are not whole 16-byte pieces need not start on one"""
+    tid, rows, cnt = TYPES[name], 45, [3, 8, 1]
+    rng = synth.rng_for(18, tid, cols)
+    mats = [synth.random_tensor(tid, rows, cols, rng) for _ in cnt]
+    step = (mats[0].size + 15) // 16 * 16 + 16
+    pool = np.zeros(step * len(cnt) + 16, np.uint8)
+    for m, w in enumerate(mats):
+        pool[m * step + off:m * step + off + w.size] = w.reshape(-1)
+    xrow = np.cumsum([0] + cnt[:-1]).astype(np.int32)
+    x = rng.standard_normal((sum(cnt), cols)).astype(np.float32)
+    pd = to_dev(pool, dev)
+    table = pointer_table(pd, [m * step + off for m in range(len(cnt))], dev)
+    y = torch.full((sum(cnt), rows), -3.0, dtype=torch.float32, device=dev)
+    lib.mv_status()
+    assert lib.mv_group_tok(tid, ptr(table), ptr(to_dev(np.array(cnt, np.int32), dev)), ptr(to_dev(xrow, dev)), len(cnt), 8, rows, cols,
+                            ptr(to_dev(x, dev)), cols, ptr(y), rows, None)
+    sync()
+    assert same_bits(y.cpu().numpy(), np.concatenate([oracle.mv_rows(tid, w, rows, cols, x[int(r):int(r) + c]) for w, r, c in zip(mats, xrow, cnt)]))
+    assert lib.mv_status() == 0
+
+
 @pytest.mark.parametrize("name", ["Q4_0", "IQ3_XXS", "Q4_K", "MXFP4"])
 def test_mv_strided_many_tokens(lib, dev, oracle, name):
     tid = TYPES[name]
