@@ -155,7 +155,9 @@ __device__ __forceinline__ uint4 fast_chunk(const uint8_t* blk, uint32_t k) {
 // ---- two chunks at once: the low and the high nibbles of the same eight bytes --------------------------------------
 // Of a 64-value K step a row has four such pairs: of the 32-value blocks pair i is chunks i % 2 and two on of block i / 2, of
 // Q4_K and Q5_K (groups 2 g and 2 g + 1 share 32 bytes) chunk i of either group. The bytes are read and unpacked once, the
-// F32 steps of the two run side by side in packed instructions.
+// F32 steps of the two run side by side in packed instructions. (4096 x 4096, 512 tokens, rounding included: MXFP4 67 -> 47 us -
+// its chunks went through the byte reader - Q5_K 70 -> 58, Q4_K 67 -> 52, Q4_0 52 -> 47. At 2048 tokens, where the products'
+// operand reads are the bound, 108-110 us as before.)
 template <uint32_t T> constexpr bool kPairChunk = (T == QTYPE_MXFP4 || T == QTYPE_Q4_0 || T == QTYPE_Q4_K || T == QTYPE_Q5_K);
 template <uint32_t T> constexpr bool kPairOfGroups = (T == QTYPE_Q4_K || T == QTYPE_Q5_K);
 
