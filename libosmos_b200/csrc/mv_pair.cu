@@ -288,7 +288,7 @@ struct Warp {  // one warp's view of a block's work on one matrix and one pass o
         for (int t = 0; t < NT; t++) acc[k][t] = 0;
       uint32_t xa = x0;
       for (uint32_t seg = 0; seg < nseg; seg++) {
-        if (!bar_wait(&full[slot], phase)) return false;
+        if (!bar_wait_warp(&full[slot], phase)) return false;
         const uint32_t sa = smem_addr(ring) + slot * (kRows * slot_row);
         const uint32_t n = seg == nseg - 1 ? last_n : seg_n;
         uint32_t at[RT];

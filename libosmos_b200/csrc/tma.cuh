@@ -65,8 +65,9 @@ __device__ __forceinline__ uint64_t global_ns() {
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
 }
-// true when the phase of `parity` has completed; gives up kWaitLimitNs after its first look
-__device__ __forceinline__ bool bar_wait(uint64_t* bar, uint32_t parity) {
+// true when the phase of `parity` has completed; gives up `limit` ns after its first look. The clock is the thread's own: of
+// a warp's lanes some may give up where the phase completes in time for others.
+__device__ __forceinline__ bool bar_wait(uint64_t* bar, uint32_t parity, uint64_t limit = kWaitLimitNs) {
   const uint32_t a = smem_addr(bar);
   uint64_t t0 = 0;
   for (uint32_t spin = 0;; spin++) {
@@ -78,10 +79,16 @@ __device__ __forceinline__ bool bar_wait(uint64_t* bar, uint32_t parity) {
         : "memory");
     if (done) return true;
     if (spin == 0) t0 = global_ns();
-    else if (global_ns() - t0 > kWaitLimitNs) return false;
+    else if (global_ns() - t0 > limit) return false;
   }
 }
-// the same for a wait that is expected to be long (an epilogue's, through a whole K loop): the look itself may suspend the
+// the same for a whole warp, with one outcome for all its lanes: when one gives up, all do. What follows a wait that ran out
+// - leaving for a block's barrier, or going on to the warp's next meeting - is then every lane's, and no lane waits at
+// either for one that took the other way.
+__device__ __forceinline__ bool bar_wait_warp(uint64_t* bar, uint32_t parity, uint64_t limit = kWaitLimitNs) {
+  return __all_sync(0xFFFFFFFFu, bar_wait(bar, parity, limit));
+}
+// bar_wait for a wait that is expected to be long (an epilogue's, through a whole K loop): the look itself may suspend the
 // warp for up to 10 us at a time - it still returns when the phase completes - so that waiting costs no issue slots
 __device__ __forceinline__ bool bar_wait_long(uint64_t* bar, uint32_t parity) {
   const uint32_t a = smem_addr(bar);
