@@ -34,6 +34,7 @@
 #include <cstring>
 
 #include "common.cuh"
+#include "tma.cuh"
 
 namespace osmos {
 namespace fp4_tc {
@@ -382,7 +383,7 @@ __global__ void __launch_bounds__(kThreads, 1) fp4_tc_kernel(const Args a, const
     const uint32_t row = 32u * warp + lane;  // this thread's weight row of the tile = its TMEM lane
     const uint32_t lane_base = tmem + ((32u * warp) << 16);
     float* y = a.y + (uint64_t) c0 * a.ys + row0 + row;
-    if (bar_wait(&sh.acc_full, 0)) {
+    if (tma::bar_wait_warp(&sh.acc_full, 0)) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       for (uint32_t col = 0; col < n_mma; col += 32) {
         uint32_t r[32];

@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(W * kWarp, (W <= 12 ? 2 : 1)) plain_dense_kern
     const uint32_t u = u_lo + warp + i * W;
     if (u >= u_hi) break;
     const uint32_t slot = i % S;
-    if (!bar_wait(&full[warp][slot], (i / S) & 1u)) {  // a copy never landed: report it and leave
+    if (!bar_wait_warp(&full[warp][slot], (i / S) & 1u)) {  // a copy never landed: report it and leave
       if (lane == 0) atomicOr(a.status, 1u);
       break;
     }

@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(kThreads, 1) lane_ring_kernel(const Args a) {
     bool ok = true;
     for (uint32_t ss = 0; ss < TS; ss++) {
       const uint32_t q = n * TS + ss, slot = q % S;
-      if (!bar_wait(&full[warp][slot], (q / S) & 1u)) {  // a copy never landed: report it and leave
+      if (!bar_wait_warp(&full[warp][slot], (q / S) & 1u)) {  // a copy never landed: report it and leave
         ok = false;
         break;
       }

@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(kThreads, 1) lane_rows_kernel(const Args a) {
     __syncwarp();
     fetch(n + 1, xq, xd);
     const uint32_t slot = n % kSlots;
-    if (!bar_wait(&full[warp][slot], (n / kSlots) & 1u)) {  // a copy never landed: report it and leave
+    if (!bar_wait_warp(&full[warp][slot], (n / kSlots) & 1u)) {  // a copy never landed: report it and leave
       if (lane == 0) atomicOr(a.status, 1u);
       break;
     }

@@ -369,7 +369,7 @@ __global__ void __launch_bounds__(kThreads, 1) lane_staged_kernel(const Args a) 
       for (uint32_t q = blockIdx.x; q < items; q += gridDim.x, it++) {
         const uint32_t stage = it % S, use = it / S;
         bool ok = true;
-        if (use > 0) ok = bar_wait(&empty[stage], (use - 1u) & 1u);  // the stage's last readers are done with it
+        if (use > 0) ok = bar_wait_warp(&empty[stage], (use - 1u) & 1u);  // the stage's last readers are done with it
         uint32_t m, grp, tile;
         decode_item(q, m, grp, tile);
         const bool aligned = ok && issue(m, grp, tile, stage);
@@ -397,7 +397,7 @@ __global__ void __launch_bounds__(kThreads, 1) lane_staged_kernel(const Args a) 
       }
       for (uint32_t q = blockIdx.x; q < items; q += gridDim.x, it++) {
         const uint32_t stage = it % S, use = it / S;
-        if (!bar_wait(&full[stage], use & 1u)) s_fail = 1;  // a copy never landed
+        if (!bar_wait_warp(&full[stage], use & 1u)) s_fail = 1;  // a copy never landed
         const uint32_t st = smem_addr(smem + p.stage0 + stage * p.stage_bytes);
         const Meta meta = metas[stage];
         const uint32_t live = meta.live, tile_sb = meta.trows * nsb;

@@ -552,13 +552,13 @@ __global__ void __launch_bounds__(kThreads, 1) mm_tc_kernel(const Args a, const 
     if (!bar_wait_long(&sh.done, 0)) {
       // (the K loop's own waits are 0.2 s each and can queue up: look again while nobody has given up)
       bool landed = false;
-      for (uint32_t tries = 0; tries < 25u && !sh.fail && !landed; tries++) landed = bar_wait_long(&sh.done, 0);
+      for (uint32_t tries = 0; tries < 25u && !__any_sync(0xFFFFFFFFu, sh.fail) && !landed; tries++) landed = bar_wait_long(&sh.done, 0);
       if (!landed) sh.fail = 1;
     }
     // (nobody else writes the word once the last product has landed or been given up: after this barrier every
     // epilogue thread reads the same value, so all of them or none take the barriers below)
     if constexpr (EPI == kGatedMean) asm volatile("bar.sync 2, %0;" ::"n"(kEpiWarps * kWarp) : "memory");
-    if (!sh.fail) {
+    if (!__any_sync(0xFFFFFFFFu, sh.fail)) {  // (one answer a warp: tensor memory is read by whole warps)
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       for (uint32_t acc = 0; acc < n_acc; acc++) {
 #pragma unroll 1

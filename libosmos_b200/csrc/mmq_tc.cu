@@ -25,6 +25,7 @@
 #include "common.cuh"
 #include "mmq_tc_api.h"
 #include "osmos_b200/mmq.h"
+#include "tma.cuh"
 
 namespace osmos {
 namespace mmq_tc {
@@ -189,7 +190,7 @@ __global__ void __launch_bounds__(kThreads, 1) q4k_tc_kernel(const Args a) {
     // the trip to memory is over when the producers want the bytes
     for (uint32_t it = 0; it < nb; it++) {
       const uint32_t rs = it % kRawStages, use = it / kRawStages;
-      if (use > 0 && !bar_wait(&sh.raw_empty[rs], (use - 1) & 1u)) {
+      if (use > 0 && !tma::bar_wait_warp(&sh.raw_empty[rs], (use - 1) & 1u)) {
         sh.fail = 1;
         break;
       }
@@ -213,7 +214,7 @@ __global__ void __launch_bounds__(kThreads, 1) q4k_tc_kernel(const Args a) {
     const uint32_t pt = tid - kFirstProdWarp * kWarp;  // 0 .. kProdThreads - 1
     for (uint32_t it = 0; it < nb; it++) {
       const uint32_t stage = it % kStages, use = it / kStages;
-      if (use > 0 && !bar_wait(&sh.empty[stage], (use - 1) & 1u)) {
+      if (use > 0 && !tma::bar_wait_warp(&sh.empty[stage], (use - 1) & 1u)) {
         sh.fail = 1;
         break;
       }
@@ -247,7 +248,7 @@ __global__ void __launch_bounds__(kThreads, 1) q4k_tc_kernel(const Args a) {
       // A: the step's raw blocks have landed; a task = (row, pair of groups): 32 bytes of nibbles -> the low nibbles'
       // group and the high nibbles' group
       const uint32_t rs = it % kRawStages;
-      if (!bar_wait(&sh.raw_full[rs], (it / kRawStages) & 1u)) {
+      if (!tma::bar_wait_warp(&sh.raw_full[rs], (it / kRawStages) & 1u)) {
         sh.fail = 1;
         break;
       }
@@ -275,9 +276,11 @@ __global__ void __launch_bounds__(kThreads, 1) q4k_tc_kernel(const Args a) {
   } else if (warp == (uint32_t) kIssuerWarp) {
     // ================= issuer =================
     uint32_t acc_it = 0;
-    for (uint32_t it = 0; it < nb && !sh.fail; it++) {
+    bool ok = true;
+    for (uint32_t it = 0; it < nb && ok; it++) {
       const uint32_t stage = it % kStages, use = it / kStages;
-      if (!bar_wait(&sh.full[stage], use & 1u)) {
+      // (one vote: whether another warp has failed and whether the wait ran out is the same for every lane)
+      if (!__all_sync(0xFFFFFFFFu, !sh.fail && bar_wait(&sh.full[stage], use & 1u))) {
         sh.fail = 1;
         break;
       }
@@ -286,8 +289,8 @@ __global__ void __launch_bounds__(kThreads, 1) q4k_tc_kernel(const Args a) {
       const uint32_t sa = smem_addr(smem + stage * kStageBytes), sb = sa + kGroups * kTileBytes;
       for (uint32_t g = 0; g < (uint32_t) kGroups; g++, acc_it++) {
         const uint32_t acc = acc_it % kAccs, ause = acc_it / kAccs;
-        if (ause > 0 && !bar_wait(&sh.acc_empty[acc], (ause - 1) & 1u)) {
-          sh.fail = 1;
+        if (ause > 0 && !tma::bar_wait_warp(&sh.acc_empty[acc], (ause - 1) & 1u)) {
+          sh.fail = 1, ok = false;
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -304,7 +307,7 @@ __global__ void __launch_bounds__(kThreads, 1) q4k_tc_kernel(const Args a) {
         }
         __syncwarp();
       }
-      if (sh.fail) break;
+      if (!ok) break;
       if (lane == 0)  // the stage's operands are free once these eight have run
         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                          smem_addr(&sh.empty[stage]))
@@ -367,7 +370,7 @@ __global__ void __launch_bounds__(kThreads, 1) q4k_tc_kernel(const Args a) {
       block_of(it, p, last);
       // the row's scales of this block: d sc and dmin m for its 8 groups, from the head the producers kept in the stage
       // (read once the stage is full: this thread may be a whole step ahead of the producers)
-      if (!bar_wait(&sh.full[stage], (it / kStages) & 1u)) {
+      if (!tma::bar_wait_warp(&sh.full[stage], (it / kStages) & 1u)) {
         sh.fail = 1;
         break;
       }

@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(kThreads, 1) mv_staged_kernel(const Args a) {
     const uint32_t u = u_lo + warp + i * kWarps;
     if (u >= u_hi) break;
     const uint32_t slot = i % S;
-    if (!bar_wait(&full[warp][slot], (i / S) & 1u)) {  // a copy never landed: report it and leave
+    if (!bar_wait_warp(&full[warp][slot], (i / S) & 1u)) {  // a copy never landed: report it and leave
       if (lane == 0) atomicOr(a.status, 1u);
       break;
     }
@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(kThreads, 1) mv_regx_kernel(const Args a) {
     const uint32_t u = u_lo + warp + i * kWarps;
     if (u >= u_hi) break;
     const uint32_t slot = i % S;
-    if (!bar_wait(&full[warp][slot], (i / S) & 1u)) {  // a copy never landed: report it and leave
+    if (!bar_wait_warp(&full[warp][slot], (i / S) & 1u)) {  // a copy never landed: report it and leave
       if (lane == 0) atomicOr(a.status, 1u);
       break;
     }

@@ -88,9 +88,9 @@ __device__ __forceinline__ bool bar_wait(uint64_t* bar, uint32_t parity, uint64_
 __device__ __forceinline__ bool bar_wait_warp(uint64_t* bar, uint32_t parity, uint64_t limit = kWaitLimitNs) {
   return __all_sync(0xFFFFFFFFu, bar_wait(bar, parity, limit));
 }
-// bar_wait for a wait that is expected to be long (an epilogue's, through a whole K loop): the look itself may suspend the
+// bar_wait_warp for a wait that is expected to be long (an epilogue's, through a whole K loop): the look itself may suspend the
 // warp for up to 10 us at a time - it still returns when the phase completes - so that waiting costs no issue slots
-__device__ __forceinline__ bool bar_wait_long(uint64_t* bar, uint32_t parity) {
+__device__ __forceinline__ bool bar_wait_long(uint64_t* bar, uint32_t parity, uint64_t limit = kWaitLimitNs) {
   const uint32_t a = smem_addr(bar);
   uint64_t t0 = 0;
   for (uint32_t spin = 0;; spin++) {
@@ -100,9 +100,9 @@ __device__ __forceinline__ bool bar_wait_long(uint64_t* bar, uint32_t parity) {
         : "=r"(done)
         : "r"(a), "r"(parity)
         : "memory");
-    if (done) return true;
+    if (__all_sync(0xFFFFFFFFu, done)) return true;
     if (spin == 0) t0 = global_ns();
-    else if (global_ns() - t0 > kWaitLimitNs) return false;
+    else if (__any_sync(0xFFFFFFFFu, global_ns() - t0 > limit)) return false;
   }
 }
 // global -> this block's shared memory, completion counted on `bar`; both addresses 16-byte aligned, bytes a multiple of 16
