@@ -64,11 +64,12 @@ bool mv_fp4_tok(const void *const *w, const int32_t *cnt, const int32_t *xrow, u
                 uint32_t cols, const float *x, uint32_t xs, float *y, uint32_t ys, void *stream);
 
 /* Not in the reference. The matvecs have kernels that stage rows through shared memory with bulk copies (16-byte aligned w
-   and x, columns in 256s; for all but seven types rows whose bytes are a multiple of 16, x and a ring of rows fitting
-   shared memory) and a generic one for every other shape: the same bits. mv_set_staged(0) forces the generic kernel (the
+   and x, columns in 256s; for all types but Q4_0, Q8_0, Q4_K, Q5_K, Q6_K, IQ4_XS and MXFP4 rows whose bytes are a multiple
+   of 16, x and a ring of rows fitting shared memory) and a generic one for every other shape: the same bits. mv_set_staged(0) forces the generic kernel (the
    tests compare them). mv_status() reads and clears the staged kernels' record on the current device (it synchronizes):
    bit 0 = a bulk copy never landed within the kernel's wait limit, whose rows were not written; bit 1 = a grouped matrix
-   did not start on 16 bytes though its rows are whole 16-byte pieces, and was left alone. */
+   was left alone: of those seven types one on an odd byte (MXFP4 may start anywhere), of the others one not on 16 bytes in a
+   call whose shape the staged kernel takes. */
 void mv_set_staged(int on);
 uint32_t mv_status(void);
 

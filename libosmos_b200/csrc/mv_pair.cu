@@ -415,12 +415,11 @@ __global__ void __launch_bounds__(kThreads, 1) mv_pair_kernel(const Args a) {
       xin = a.x + (uint64_t) (m / a.x_div) * a.x_mat, yout = a.y + (uint64_t) m * a.rows, live = 1;
     }
     me.mat = a.wt[m];
-    if ((uintptr_t) me.mat & 15u) {  // such a matrix cannot be copied in bulk:
-      if (me.row_bytes % 16u == 0) {  // reported, its rows left alone
+    if ((uintptr_t) me.mat & 15u) {  // such a matrix cannot be copied in bulk: read where it lies
+      if (((uintptr_t) me.mat & 1u) && T != QTYPE_MXFP4) {  // (but for MXFP4's bytes a block is read by halves: reported, its rows left alone)
         if (tid == 0) atomicOr(a.status, 2u);
         return;
       }
-      // where an expert's bytes need not be whole 16-byte pieces, its matrix need not start on one: read where it lies
       rows_in_place<T>(me.mat, me.row_bytes, a, xin, yout, live);
       return;
     }

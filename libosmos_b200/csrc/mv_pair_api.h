@@ -13,7 +13,7 @@ using mvs::Request;
 // launch was refused
 int try_launch(uint32_t type, const Request& r, void* stream);
 // the current device's status word, read and cleared (synchronizes): bit 0 a copy never landed, bit 1 a grouped
-// entry's matrix was not 16-byte aligned (its rows were not written)
+// entry's matrix started on an odd byte (its rows were not written; MXFP4's are)
 uint32_t read_status();
 
 }  // namespace mvp

@@ -202,6 +202,44 @@ def test_mv_grouped_matrices_anywhere(lib, dev, oracle, name, cols, off):
     assert lib.mv_status() == 0
 
 
+def _grouped_at(lib, dev, oracle, name, cols, rows, off, cnt=(3, 8, 1)):
+    """mv_group_tok (up to eight tokens) over matrices that start `off` bytes past a multiple of 16: y, and the oracle's"""
+    tid, cnt = TYPES[name], list(cnt)
+    rng = synth.rng_for(19, tid, cols, off)
+    mats = [synth.random_tensor(tid, rows, cols, rng) for _ in cnt]
+    step = (mats[0].size + 15) // 16 * 16 + 16
+    pool = np.zeros(step * len(cnt) + 16, np.uint8)
+    for m, w in enumerate(mats):
+        pool[m * step + off:m * step + off + w.size] = w.reshape(-1)
+    xrow = np.cumsum([0] + cnt[:-1]).astype(np.int32)
+    x = rng.standard_normal((sum(cnt), cols)).astype(np.float32)
+    pd = to_dev(pool, dev)
+    table = pointer_table(pd, [m * step + off for m in range(len(cnt))], dev)
+    y = torch.full((sum(cnt), rows), -3.0, dtype=torch.float32, device=dev)
+    lib.mv_status()
+    assert lib.mv_group_tok(tid, ptr(table), ptr(to_dev(np.array(cnt, np.int32), dev)), ptr(to_dev(xrow, dev)), len(cnt), 8, rows, cols,
+                            ptr(to_dev(x, dev)), cols, ptr(y), rows, None)
+    sync()
+    want = np.concatenate([oracle.mv_rows(tid, w, rows, cols, x[int(r):int(r) + c]) for w, r, c in zip(mats, xrow, cnt)])
+    return y.cpu().numpy(), want
+
+
+@pytest.mark.parametrize("name,cols", [("Q4_0", 512), ("Q8_0", 512), ("Q8_0", 3584), ("Q4_K", 768), ("Q4_K", 4864), ("Q5_K", 512), ("Q5_K", 4352)])
+@pytest.mark.parametrize("off", [2, 8])
+def test_mv_grouped_whole_rows_anywhere(lib, dev, oracle, name, cols, off):
+    """nor need matrices whose rows are whole 16-byte pieces - short rows, and rows too long for the staged kernel's ring beside
+    eight tokens, which were always computed where they lie"""
+    got, want = _grouped_at(lib, dev, oracle, name, cols, 37, off)
+    assert same_bits(got, want) and lib.mv_status() == 0
+
+
+def test_mv_grouped_odd_byte_reported(lib, dev, oracle):
+    """a matrix on an odd byte, whose halves cannot be read, is reported and left alone"""
+    for name in ("Q4_0", "Q4_K", "Q6_K"):
+        got, _want = _grouped_at(lib, dev, oracle, name, 512, 21, 5)
+        assert (got == -3.0).all() and lib.mv_status() == 2
+
+
 @pytest.mark.parametrize("name", ["Q4_0", "IQ3_XXS", "Q4_K", "MXFP4"])
 def test_mv_strided_many_tokens(lib, dev, oracle, name):
     tid = TYPES[name]
