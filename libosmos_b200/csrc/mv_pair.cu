@@ -26,6 +26,7 @@
 
 #include "decode.cuh"
 #include "dispatch.cuh"
+#include "mv_room.h"
 #include "packed.cuh"
 #include "tma.cuh"
 
@@ -508,16 +509,10 @@ int launch(const Request& r, const Device* dev, cudaStream_t s) {
   a.wt = (const uint8_t* const*) r.wt, a.cnt = r.cnt, a.xrow = r.xrow, a.x_mat = r.x_mat, a.x_div = r.x_div;
   // the tokens a pass holds beside rings of two slots; shorter slots where they save a pass over the weights (4096 x 4096
   // MXFP4, 8 tokens: 26.9 us in two passes of slots of eight stretches)
-  uint32_t best = 0;
-  for (uint32_t seg = kSegOf<RT>; seg; seg >>= 1) {
-    const uint32_t rings = 2u * kWarps * 2u * RT * slot_row_bytes<T>(r.cols, seg);
-    if (rings + 128u + x_bytes(1, r.cols) > kLimit) continue;
-    uint32_t fit = (kLimit - rings - 128u) / x_bytes(1, r.cols);
-    if (fit > kMaxTok) fit = kMaxTok;
-    const uint32_t passes = (r.n_tok + fit - 1) / fit;
-    if (!best || passes < best) best = passes, a.seg = seg, a.fit = fit;
-  }
-  if (!best) return 0;
+  const mv_room::Passes room = mv_room::pair_passes(kLimit, kSegOf<RT>, kMaxTok, r.n_tok, r.cols,
+                                                    [&](uint32_t seg) { return 2u * kWarps * 2u * RT * slot_row_bytes<T>(r.cols, seg); });
+  if (!room.seg) return 0;
+  a.seg = room.seg, a.fit = room.fit;
   a.smem = kLimit;
   const uint32_t units = (r.rows + 2 * RT - 1) / (2 * RT);
   dim3 grid((uint32_t) dev->sms);
@@ -567,7 +562,7 @@ int by_shape(const Request& r, cudaStream_t s) {
 
 int try_launch(uint32_t type, const Request& r, void* stream) {
   if (!r.rows || !r.n_tok || r.n_tok > kMaxTok || !r.cols || r.cols % 256) return 0;
-  if ((uint64_t) r.cols * 2u > 0x7FFFFFFFull || r.rows > 0x7FFFFFFFu) return 0;  // (a row's bytes and a unit's rows in 32 bits)
+  if (r.rows > 0x7FFFFFFFu) return 0;  // (a unit's rows in 32 bits; a row's bytes are where a token's x fits)
   if (r.wt) {  // every entry's x row starts on 16 bytes when the first does and the strides are whole words of 16
     if (((uintptr_t) r.x & 15u) || r.xs % 4 || r.x_mat % 4 || !r.n_entries || r.n_entries > 65535u) return 0;
   } else if ((((uintptr_t) r.w | (uintptr_t) r.x) & 15u) || (r.n_tok > 1 && r.xs % 4)) {

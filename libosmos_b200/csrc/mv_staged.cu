@@ -19,6 +19,7 @@
 
 #include "decode.cuh"
 #include "dispatch.cuh"
+#include "mv_room.h"
 #include "tma.cuh"
 
 namespace osmos {
@@ -465,11 +466,8 @@ int launch(const Request& r, const Device* dev, uint32_t slots, uint32_t cnt_lo,
 // as deep a ring as fits beside n_tok tokens' x (0 tokens: x in registers)
 template <uint32_t T>
 uint32_t slots_for(uint32_t rw, uint32_t x_tokens, uint32_t cols) {
-  const uint32_t row_bytes = cols / Fmt<T>::values * Fmt<T>::bytes, budget = kSmemLimit<T> - 16u;
-  const uint32_t x_bytes = (x_tokens * cols * 4u + 127u) & ~127u;
-  if (x_bytes >= budget) return 0;
-  const uint32_t n = (budget - x_bytes) / (kWarps * rw * row_bytes);
-  return n > (uint32_t) kMaxSlots ? (uint32_t) kMaxSlots : n;
+  const uint64_t row_bytes = (uint64_t) (cols / Fmt<T>::values) * Fmt<T>::bytes;
+  return mv_room::staged_slots(kSmemLimit<T> - 16u, kWarps, (uint32_t) kMaxSlots, rw * row_bytes, x_tokens, cols);
 }
 
 // what mv_pair.cu takes: every shape of the first three types, the grouped forms of all seven
