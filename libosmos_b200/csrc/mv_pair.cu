@@ -53,11 +53,19 @@ struct Args {
   uint32_t fit;       // tokens whose x a pass holds
   uint32_t smem;      // dynamic shared memory, bytes: x of a pass, then the rings
   uint32_t* status;
-  // grouped forms: blockIdx.y is the entry
+  // grouped forms: a block finds its entry and its part of that entry's rows (find_entry)
   const uint8_t* const* wt;
   const int32_t *cnt, *xrow;
-  uint32_t x_mat, x_div;
+  uint32_t n_entries, x_mat, x_div;
+  uint32_t parts;  // blocks an entry
+  uint32_t wave;   // blocks that the live entries are dealt anew over when they have fewer; 0: a block has the entry of its place
 };
+
+// parts of an entry's units, `most` at most: as few as leave a warp of the largest no more units than that many would
+__host__ __device__ inline uint32_t even_parts(uint32_t units, uint32_t most) {
+  const uint32_t rounds = (units + kWarps * most - 1) / (kWarps * most);
+  return (units + kWarps * rounds - 1) / (kWarps * rounds);
+}
 
 // the eight bytes sh / 8 bytes into the aligned word at `al`, out of it and the two after it
 __device__ __forceinline__ uint2 lds_8_bytes(uint32_t al, uint32_t sh) {
@@ -361,24 +369,71 @@ struct Warp {  // one warp's view of a block's work on one matrix and one pass o
 };
 
 // a block's share of a matrix that does not start on 16 bytes: mv.cu's sums straight from global memory, a row a warp, a token
-// at a time
+// at a time. (By value: with the kernel's arguments taken by reference every thread of the kernel copied them to its stack first -
+// 12 Q4_K entries of 2048 x 512 at a token each 15.1 us, 12.7 so.)
 template <uint32_t T>
-__device__ __noinline__ void rows_in_place(const uint8_t* mat, uint32_t row_bytes, const Args& a, const float* x, float* y, uint32_t live) {
-  const uint32_t lane = threadIdx.x % kWarp, warp = threadIdx.x / kWarp, lo = (uint32_t) ((uint64_t) blockIdx.x * a.rows / gridDim.x),
-                 hi = (uint32_t) ((uint64_t) (blockIdx.x + 1) * a.rows / gridDim.x);
+__device__ __noinline__ void rows_in_place(const uint8_t* mat, uint32_t row_bytes, uint32_t cols, uint32_t lo, uint32_t hi, const float* x, uint32_t xs,
+                                           float* y, uint32_t ys, uint32_t live) {
+  const uint32_t lane = threadIdx.x % kWarp, warp = threadIdx.x / kWarp;
   for (uint32_t r = lo + warp; r < hi; r += kWarps)
     for (uint32_t t = 0; t < live; t++) {
       float s = 0.0f;
-      for (uint32_t c = lane; c < a.cols / kChunk; c += kWarp) {
+      for (uint32_t c = lane; c < cols / kChunk; c += kWarp) {
         float v[kChunk];
         decode8<T>(mat + (uint64_t) r * row_bytes + (c / Fmt<T>::chunks) * Fmt<T>::bytes, (int) (c % Fmt<T>::chunks), v, Grids{});
-        const float* xc = x + (uint64_t) t * a.xs + c * kChunk;
+        const float* xc = x + (uint64_t) t * xs + c * kChunk;
 #pragma unroll
         for (int j = 0; j < kChunk; j++) s = __fmaf_rn(v[j], xc[j], s);
       }
       s = xor_tree<kWarp>(s);
-      if (lane == 0) y[(uint64_t) t * a.ys + r] = s;
+      if (lane == 0) y[(uint64_t) t * ys + r] = s;
     }
+}
+
+// A grouped launch's block finds its work. The blocks go to the entries that have tokens, `parts` to each in turn; where the live
+// ones are so few that this leaves SMs idle - the host knows how many entries there are, not how many have tokens - a wave of
+// blocks is dealt to them anew, down to a unit a warp (four live of 64, one token, Q6_K 2048 x 7168: 71.6 us without, 21.9 so; the
+// kernels before this one 37). Every thread of the block calls it; false: a block too many. The look through the counts is two
+// meetings of the block's warps (128 live of 128, Q4_K 1536 x 4096: 251.5 us without, 258 so): not for few entries, nor for more than
+// the block has threads.
+struct Work {
+  const uint8_t* mat;
+  uint32_t m, part, parts;
+  int32_t cnt, xrow;  // (by token)
+};
+__device__ __forceinline__ bool find_entry(const Args& a, uint32_t units, Work& f) {
+  f.parts = a.parts;
+  if (a.wave) {
+    __shared__ uint32_t s_live[kWarps];
+    __shared__ Work s_found;
+    const uint32_t tid = threadIdx.x, lane = tid % kWarp, warp = tid / kWarp;
+    Work mine{nullptr, tid, 0, 0, 0, 0};
+    if (tid < a.n_entries) mine.cnt = a.cnt[tid], mine.xrow = a.xrow[tid], mine.mat = a.wt[tid];  // (one trip for all the tables)
+    const uint32_t on = __ballot_sync(0xFFFFFFFFu, mine.cnt > 0);
+    if (lane == 0) s_live[warp] = __popc(on);
+    __syncthreads();
+    uint32_t live = 0, before = 0;
+#pragma unroll
+    for (uint32_t w = 0; w < (uint32_t) kWarps; w++) {
+      if (w == warp) before = live;
+      live += s_live[w];
+    }
+    uint32_t parts = a.parts;
+    if (live && live * parts < a.wave) {
+      const uint32_t most = units / kWarps, each = a.wave / live, to = each < most ? each : most;
+      if (to > parts) parts = even_parts(units, to);
+    }
+    const uint32_t m = blockIdx.x / parts;
+    if (m >= live) return false;
+    if (mine.cnt > 0 && before + __popc(on & ((1u << lane) - 1u)) == m) s_found = mine;
+    __syncthreads();
+    f = s_found;
+    f.parts = parts, f.part = blockIdx.x - m * parts;
+    return true;
+  }
+  f.m = blockIdx.x / a.parts, f.part = blockIdx.x - f.m * a.parts, f.mat = a.wt[f.m], f.cnt = 1, f.xrow = 0;
+  if (a.cnt) f.cnt = a.cnt[f.m], f.xrow = a.xrow[f.m];
+  return f.cnt > 0;
 }
 
 template <uint32_t T, int RT, bool GROUP>
@@ -398,6 +453,7 @@ __global__ void __launch_bounds__(kThreads, 1) mv_pair_kernel(const Args a) {
   const float* xin = a.x;
   float* yout = a.y;
   uint32_t live = a.n_tok;
+  [[maybe_unused]] uint32_t part, parts;  // (grouped: the block's share of its entry's rows)
   if (me.lane == 0) {
     for (uint32_t s = 0; s < kMaxSlots; s++) bar_init(&full[warp][s], 2 * RT);
     bar_init_fence();
@@ -406,27 +462,28 @@ __global__ void __launch_bounds__(kThreads, 1) mv_pair_kernel(const Args a) {
   if constexpr (GROUP) {
     pdl_wait();  // (a dependent launch: the tables and x may be the output of the kernel ahead)
     pdl_launch_next();
-    const uint32_t m = blockIdx.y;
+    Work f;
+    if (!find_entry(a, (a.rows + 2 * RT - 1) / (2 * RT), f)) return;  // (the whole block)
+    part = f.part, parts = f.parts, me.mat = f.mat;
     if (a.cnt) {
-      const int32_t c = a.cnt[m];
-      if (c <= 0) return;  // (the whole block)
-      const uint64_t r0 = (uint64_t) a.xrow[m];
-      xin = a.x + r0 * a.xs, yout = a.y + r0 * a.ys, live = (uint32_t) c < a.n_tok ? (uint32_t) c : a.n_tok;
+      const uint64_t r0 = (uint64_t) f.xrow;
+      xin = a.x + r0 * a.xs, yout = a.y + r0 * a.ys, live = (uint32_t) f.cnt < a.n_tok ? (uint32_t) f.cnt : a.n_tok;
     } else {
-      xin = a.x + (uint64_t) (m / a.x_div) * a.x_mat, yout = a.y + (uint64_t) m * a.rows, live = 1;
+      xin = a.x + (uint64_t) (f.m / a.x_div) * a.x_mat, yout = a.y + (uint64_t) f.m * a.rows, live = 1;
     }
-    me.mat = a.wt[m];
     if ((uintptr_t) me.mat & 15u) {  // such a matrix cannot be copied in bulk: read where it lies
       if (((uintptr_t) me.mat & 1u) && T != QTYPE_MXFP4) {  // (but for MXFP4's bytes a block is read by halves: reported, its rows left alone)
         if (tid == 0) atomicOr(a.status, 2u);
         return;
       }
-      rows_in_place<T>(me.mat, me.row_bytes, a, xin, yout, live);
+      rows_in_place<T>(me.mat, me.row_bytes, a.cols, (uint32_t) ((uint64_t) part * a.rows / parts), (uint32_t) ((uint64_t) (part + 1) * a.rows / parts),
+                       xin, a.xs, yout, a.ys, live);
       return;
     }
   }
   const uint32_t units = (a.rows + 2 * RT - 1) / (2 * RT);
-  me.u0 = (uint32_t) ((uint64_t) blockIdx.x * units / gridDim.x) + warp, me.u_hi = (uint32_t) ((uint64_t) (blockIdx.x + 1) * units / gridDim.x);
+  if constexpr (GROUP) me.u0 = (uint32_t) ((uint64_t) part * units / parts) + warp, me.u_hi = (uint32_t) ((uint64_t) (part + 1) * units / parts);
+  else me.u0 = (uint32_t) ((uint64_t) blockIdx.x * units / gridDim.x) + warp, me.u_hi = (uint32_t) ((uint64_t) (blockIdx.x + 1) * units / gridDim.x);
   // the tokens in as few passes as their x allows, evenly; the rings take the rest of the block's shared memory
   const uint32_t passes = (live + a.fit - 1) / a.fit, per = (live + passes - 1) / passes;
   const uint32_t ring_off = (x_bytes(per, a.cols) + 127u) & ~127u, slot_bytes = 2 * RT * me.slot_row;
@@ -520,11 +577,19 @@ int launch(const Request& r, const Device* dev, cudaStream_t s) {
   if constexpr (GROUP) {
     // an entry's rows over a few blocks, about four units a warp each and at most eight - more, down to a unit a warp, where
     // the entries are too few for three blocks an SM (one token's four MXFP4 experts of 1536 x 4096, the
-    // layer: 154 us with the first rule alone, 70 with this one; the staged kernel 162)
+    // layer: 154 us with the first rule alone, 70 with this one; the staged kernel 162), but a quarter fewer or less where their warps
+    // take no more units each for it (68 experts top-3 of that shape, six tokens: 197 us a layer with 23 blocks an entry, whose
+    // warps take one unit or two, 173 with 12; staged 172)
+    const uint32_t sms = (uint32_t) dev->sms;
     const uint32_t some = units / (4u * kWarps) > 8u ? 8u : units / (4u * kWarps), most = units / kWarps;
-    const uint32_t want = (3u * (uint32_t) dev->sms + r.n_entries - 1) / r.n_entries, more = want < most ? want : most;
-    grid.x = some > more ? some : more, grid.y = r.n_entries;
-    if (grid.x < 1u) grid.x = 1u;
+    const uint32_t want = (3u * sms + r.n_entries - 1) / r.n_entries, more = want < most ? want : most;
+    a.parts = some > more ? some : more;
+    if (a.parts < 1u) a.parts = 1u;
+    if (const uint32_t even = even_parts(units, a.parts); more > some && 4u * even <= 3u * a.parts) a.parts = even;
+    const uint64_t blocks = (uint64_t) r.n_entries * a.parts;
+    if (blocks > 0x7FFFFFFFull) return 0;
+    grid.x = (uint32_t) blocks, a.n_entries = r.n_entries;
+    if (r.cnt && r.n_entries > 12u && r.n_entries <= (uint32_t) kThreads) a.wave = grid.x < sms ? grid.x : sms;
   }
   static bool sized[64] = {};  // (one record a template instance, one flag a device)
   auto kernel = mv_pair_kernel<T, RT, GROUP>;

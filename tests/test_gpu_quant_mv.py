@@ -179,6 +179,44 @@ def test_mv_paired_lanes_grouped(lib, dev, oracle, name, cols, rows):
     assert lib.mv_status() == 0
 
 
+@pytest.mark.parametrize("name", ["Q8_0", "Q4_K", "Q6_K", "MXFP4"])
+@pytest.mark.parametrize("entries,live,rows,cols", [
+    (13, [12], 450, 512),                         # one live entry, the last, over as many blocks as its rows allow
+    (64, [0, 31, 32, 63], 1030, 256),             # a few, across the warps that look for them
+    (64, range(64), 130, 256),                    # all of them
+    (40, range(0, 40, 2), 515, 512),              # blocks enough as they are
+    (20, [], 64, 256),                            # none
+    (512, [0, 511], 70, 256), (513, [0, 511, 512], 70, 256)])  # as many as a block has threads, and one more
+def test_mv_paired_lanes_few_live(lib, dev, oracle, name, entries, live, rows, cols):
+    """tables of many entries few of which have tokens: the live ones' rows, nobody else's; and rows of x in another order"""
+    tid, live = TYPES[name], list(live)
+    rng = synth.rng_for(22, tid, entries, rows, cols)
+    mats = [synth.random_tensor(tid, rows, cols, rng) for _ in range(min(entries, 5))]  # (the entries share a few matrices)
+    step = (mats[0].size + 15) // 16 * 16
+    pool = np.zeros(step * len(mats), np.uint8)
+    for m, w in enumerate(mats):
+        pool[m * step:m * step + w.size] = w.reshape(-1)
+    cnt = np.zeros(entries, np.int32)
+    cnt[live] = [1 + i % 4 for i in range(len(live))]
+    xrow = (cnt.sum() - np.cumsum(cnt)).astype(np.int32)  # (the last entry's rows first)
+    total = max(1, int(cnt.sum()))
+    x = rng.standard_normal((total, cols)).astype(np.float32)
+    pd, xd = to_dev(pool, dev), to_dev(x, dev)
+    table = pointer_table(pd, [m % len(mats) * step for m in range(entries)], dev)
+    cd, rd = to_dev(cnt, dev), to_dev(xrow, dev)
+    lib.mv_status()
+    for max_cnt in (8, 1):
+        y = torch.full((total, rows), -3.0, dtype=torch.float32, device=dev)
+        assert lib.mv_group_tok(tid, ptr(table), ptr(cd), ptr(rd), entries, max_cnt, rows, cols, ptr(xd), cols, ptr(y), rows, None)
+        sync()
+        want = np.full((total, rows), -3.0, np.float32)
+        for m in live:
+            r = slice(int(xrow[m]), int(xrow[m]) + min(int(cnt[m]), max_cnt))
+            want[r] = oracle.mv_rows(tid, mats[m % len(mats)], rows, cols, x[r])
+        assert same_bits(y.cpu().numpy(), want)
+    assert lib.mv_status() == 0
+
+
 @pytest.mark.parametrize("name,cols,off", [("Q6_K", 768, 2), ("Q6_K", 256, 10), ("MXFP4", 768, 8), ("MXFP4", 256, 3), ("IQ4_XS", 768, 8)])
 def test_mv_grouped_matrices_anywhere(lib, dev, oracle, name, cols, off):
     """matrices whose rows are not whole 16-byte pieces need not start on one"""
