@@ -79,6 +79,7 @@ template <int J> __device__ __forceinline__ float biased(uint32_t bytes) {
 // d (n - bias) for the four bytes n of `bytes`, each one fmaf: d (32768 + n) - d (32768 + bias), where the second
 // product `c` is exact (d has 11 significant bits, 32768 + bias at most 13) and so is the difference - the same bits
 // as mul_rn(d, (float) (n - bias)), whose product is exact too.
+// (An infinite d makes every value NaN here and an infinity there, but for the code whose difference is 0: see sum_again.)
 __device__ __forceinline__ void scaled4(uint32_t bytes, float d, float c, float* v) {
   v[0] = __fmaf_rn(d, biased<0>(bytes), c), v[1] = __fmaf_rn(d, biased<1>(bytes), c);
   v[2] = __fmaf_rn(d, biased<2>(bytes), c), v[3] = __fmaf_rn(d, biased<3>(bytes), c);
@@ -178,6 +179,32 @@ template <> struct LanePlan<QTYPE_MXFP4> {
   }
 };
 
+// A warp's rows whose sums came out NaN, summed again from global memory with mv.cu's values: where scaled4 met an infinite
+// scale the sum is NaN for certain, so no other row needs a look. Off the loop: what it costs there is a compare a row.
+// (Arguments by value: taken by reference they would be copied to every thread's stack at the kernel's start.)
+template <uint32_t T, int RW>
+__device__ __noinline__ void sum_again(const uint8_t* w, uint32_t rows, uint32_t cols, const float* x, uint32_t xs, float* y, uint32_t ys, uint32_t u,
+                                       uint32_t u_hi, uint32_t n_tok) {
+  const uint32_t lane = threadIdx.x % kWarp, row_bytes = cols / Fmt<T>::values * Fmt<T>::bytes;
+  __syncwarp();  // (the sums, stored by the first lane, before every lane's look at them)
+  for (; u < u_hi; u += kWarps)
+    for (uint32_t r = u * RW; r < u * RW + RW && r < rows; r++)
+      for (uint32_t t = 0; t < n_tok; t++) {
+        float* at = y + (uint64_t) t * ys + r;
+        if (!__any_sync(0xFFFFFFFFu, isnan(*at))) continue;
+        float s = 0.0f;
+        for (uint32_t c = lane; c < cols / kChunk; c += kWarp) {
+          float v[kChunk];
+          decode8<T>(w + (uint64_t) r * row_bytes + (c / Fmt<T>::chunks) * Fmt<T>::bytes, (int) (c % Fmt<T>::chunks), v, Grids{});
+          const float* xc = x + (uint64_t) t * xs + c * kChunk;
+#pragma unroll
+          for (int j = 0; j < kChunk; j++) s = __fmaf_rn(v[j], xc[j], s);
+        }
+        s = xor_tree<kWarp>(s);
+        if (lane == 0) *at = s;
+      }
+}
+
 template <uint32_t T, int NT, int RW, bool GROUP>
 __global__ void __launch_bounds__(kThreads, 1) mv_staged_kernel(const Args a) {
   extern __shared__ __align__(128) uint8_t smem[];
@@ -243,12 +270,14 @@ __global__ void __launch_bounds__(kThreads, 1) mv_staged_kernel(const Args a) {
   LanePlan<T> plan(lane);
   if constexpr (T == QTYPE_MXFP4) plan.tbl = smem_addr(e2m1_values);
 
+  bool again = false;  // (one of the types of scaled4: a sum was NaN)
   for (uint32_t i = 0;; i++) {
     const uint32_t u = u_lo + warp + i * kWarps;
     if (u >= u_hi) break;
     const uint32_t slot = i % S;
     if (!bar_wait_warp(&full[warp][slot], (i / S) & 1u)) {  // a copy never landed: report it and leave
       if (lane == 0) atomicOr(a.status, 1u);
+      again = false;
       break;
     }
     const uint8_t* sp = ring + slot * a.slot_bytes;
@@ -290,8 +319,11 @@ __global__ void __launch_bounds__(kThreads, 1) mv_staged_kernel(const Args a) {
       for (int t = 0; t < NT; t++) {
         const float s = xor_tree<kWarp>(acc[q][t]);
         if (lane == 0 && r0 + q < a.rows && (uint32_t) t < live) yout[(uint64_t) t * a.ys + r0 + q] = s;
+        if constexpr (kPlainPair<T>) again = again || isnan(s);
       }
   }
+  if constexpr (kPlainPair<T> && !GROUP)
+    if (again) sum_again<T, RW>(a.w, a.rows, a.cols, a.x, a.xs, a.y, a.ys, u_lo + warp, u_hi, live);
 }
 
 constexpr int kRegIters = 8;  // 256-value stretches of a row whose x a lane can keep in registers (cols <= 2048)
@@ -355,12 +387,14 @@ __global__ void __launch_bounds__(kThreads, 1) mv_regx_kernel(const Args a) {
   LanePlan<T> plan(lane);
   if constexpr (T == QTYPE_MXFP4) plan.tbl = smem_addr(e2m1_values);
 
+  bool again = false;  // (one of the types of scaled4: a sum was NaN)
   for (uint32_t i = 0;; i++) {
     const uint32_t u = u_lo + warp + i * kWarps;
     if (u >= u_hi) break;
     const uint32_t slot = i % S;
     if (!bar_wait_warp(&full[warp][slot], (i / S) & 1u)) {  // a copy never landed: report it and leave
       if (lane == 0) atomicOr(a.status, 1u);
+      again = false;
       break;
     }
     const uint8_t* sp = ring + slot * a.slot_bytes;
@@ -415,8 +449,11 @@ __global__ void __launch_bounds__(kThreads, 1) mv_regx_kernel(const Args a) {
     for (int q = 0; q < RW; q++) {
       const float s = xor_tree<kWarp>(acc[q]);
       if (lane == 0 && r0 + q < a.rows) yout[r0 + q] = s;
+      if constexpr (kPlainPair<T>) again = again || isnan(s);
     }
   }
+  if constexpr (kPlainPair<T> && !GROUP)
+    if (again) sum_again<T, RW>(a.w, a.rows, a.cols, a.x, a.xs, a.y, a.ys, u_lo + warp, u_hi, 1u);
 }
 
 struct Device {

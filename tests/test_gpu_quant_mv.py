@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 import torch
 
-from helpers import pointer_table, ptr, same_bits, sync, to_dev
+from helpers import pointer_table, ptr, same_bits, same_bits_or_nan, special_scales, sync, to_dev
 from libosmos_b200 import synth
 from oracle.oracle import BLOCK, LANE_TYPES, TYPES
 
@@ -125,7 +125,9 @@ PAIRED = ["Q4_0", "Q8_0", "Q4_K", "Q5_K", "Q6_K", "IQ4_XS", "MXFP4"]  # (the typ
 @pytest.mark.parametrize("cols,rows", [(256, 1), (256, 7), (768, 66), (2048, 35), (2304, 5), (4352, 33), (9472, 6), (768, 8 * 16 * 160 + 5)])
 def test_mv_paired_lanes(lib, dev, oracle, name, cols, rows):
     """rows that start anywhere in a 16-byte piece (the matrix's last bytes among them), one and several segments of a row,
-    tokens in one pass and in two, one and two rows a thread; every token count, strided x and y"""
+    tokens in one pass and in two, one and two rows a thread; every token count, strided x and y. (Few rows of Q4_0, Q8_0,
+    IQ4_XS and MXFP4 go to the staged kernel at 1, 2, 4 and 8 tokens, Q8_0 at one and two at any height:
+    test_mv_paired_lanes_tall has the rest.)"""
     tid = TYPES[name]
     xs, ys = cols + 8, (rows + 7) // 8 * 8 + 8
     rng = synth.rng_for(15, tid, rows, cols)
@@ -140,6 +142,58 @@ def test_mv_paired_lanes(lib, dev, oracle, name, cols, rows):
         sync()
         got = y.cpu().numpy()
         assert same_bits(got[:n, :rows], want[:n]) and (got[:n, rows:] == -3.0).all() and (got[n:] == -3.0).all()
+    assert lib.mv_status() == 0
+
+
+@pytest.mark.parametrize("name", PAIRED)
+@pytest.mark.parametrize("cols,rows", [(512, 4003), (2304, 8 * 16 * 160 + 5)])
+def test_mv_paired_lanes_tall(lib, dev, oracle, name, cols, rows):
+    """more rows than the staged kernel is asked for, and two rows a thread over several segments of a row; every token count:
+    some rows against the oracle, all of them against the generic kernel"""
+    tid = TYPES[name]
+    rng = synth.rng_for(20, tid, rows, cols)
+    w = synth.random_tensor(tid, rows, cols, rng)
+    x = rng.standard_normal((8, cols)).astype(np.float32)
+    row_bytes = w.size // rows
+    some = np.unique(np.concatenate([np.arange(3), rng.integers(0, rows, 40), rows - 1 - np.arange(3)]))
+    want = oracle.mv_rows(tid, np.ascontiguousarray(w.reshape(rows, row_bytes)[some]).reshape(-1), len(some), cols, x)
+    wd, xd = to_dev(w, dev), to_dev(x, dev)
+    generic = torch.full((8, rows), np.nan, dtype=torch.float32, device=dev)
+    lib.mv_status()
+    lib.mv_set_staged(0)
+    try:
+        assert lib.mv_run(tid, ptr(wd), rows, cols, ptr(xd), 8, ptr(generic), None)
+    finally:
+        lib.mv_set_staged(1)
+    for n in range(1, 9):
+        y = torch.full((n, rows), np.nan, dtype=torch.float32, device=dev)
+        assert lib.mv_run(tid, ptr(wd), rows, cols, ptr(xd), n, ptr(y), None)
+        sync()
+        got = y.cpu().numpy()
+        assert same_bits(got[:, some], want[:n]) and same_bits(got, generic.cpu().numpy()[:n])
+    assert lib.mv_status() == 0
+
+
+@pytest.mark.parametrize("name", PAIRED + ["IQ3_XXS", "IQ1_S", "IQ1_M"])
+@pytest.mark.parametrize("cols,rows", [(2048, 37), (512, 8 * 16 * 160 + 3)])
+@pytest.mark.parametrize("infinite", [False, True])
+def test_mv_special_scales(lib, dev, oracle, name, cols, rows, infinite):
+    """negative, zero, subnormal and large scales give the oracle's bits on every path; infinite ones an infinity or a NaN where
+    the oracle has one"""
+    if infinite and name == "MXFP4":
+        pytest.skip("a scale of MXFP4 is finite")
+    tid = TYPES[name]
+    rng = synth.rng_for(21, tid, rows, cols)
+    w = special_scales(tid, synth.random_tensor(tid, rows, cols, rng), rng, infinite, 0.02 if infinite else 0.5)
+    x = np.abs(rng.standard_normal((8, cols))).astype(np.float32)
+    want = oracle.mv_rows(tid, w, rows, cols, x)
+    assert np.isinf(want).any() if infinite and name in PAIRED else np.isfinite(want).all() != infinite
+    wd, xd = to_dev(w, dev), to_dev(x, dev)
+    for n in (1, 2, 3, 4, 8):
+        y = torch.full((n, rows), -3.0, dtype=torch.float32, device=dev)
+        assert lib.mv_run(tid, ptr(wd), rows, cols, ptr(xd), n, ptr(y), None)
+        sync()
+        assert same_bits_or_nan(y.cpu().numpy(), want[:n])
     assert lib.mv_status() == 0
 
 
@@ -215,6 +269,13 @@ def test_mv_paired_lanes_few_live(lib, dev, oracle, name, entries, live, rows, c
             want[r] = oracle.mv_rows(tid, mats[m % len(mats)], rows, cols, x[r])
         assert same_bits(y.cpu().numpy(), want)
     assert lib.mv_status() == 0
+
+
+@pytest.mark.parametrize("name,cols", [("MXFP4", 7168), ("MXFP4", 9472), ("Q6_K", 7168), ("Q6_K", 9472)])
+def test_mv_paired_lanes_grouped_in_passes(lib, dev, oracle, name, cols):
+    """entries whose tokens' x takes more than one pass over the weights"""
+    got, want = _grouped_at(lib, dev, oracle, name, cols, 75, 0, cnt=(5, 8, 1, 6, 2, 7, 3, 4))
+    assert same_bits(got, want) and lib.mv_status() == 0
 
 
 @pytest.mark.parametrize("name,cols,off", [("Q6_K", 768, 2), ("Q6_K", 256, 10), ("MXFP4", 768, 8), ("MXFP4", 256, 3), ("IQ4_XS", 768, 8)])
