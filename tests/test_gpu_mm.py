@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 import torch
 
-from helpers import ptr, same_bits, sync, to_dev
+from helpers import ptr, same_bits, special_scales, sync, to_dev
 from libosmos_b200 import synth
 from oracle.oracle import TYPES
 
@@ -256,3 +256,66 @@ def test_mm_run_gated_mean(lib, dev, oracle, hc, dim, cols, counts):
     assert not lib.mm_run_gated_mean(tid, ptr(wd), 9, dim, cols, ptr(xb), 8, ptr(xnd), f, None, 0, None, None)
     assert not lib.mm_run_gated_mean(tid, ptr(wd), hc, dim + 8, cols, ptr(xb), 8, ptr(xnd), f, None, 0, None, None)  # dim not 16s
     assert not lib.mm_run_gated_mean(tid, ptr(wd), hc, dim, cols, ptr(xb), 2049, ptr(xnd), f, None, 0, None, None)
+
+
+def _one_hot_product(lib, dev, tid, wd, rows, cols):
+    """mm_run over one-hot activations, a token a column: y[t, r] is the f16 weight W[r, t] (and zeros), exactly"""
+    y = torch.empty((cols, rows), dtype=torch.float32, device=dev)
+    lib.mm_status()
+    assert lib.mm_fits(tid, rows, cols)
+    x = _x16(lib, dev, np.eye(cols, dtype=np.float32), cols)
+    for t in range(0, cols, 512):  # (tokens a call: whole tiles of x16, MM_TILE rows of cols values each)
+        n = min(512, cols - t)
+        assert lib.mm_run(tid, wd, rows, cols, ptr(x) + 2 * t * cols, n, ptr(y) + 4 * t * rows, rows, None)
+    sync()
+    assert lib.mm_status() == 0
+    return y.cpu().numpy().T
+
+
+def _f16_weights(oracle, tid, w, rows, cols):
+    with np.errstate(over="ignore"):
+        return oracle.dequant(tid, w, rows * cols).reshape(rows, cols).astype(np.float16).astype(np.float32)
+
+
+def test_mm_mxfp4_every_exponent(lib, dev, oracle):
+    """MXFP4's three ways to f16 - too small for it, one product, more than one - and their edges: every exponent with every
+    code, a value a row (the rest of the row zeros, so that an infinite one meets no other); then rows full of codes"""
+    tid, cols = TYPES["MXFP4"], 128
+    rows = 256 * 16
+    blocks = np.zeros((rows, cols // 32, 17), np.uint8)
+    blocks[:, :, 0] = 120
+    e, code = np.arange(rows) // 16, np.arange(rows) % 16
+    at = (np.arange(rows) * 37) % cols
+    blk, j = at // 32, at % 32  # (value j of a block: byte j % 16, the low nibble of the first sixteen)
+    blocks[np.arange(rows), blk, 0] = e
+    blocks[np.arange(rows), blk, 1 + j % 16] = np.where(j < 16, code, code << 4)
+    want = _f16_weights(oracle, tid, blocks.reshape(-1), rows, cols)
+    assert np.isinf(want).any() and ((want != 0) & (np.abs(want) < 2.0 ** -14)).any()
+    got = _one_hot_product(lib, dev, tid, ptr(to_dev(blocks.reshape(-1), dev)), rows, cols)
+    inf = np.isinf(want).any(axis=1)
+    assert np.array_equal(got[~inf], want[~inf])
+    assert np.array_equal(got[inf, at[inf]], want[inf, at[inf]]) and np.isnan(np.delete(got[inf][0], at[inf][0])).all()  # (inf x 0)
+    rows = 256  # every exponent whose values are finite in f16, all codes, up to the largest
+    rng = synth.rng_for(57)
+    raw = rng.integers(0, 256, size=(rows, cols // 32, 17), dtype=np.uint8)
+    raw[:, :, 0] = rng.integers(90, 140, size=(rows, cols // 32))
+    want = _f16_weights(oracle, tid, raw.reshape(-1), rows, cols)
+    assert np.isfinite(want).all()
+    assert np.array_equal(_one_hot_product(lib, dev, tid, ptr(to_dev(raw.reshape(-1), dev)), rows, cols), want)
+
+
+@pytest.mark.parametrize("name,cols", [("MXFP4", 128), ("MXFP4", 384), ("MXFP4", 640), ("Q4_0", 128), ("Q4_0", 384), ("Q4_0", 640), ("Q8_0", 384),
+                                       ("Q4_K", 256), ("Q4_K", 768), ("Q5_K", 256), ("Q5_K", 768), ("Q6_K", 256), ("Q6_K", 768)])
+@pytest.mark.parametrize("off", [0, 2, 6, 8])
+def test_mm_decoded_weights(lib, dev, oracle, name, cols, off):
+    """every weight as the product sees it: rows that end within a K block or start anywhere in a 16-byte piece, a matrix on a
+    word and in the middle of one (of Q4_K and Q5_K another decoder); scales of either sign, zero, subnormal and large"""
+    tid, rows = TYPES[name], 144
+    rng = synth.rng_for(58, tid, cols, off)
+    w = special_scales(tid, synth.random_tensor(tid, rows, cols, rng), rng)
+    want = _f16_weights(oracle, tid, w, rows, cols)
+    assert np.isfinite(want).all()
+    pool = np.zeros(w.size + 32, np.uint8)
+    pool[off:off + w.size] = w
+    got = _one_hot_product(lib, dev, tid, ptr(to_dev(pool, dev)) + off, rows, cols)
+    assert np.array_equal(got, want)

@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 import torch
 
-from helpers import pointer_table, ptr, same_bits, sync, to_dev
+from helpers import pointer_table, ptr, same_bits, same_bits_or_nan, special_scales, sync, to_dev
 from libosmos_b200 import synth
 from oracle.oracle import LANE_TYPES, TYPES
 
@@ -154,6 +154,26 @@ def test_lane_ring_row_widths(lib, dev, oracle, name, cols):
             g, u = (oracle.q8_rows(tid, w[m], rows, cols, wq[r], wd[r]) for w in (gate, up))
             assert same_bits(y.cpu().numpy()[r], u)
             assert same_bits(h.cpu().numpy()[r], oracle.swiglu_lane(g, u, 1.5, scale[r]))
+    assert lib.q8_status() == 0
+
+
+@pytest.mark.parametrize("name", ["IQ1_S", "IQ1_M", "IQ2_XXS", "IQ3_XXS"])
+@pytest.mark.parametrize("cols", [2048, 5120])
+@pytest.mark.parametrize("infinite", [False, True])
+def test_lane_special_scales(lib, dev, oracle, name, cols, infinite):
+    """negative, zero, subnormal, large and infinite scales on the int8 lane: the oracle's bits, its infinities and NaNs"""
+    tid, rows, cnt = TYPES[name], 64, [3, 1]
+    rng = synth.rng_for(30, tid, cols)
+    mats = [special_scales(tid, synth.random_tensor(tid, rows, cols, rng), rng, infinite, 0.02 if infinite else 0.5) for _ in cnt]
+    x = rng.standard_normal((4, cols)).astype(np.float32)
+    wq, wd = oracle.q8_round(x)
+    _p, tab, cd, rd = _tables(dev, mats, cnt, [0, 3])
+    y = torch.full((4, rows), -9.0, dtype=torch.float32, device=dev)
+    lib.q8_status()
+    assert lib.q8_group_tok(tid, ptr(tab), ptr(cd), ptr(rd), None, 2, 8, rows, cols, ptr(to_dev(wq, dev)), ptr(to_dev(wd, dev)), ptr(y), rows, None)
+    sync()
+    want = np.concatenate([oracle.q8_rows(tid, mats[0], rows, cols, wq[:3], wd[:3]), oracle.q8_rows(tid, mats[1], rows, cols, wq[3:], wd[3:])])
+    assert np.isfinite(want).all() != infinite and same_bits_or_nan(y.cpu().numpy(), want)
     assert lib.q8_status() == 0
 
 
