@@ -580,7 +580,7 @@ def run_ours(args):
             roof.update({"kernel": "q8_gate_up (lane_ring_kernel, %s, fused gate + up + activation) on rank 0" % cfg["type"],
                          "achieved": achieved, "frac": achieved / peak,
                          "traffic": 296292352 if (world == 1 and cfg["name"] == workloads.MOE_IQ3["name"]) else None,
-                         "traffic_source": "dram__bytes_read.sum + dram__bytes_write.sum of one launch, profiles/lane_ring_rows_iq3xxs_moe.md"
+                         "traffic_source": "dram__bytes_read.sum + dram__bytes_write.sum of one launch, captured by ncu"
                          if (world == 1 and cfg["name"] == workloads.MOE_IQ3["name"]) else None,
                          "algorithmic_bytes_per_launch": float(np.mean(alg)), "us_per_launch": float(np.mean(k_ms) * 1e3)})
         cpu = None

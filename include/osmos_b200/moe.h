@@ -48,7 +48,7 @@ typedef struct Q4xExpertTiles
   int32_t *off;                              /* scratch: 3 * n_exp ints */
 } Q4xExpertTiles;
 
-#define Q4X_TILE_RUNS 4 /* an entry's token tiles: 1, 2, 4 or 8 (16 .. 128 tokens), a launch each */
+#define Q4X_TILE_RUNS 4 /* an entry's token tiles: 1, 2, 4 or 8 (16 .. 128 tokens); the products take them all in one launch */
 typedef struct Q4xExpertBounds
 {
   uint32_t first[Q4X_TILE_RUNS], count[Q4X_TILE_RUNS];

@@ -92,10 +92,11 @@ __device__ __forceinline__ uint64_t tile_desc_sw32(uint32_t addr) {
 constexpr uint32_t kIdesc = (1u << 4) | (0u << 7) | (0u << 10) | ((uint32_t) (kN >> 3) << 17) | ((uint32_t) (kM >> 4) << 24);
 
 // ---- the common types' chunks straight to f16 -----------------------------------------------------------------
-// Eight values of a block whose bytes lie in shared memory at `blk` (4-byte aligned here), as eight f16 in a uint4:
-// the same F32 value decode8 gives (each product rounded once), then rounded to f16. Small integers reach F32 by a
-// byte permute (byte n into bits 8 .. 15 of 0x47000000 = 32768 + n), and a product d n as fmaf(d, 32768 + n,
-// -32768 d): the subtrahend is a power of two times d, so the one rounding is the product's own.
+// Eight values of a Q8_0 or a Q6_K block whose bytes lie in shared memory at `blk` (Q8_0: on a half-word; Q6_K: anywhere), as
+// eight f16 in a uint4: the same F32 value decode8 gives (each product rounded once), then rounded to f16. Small integers
+// reach F32 by a byte permute (byte n into bits 8 .. 15 of 0x47000000 = 32768 + n), and Q8_0's product d n as
+// fmaf(d, 32768 + n, -32768 d): the subtrahend is a power of two times d, so the one rounding is the product's own (of an
+// infinite d it is NaN, where d n is an infinity).
 template <int J> __device__ __forceinline__ float biased(uint32_t bytes) {
   return __uint_as_float(__byte_perm(bytes, 0x47000000u, 0x7404 | (J << 4)));
 }

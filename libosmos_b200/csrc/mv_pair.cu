@@ -11,8 +11,9 @@
 // read of x whose neighbouring lanes ask for the same piece takes two passes of shared memory, one whose halves do takes
 // four, like 32 different pieces (measured: 2.0 against 4.0 cycles a warp).
 //
-// Bound by instruction issue and shared-memory passes: about 5 instructions a value at one token (a byte permute, half of an
-// add, half of a multiply, half of an fmaf, the unpacking), and from three tokens on x's reads. Measured, against a lane a
+// Bound by instruction issue at one token - 6.8 instructions a value all told (Q6_K 98304 x 2048, 60.3 us: 68 % of the issue slots,
+// the integer pipe 66 %, shared memory 28 %, DRAM 34 %: what is left is four warps a scheduler with a chain each, and 9 %
+// of the launch before the first slot and after the last) - and from three tokens on by x's reads. Measured, against a lane a
 // thread (mv_staged.cu): 49152 x 2048 at one token Q6_K 41.1 -> 29.5 us (2.8 TB/s), Q5_K 45.1 -> 33.4, Q4_K 39.6 -> 29.9, IQ4_XS
 // 42.1 -> 27.7; at eight tokens 80-85 -> 64-69; Q4_K 2048 x 7168 at five 22.6 -> 12.0; 1536 x 4096 MXFP4 matrices of 64 experts
 // at 64 picks 239 -> 111 us.
