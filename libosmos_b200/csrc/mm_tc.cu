@@ -7,26 +7,29 @@
 // partitions; a token's column is computed from that column alone, so its bits do not depend on the tokens beside
 // it or on where in the batch it stands.
 //
-// A block computes 128 weight rows x 128, 256 or 512 tokens of one matrix (the most that still leaves every SM a
-// block), a weight decoded once a block.
-// Twenty-five warps, four roles:
-//   loader (4 warps)     cp.async of the tokens' 16-byte pieces of x16 into the B operand's layout, its arrivals on the
-//                        stage's second "full" mbarrier made by the hardware when the copies land
-//   producers (16 warps, two teams of 8 on alternate steps) per 64-value step of K: decode the rows' 8-value chunks to f16 and store them as the A
-//                        operand (four K = 16 sub-tiles of 128 rows, K-major core matrices of 8 rows x 16 bytes), and
-//                        cp.async the tokens' 16-byte pieces of x16 into the same layout (B, four sub-tiles a
-//                        128-token accumulator); a proxy fence and an arrive on the stage's "full" mbarrier. Two stages; the rows'
-//                        bytes reach the decoders through shared memory, 256 values of K at a time (128 of Q8_0).
-//   issuer (1 warp)      per step and accumulator four tcgen05.mma M128 N128 K16 (the first of the whole K loop
-//                        overwrites, the rest accumulate), then tcgen05.commit onto the stage's "empty" mbarrier; after
-//                        the last step a commit onto "done".
+// The decoded weights are the products' operand in TENSOR MEMORY: a producer thread is a weight row, decodes 64 values
+// of it and writes them to its own lane (tcgen05.st), so a decoded tile costs no shared-memory stores, no proxy fence and no
+// operand reads from shared memory - which only the activations pass through.
+//
+// Blocks are persistent, one an SM; a tile is 128 weight rows x up to 256 tokens of one matrix. Tensor memory: two
+// accumulators of 128 columns - a tile of up to 128 tokens takes one, so that its sums are stored while the next tile's
+// products run; a larger tile takes both - and eight stages of 32 columns, 64 values of K each.
+// Twenty-four warps, five roles that never meet in a tile:
 //   epilogue (4 warps)   thread = one weight row (its TMEM lane): tcgen05.ld the sums, scale, store y[t][row] - or, for
 //                        mm_run_silu, silu(scale sum) to y and as f16 into the next product's tiled activations; for
 //                        mm_run_gated_mean the block's rows are hc streams' rows of the same dim values (row map
 //                        below), each thread gates its sum, and the streams are added in order through shared memory
-//                        (the operand ring, idle by then).
-// Every mbarrier wait is bounded (%globaltimer); a wait that runs out raises the status word, every role falls through
-// to the common exit and tensor memory is released.
+//   producers (16 warps, four teams of four on every fourth K step) decode the rows' bytes out of shared memory
+//   issuer (1 warp)      a K step's tcgen05.mma M128 N<=128 K16 (four an accumulator; the first of a tile overwrites, the
+//                        rest accumulate), then tcgen05.commit onto the step's "empty" mbarrier; after a tile's last step a
+//                        commit onto its accumulators' "full" ones
+//   raw loaders (2 warps) cp.async of the rows' bytes, 256 values of K at a time (128 of the widest types), a ring of
+//                        three or four
+//   token loader (1 warp) the tokens' x16, a K step at a time: one tensor-map copy (mm_run), or 16-byte cp.async pieces
+//                        (mm_group: an expert's tokens start anywhere in x16, and a copy of a 512-byte fragment each costs ~45
+//                        cycles to issue), its arrivals on the stage's mbarrier made by the hardware when the copies land
+// Every mbarrier wait is bounded (%globaltimer) with one outcome a warp; a wait that runs out raises the status word, every
+// role falls through to the common exit and tensor memory is released.
 #include <cuda.h>
 
 #include <cstring>
@@ -46,208 +49,314 @@ namespace {
 
 using namespace tma;
 
-constexpr int kM = 128, kN = 128;  // rows a block; tokens an accumulator
-constexpr int kMaxAcc = 4;         // accumulators a block: 512 tokens
-constexpr int kEpiWarps = 4, kProdWarps = 16;
-constexpr int kLoaderWarps = 4;
-// Roles go by the warp scheduler a warp lives on (its index mod 4): scheduler 0 has the issuer - whose chain of tcgen05
-// instructions a step is the critical path, and must not queue for issue slots behind the decoders - the four loaders
-// and one producer; the other fifteen producers share schedulers 1 to 3 with the epilogue warps.
-constexpr int kIssuerWarp = 4;
-__host__ __device__ constexpr int loader_of(int warp) { return (warp >= 8 && warp <= 20 && warp % 4 == 0) ? (warp - 8) / 4 : -1; }
-__host__ __device__ constexpr int producer_of(int warp) {
-  return warp == 24 ? 15 : (warp >= 5 && warp <= 23 && warp % 4 != 0) ? ((warp - 5) / 4) * 3 + warp % 4 - 1 : -1;
-}
-static_assert(producer_of(5) == 0 && producer_of(7) == 2 && producer_of(9) == 3 && producer_of(23) == 14 && producer_of(24) == 15 &&
-                  producer_of(8) == -1 && producer_of(4) == -1 && loader_of(8) == 0 && loader_of(20) == 3 && loader_of(24) == -1,
-              "sixteen producers, four loaders");
-constexpr int kProdThreads = kProdWarps * kWarp, kLoaderThreads = kLoaderWarps * kWarp;
-// The producers work as kGroups teams, team g on the K steps g, g + kGroups, ...: a step's chain (raw bytes out of
-// shared memory, decode, store, proxy fence, arrival) is latency, and two steps' chains run side by side.
-// (A team comes back to a stage after at most as many steps as the ring is deep, so its parity waits never skip a phase.)
-constexpr int kGroups = 2, kTeamThreads = kProdThreads / kGroups;
-constexpr int kThreads = (kEpiWarps + 1 + kLoaderWarps + kProdWarps) * kWarp;
-constexpr int kStep = 64;                        // values of K a stage
-constexpr int kSubTile = kM * 32;                // one K = 16 operand sub-tile: 128 rows x 32 bytes
-constexpr int kSubs = kStep / 16;                // sub-tiles a stage an operand: 4
-constexpr int kStageA = kSubs * kSubTile;        // 16 KB
-constexpr int kMaxStages = 4;
+constexpr int kM = 128, kN = 128;  // rows a tile; tokens an accumulator
+constexpr int kMaxAcc = 4;         // mm_col_tiles' largest class
+constexpr int kEpiWarps = 4, kProdWarps = 16, kRawWarps = 2;
+constexpr int kTeams = 4;          // producer teams: team t on the K steps t, t + 4, ...; its warp w has the rows 32 w .. 32 w + 31
+constexpr int kFirstProd = kEpiWarps, kIssuerWarp = kFirstProd + kProdWarps, kFirstRaw = kIssuerWarp + 1, kTokenWarp = kFirstRaw + kRawWarps;
+constexpr int kThreads = (kTokenWarp + 1) * kWarp;
+static_assert(kFirstProd % 4 == 0 && kProdWarps == 4 * kTeams, "a producer warp's rows are its quarter of tensor memory (its index mod 4)");
+constexpr int kStep = 64;                  // values of K a stage
+constexpr int kSubs = kStep / 16;          // K = 16 products a stage
+constexpr uint32_t kSteps = 8;             // stages of decoded weights
+constexpr uint32_t kAccCols = 2 * kN;      // tensor memory: the accumulators' columns, then the stages', 32 each
+constexpr uint32_t kStageCols = kStep / 2;
+static_assert(kAccCols + kSteps * kStageCols == 512, "all of tensor memory");
+constexpr uint32_t kMaxSpan = 2 * kN;      // tokens a tile
+constexpr uint32_t kMaxMats = 768;        // matrices a launch: their first tiles are kept in shared memory
 
 __device__ uint32_t g_status;
 
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+// shared-memory matrix descriptor of one K = 16 sub-tile of tokens: x16's fragments as they lie - a token's 16 values 32 bytes - as
+// rows of 64 bytes, two tokens each, with the 64-byte swizzle; 8 rows are 512 bytes. A product takes the first 32 bytes of
+// each row, the even tokens, or (the address 32 bytes on) the second, the odd ones: a copy of rows of 32 bytes under the
+// 32-byte swizzle would be one product's operand, but moves 30 bytes a cycle, half of these.
+__device__ __forceinline__ uint64_t tile_desc_sw64(uint32_t addr) {
+  return (uint64_t) ((addr >> 4) & 0x3FFFu) | (uint64_t) 1 << 16 | (uint64_t) (512u >> 4) << 32 | (uint64_t) 1 << 46 | (uint64_t) 4 << 61;
 }
-// shared-memory matrix descriptor of one sub-tile: K-major, no swizzle, core matrices of 8 rows x 16 bytes; the next
-// 16 bytes of K are 128 bytes on (leading offset), the next 8 rows 256 bytes on (stride offset)
-__device__ __forceinline__ uint64_t tile_desc(uint32_t addr) {
-  return (uint64_t) ((addr >> 4) & 0x3FFFu) | (uint64_t) (128u >> 4) << 16 | (uint64_t) (256u >> 4) << 32 | (uint64_t) 1 << 46;
-}
-// the same for a sub-tile a tensor-map copy wrote with the 32-byte swizzle: rows of 32 bytes (one MMA's K), the two
-// 16-byte halves of a row exchanged in every second group of four rows; 8 rows are 256 bytes
-__device__ __forceinline__ uint64_t tile_desc_sw32(uint32_t addr) {
-  return (uint64_t) ((addr >> 4) & 0x3FFFu) | (uint64_t) 1 << 16 | (uint64_t) (256u >> 4) << 32 | (uint64_t) 1 << 46 | (uint64_t) 6 << 61;
-}
-// instruction descriptor: D F32, A and B f16, both K-major, N = 128, M = 128
-constexpr uint32_t kIdesc = (1u << 4) | (0u << 7) | (0u << 10) | ((uint32_t) (kN >> 3) << 17) | ((uint32_t) (kM >> 4) << 24);
+// instruction descriptor: D F32, A and B f16, both K-major, M = 128, N = n
+__device__ __forceinline__ uint32_t idesc(uint32_t n) { return (1u << 4) | (n >> 3) << 17 | (uint32_t) (kM >> 4) << 24; }
 
-// ---- the common types' chunks straight to f16 -----------------------------------------------------------------
-// Eight values of a Q8_0 or a Q6_K block whose bytes lie in shared memory at `blk` (Q8_0: on a half-word; Q6_K: anywhere), as
-// eight f16 in a uint4: the same F32 value decode8 gives (each product rounded once), then rounded to f16. Small integers
-// reach F32 by a byte permute (byte n into bits 8 .. 15 of 0x47000000 = 32768 + n), and Q8_0's product d n as
-// fmaf(d, 32768 + n, -32768 d): the subtrahend is a power of two times d, so the one rounding is the product's own (of an
-// infinite d it is NaN, where d n is an infinity).
-template <int J> __device__ __forceinline__ float biased(uint32_t bytes) {
-  return __uint_as_float(__byte_perm(bytes, 0x47000000u, 0x7404 | (J << 4)));
+__device__ __forceinline__ void bar_arrive_n(uint64_t* bar, uint32_t n) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(n) : "memory");
 }
+__device__ __forceinline__ void arrive_when_copied(uint64_t* bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_addr(bar)) : "memory");
+}
+
+// ---- the rows' raw bytes in shared memory ---------------------------------------------------------------------------
+// This many values of K at a time (a whole number of blocks), in slots of an odd number of 16-byte pieces a row: the 16-byte
+// reads of a warp - 32 rows - then take no more passes than their bytes need.
+template <uint32_t T> constexpr uint32_t kRawK = (T == QTYPE_Q8_0 || T == QTYPE_MXFP8) ? 128u : 256u;
+template <uint32_t T> constexpr uint32_t kRawBytes = kRawK<T> / Fmt<T>::values * Fmt<T>::bytes;
+template <uint32_t T> constexpr uint32_t kRawSlot = ((kRawBytes<T> + 30u + 15u) & ~15u) | 16u;
+template <uint32_t T> constexpr uint32_t kRawPieces = (kRawBytes<T> + 30u) / 16u;  // of a row that starts anywhere in its first piece
+template <uint32_t T> constexpr uint32_t kRawStages = (92u * 1024u) / (kM * kRawSlot<T>) < 4u ? (92u * 1024u) / (kM * kRawSlot<T>) : 4u;
+// shared memory: the tokens' ring (1024-byte aligned), the raw ring, the gated mean's exchange, the matrices' first tiles
+template <uint32_t EPI> constexpr uint32_t kTokenRing = (EPI == 2u ? 96u : 128u) * 1024u;
+constexpr uint32_t kChunkTok = 16;  // tokens the epilogue reads at a time
+constexpr uint32_t kExchange = kChunkTok * kM * 4u;
+template <uint32_t T, uint32_t EPI> constexpr uint32_t kRawAt = kTokenRing<EPI>;
+template <uint32_t T, uint32_t EPI> constexpr uint32_t kExAt = kRawAt<T, EPI> + kRawStages<T> * kM * kRawSlot<T>;
+template <uint32_t T, uint32_t EPI> constexpr uint32_t kFirstAt = kExAt<T, EPI> + (EPI == 2u ? kExchange : 0u);
+template <uint32_t T, uint32_t EPI> constexpr uint32_t kSmem = kFirstAt<T, EPI> + (kMaxMats + 1u) * 4u;
+
 __device__ __forceinline__ uint32_t half2_bits(float lo, float hi) {
   const __half2 h = __floats2half2_rn(lo, hi);
   return *(const uint32_t*) &h;
 }
-// the rows' bytes come through shared memory this many values of K at a time (a whole number of blocks; fewer for the
-// widest type, whose two raw buffers would otherwise cost the ring a stage), in slots of an odd number of 16-byte
-// pieces a row
-template <uint32_t T> constexpr uint32_t kRawK = (T == QTYPE_Q8_0) ? 128u : 256u;
-template <uint32_t T> constexpr uint32_t kRawBytes = kRawK<T> / Fmt<T>::values * Fmt<T>::bytes;
-template <uint32_t T> constexpr uint32_t kRawSlot = ((kRawBytes<T> + 30u + 15u) & ~15u) | 16u;
-template <uint32_t T> constexpr bool kFastChunk = (T == QTYPE_Q8_0 || T == QTYPE_Q6_K);
-
-// the eight bytes at shared address `at` (any alignment) out of the three aligned words around them (the third may lie
-// past the last byte asked for: a row's slot in the raw buffer has the room)
-__device__ __forceinline__ uint2 lds_8_bytes(uint32_t at) {
-  const uint32_t al = at & ~3u, sh = (at & 3u) * 8u;
-  const uint32_t r0 = lds32(al), r1 = lds32(al + 4), r2 = lds32(al + 8);
-  return make_uint2(__funnelshift_r(r0, r1, sh), __funnelshift_r(r1, r2, sh));
+__device__ __forceinline__ uint32_t half2_bits(uint64_t v) {
+  float lo, hi;
+  unpack2(v, lo, hi);
+  return half2_bits(lo, hi);
 }
-// byte J of `bytes` - 0x80 + 2 n with n < 64 - as the F32 64 + n: bits 16 .. 23 of 0x42000000
-template <int J> __device__ __forceinline__ float biased64(uint32_t bytes) {
-  return __uint_as_float(__byte_perm(bytes, 0x42000000u, 0x7044 | (J << 8)));
-}
+__device__ __forceinline__ uint32_t lds_half(uint32_t at) { return lds8(at) | lds8(at + 1) << 8; }  // (any address)
 
-template <uint32_t T>
-__device__ __forceinline__ uint4 fast_chunk(const uint8_t* blk, uint32_t k) {
-  uint4 out;
-  if constexpr (T == QTYPE_Q6_K) {
-    // chunk k: sub-block j = k / 4; a half of the block has 64 bytes of low nibbles and 32 of top bit pairs
-    const uint32_t at = smem_addr(blk), j = k >> 2, kk = k & 3u, h = j >> 2, r = j & 3u;
-    const uint2 q = lds_8_bytes(at + 64u * h + 32u * (r & 1u) + 8u * kk), t = lds_8_bytes(at + 128u + 32u * h + 8u * kk);
-    const int sc = (int) (int8_t) lds8(at + 192u + 2u * j + (kk >> 1));
-    const float ds = mul_rn(half_value(lds16(at + 208u)), (float) sc);
-    const uint32_t s4 = 4u * (r >> 1), s2 = 2u * r;
-    // 64 + n made by a byte permute, less 96: the code n - 32, exactly; times d s, rounded once, as decode8's
-    const uint32_t u0 = kTops | ((q.x >> s4) & kLow4) << 1 | ((t.x >> s2) & kLow2) << 5;
-    const uint32_t u1 = kTops | ((q.y >> s4) & kLow4) << 1 | ((t.y >> s2) & kLow2) << 5;
-    auto value = [&](float b) -> float { return mul_rn(ds, __fadd_rn(b, -96.0f)); };
-    out.x = half2_bits(value(biased64<0>(u0)), value(biased64<1>(u0))), out.y = half2_bits(value(biased64<2>(u0)), value(biased64<3>(u0)));
-    out.z = half2_bits(value(biased64<0>(u1)), value(biased64<1>(u1))), out.w = half2_bits(value(biased64<2>(u1)), value(biased64<3>(u1)));
-  } else {  // Q8_0: d q, the signed byte as q + 128; a block's f16 scale, then its bytes (2-byte aligned: read by halves)
-    const uint16_t* hp = (const uint16_t*) blk;
-    const float d = half_value(hp[0]), c = mul_rn(d, -32896.0f);
-    const uint16_t* q = hp + 1 + 4 * k;
-    const uint32_t m0 = ((uint32_t) q[0] | (uint32_t) q[1] << 16) ^ 0x80808080u, m1 = ((uint32_t) q[2] | (uint32_t) q[3] << 16) ^ 0x80808080u;
-    out.x = half2_bits(__fmaf_rn(d, biased<0>(m0), c), __fmaf_rn(d, biased<1>(m0), c));
-    out.y = half2_bits(__fmaf_rn(d, biased<2>(m0), c), __fmaf_rn(d, biased<3>(m0), c));
-    out.z = half2_bits(__fmaf_rn(d, biased<0>(m1), c), __fmaf_rn(d, biased<1>(m1), c));
-    out.w = half2_bits(__fmaf_rn(d, biased<2>(m1), c), __fmaf_rn(d, biased<3>(m1), c));
-  }
-  return out;
-}
-
-// ---- two chunks at once: the low and the high nibbles of the same eight bytes --------------------------------------
-// Of a 64-value K step a row has four such pairs: of the 32-value blocks pair i is chunks i % 2 and two on of block i / 2, of
-// Q4_K and Q5_K (groups 2 g and 2 g + 1 share 32 bytes) chunk i of either group. The bytes are read and unpacked once, the
-// F32 steps of the two run side by side in packed instructions. (4096 x 4096, 512 tokens, rounding included: MXFP4 67 -> 47 us -
-// its chunks went through the byte reader - Q5_K 70 -> 58, Q4_K 67 -> 52, Q4_0 52 -> 47. At 2048 tokens, where the products'
-// operand reads are the bound, 108-110 us as before.)
-template <uint32_t T> constexpr bool kPairChunk = (T == QTYPE_MXFP4 || T == QTYPE_Q4_0 || T == QTYPE_Q4_K || T == QTYPE_Q5_K);
-template <uint32_t T> constexpr bool kPairOfGroups = (T == QTYPE_Q4_K || T == QTYPE_Q5_K);
-
-__device__ __forceinline__ void store_pairs(const uint64_t (&v)[8], uint4& lo, uint4& hi) {
-  float a[8], b[8];
+// the words of PIECES aligned 16-byte pieces of shared memory; bytes and words out of them at offsets known when compiled
+template <int PIECES> struct Pieces {
+  uint32_t w[4 * PIECES];
+  __device__ __forceinline__ void load(uint32_t at) {
 #pragma unroll
-  for (int j = 0; j < 8; j++) unpack2(v[j], a[j], b[j]);
-  lo = make_uint4(half2_bits(a[0], a[1]), half2_bits(a[2], a[3]), half2_bits(a[4], a[5]), half2_bits(a[6], a[7]));
-  hi = make_uint4(half2_bits(b[0], b[1]), half2_bits(b[2], b[3]), half2_bits(b[4], b[5]), half2_bits(b[6], b[7]));
+    for (int i = 0; i < PIECES; i++) {
+      const int4 v = lds128(at + 16u * i);
+      w[4 * i] = (uint32_t) v.x, w[4 * i + 1] = (uint32_t) v.y, w[4 * i + 2] = (uint32_t) v.z, w[4 * i + 3] = (uint32_t) v.w;
+    }
+  }
+  __device__ __forceinline__ uint32_t word(int o) const { return o % 4 ? __funnelshift_r(w[o / 4], w[o / 4 + 1], 8 * (o % 4)) : w[o / 4]; }
+  __device__ __forceinline__ uint32_t byte(int o) const { return __byte_perm(w[o / 4], 0, 0x4440 + o % 4); }
+  __device__ __forceinline__ uint32_t half(int o) const { return word(o) & 0xFFFFu; }
+};
+// the step's bytes, N of them from any address, moved to the front of Pieces: the pieces around them, then the words and bytes
+// shifted into place (a warp's aligned 4-byte reads of its 32 rows would meet four to a bank)
+template <int N> struct Moved : Pieces<(N + 3) / 16 + 2> {
+  __device__ __forceinline__ void load(uint32_t at) {
+    constexpr int kWords = (N + 3) / 4, kAll = 4 * ((N + 3) / 16 + 2);
+    static_assert(kWords + 4 <= kAll, "the words moved");
+    Pieces<(N + 3) / 16 + 2>::load(at & ~15u);
+    uint32_t(&w)[kAll] = this->w;
+    const bool two = (at & 8u) != 0, one = (at & 4u) != 0;
+    const uint32_t sh = (at & 3u) * 8u;
+#pragma unroll
+    for (int i = 0; i < kWords + 2; i++) w[i] = two ? w[i + 2] : w[i];
+#pragma unroll
+    for (int i = 0; i < kWords + 1; i++) w[i] = one ? w[i + 1] : w[i];
+#pragma unroll
+    for (int i = 0; i < kWords; i++) w[i] = __funnelshift_r(w[i], w[i + 1], sh);
+  }
+};
+__device__ __forceinline__ uint4 lds_16(uint32_t at, bool whole) {  // 16 bytes on a word; whole: on 16 bytes
+  if (whole) {
+    const int4 v = lds128(at);
+    return make_uint4((uint32_t) v.x, (uint32_t) v.y, (uint32_t) v.z, (uint32_t) v.w);
+  }
+  return make_uint4(lds32(at), lds32(at + 4u), lds32(at + 8u), lds32(at + 12u));
 }
 
+// ---- 64 values of a row to f16 --------------------------------------------------------------------------------------
+// Every value is the F32 decode8 gives, then rounded to f16. A code n < 1024 in the low bits of a half IS the subnormal f16
+// n 2^-24, which reaches F32 exactly (the bits of a word's codes are masked in place, two at a time; the conversion runs beside the
+// integer pipe, which a byte permute a code kept busy); the scale is taken 2^24 times larger. Where d n (the scale's product
+// with the integer fields included) has at most 24 significant bits, as in all of these types, fma(d, n, c) is the product
+// rounded, exactly, and then the sum, rounded: decode8's two operations. An infinite or NaN scale is not exact times 2^24 or an
+// integer, so such a step goes through decode8 (`odd`: the warp's, as tcgen05.st is the whole warp's).
+__device__ __forceinline__ float low_half(uint32_t h) { return __half2float(__ushort_as_half((unsigned short) (h & 0xFFFFu))); }
+__device__ __forceinline__ float high_half(uint32_t h) { return __half2float(__ushort_as_half((unsigned short) (h >> 16))); }
+struct Affine {  // n 2^-24 -> d n + c
+  uint64_t d, c;
+  __device__ __forceinline__ Affine(float scale, float plus) : d(pack2(mul_rn(scale, 16777216.0f), mul_rn(scale, 16777216.0f))), c(pack2(plus, plus)) {}
+  // codes 0 and 2 (a0), 1 and 3 (a1) in the halves -> (r0, r1): the four values in order, as f16
+  __device__ __forceinline__ void halves(uint32_t a0, uint32_t a1, uint32_t& r0, uint32_t& r1) const {
+    r0 = half2_bits(fma2(d, pack2(low_half(a0), low_half(a1)), c));
+    r1 = half2_bits(fma2(d, pack2(high_half(a0), high_half(a1)), c));
+  }
+  __device__ __forceinline__ void bytes(uint32_t u, uint32_t& r0, uint32_t& r1) const { halves(u & 0x00FF00FFu, __byte_perm(u, 0, 0x4341), r0, r1); }
+};
 // an E2M1 code's bits as an F16's sign, exponent's low two bits and mantissa's top one are its value times 2^-14 (a
 // subnormal code is a subnormal F16): `top` holds such upper bytes of four values, times f
-__device__ __forceinline__ uint2 e2m1_halves(uint32_t top, __half2 f) {
+__device__ __forceinline__ void e2m1_halves(uint32_t top, __half2 f, uint32_t& r0, uint32_t& r1) {
   const uint32_t p0 = __byte_perm(top, 0, 0x1404), p1 = __byte_perm(top, 0, 0x3424);
   const __half2 h0 = __hmul2_rn(*(const __half2*) &p0, f), h1 = __hmul2_rn(*(const __half2*) &p1, f);
-  return make_uint2(*(const uint32_t*) &h0, *(const uint32_t*) &h1);
+  r0 = *(const uint32_t*) &h0, r1 = *(const uint32_t*) &h1;
 }
-__device__ __forceinline__ void scale_halves(uint4& v, uint32_t f2) {
-  const __half2 f = *(const __half2*) &f2;
-  uint32_t* w = (uint32_t*) &v;
+__device__ __forceinline__ bool inf_or_nan(uint32_t half_bits) { return (half_bits & 0x7C00u) == 0x7C00u; }
+
+// K step `sub` of the raw K block whose row starts at shared address `at` (p: the same as a pointer): put(q, r) takes the
+// values 16 q .. 16 q + 15 as eight f16 pairs; the whole warp calls it, in step
+template <uint32_t T, class Put>
+__device__ __forceinline__ void decode_step_any(const uint8_t* p, uint32_t sub, const Grids& g, const Put& put) {
+#pragma unroll 1
+  for (uint32_t q = 0; q < (uint32_t) kSubs; q++) {
+    uint32_t r[8];
 #pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const __half2 h = __hmul2_rn(*(const __half2*) &w[i], f);
-    w[i] = *(const uint32_t*) &h;
+    for (uint32_t i = 0; i < 2; i++) {
+      const uint32_t cl = sub * (kStep / kChunk) + 2u * q + i;  // the chunk's index in its K block
+      float v[kChunk];
+      decode8<T>(p + (cl / Fmt<T>::chunks) * Fmt<T>::bytes, (int) (cl % Fmt<T>::chunks), v, g);
+#pragma unroll
+      for (uint32_t j = 0; j < 4; j++) r[4 * i + j] = half2_bits(v[2 * j], v[2 * j + 1]);
+    }
+    put(q, r);
   }
 }
 
-// pair i of the step whose block (of the 32-value types: whose pair's block) starts at shared address `at`; g: the step's
-// place in a 256-value block. Q4_K and Q5_K: `at` on a word. Read first, decoded after: a thread's several pairs are all
-// read before the first is decoded and stored, so that their shared-memory latencies run together.
-struct PairBytes {
-  uint2 q, f;            // the eight bytes; Q5_K's fifth bits
-  uint32_t h[4];         // the block's head: Q4_K / Q5_K its first four words, else the scale
-};
-template <uint32_t T>
-__device__ __forceinline__ void load_pair(uint32_t at, uint32_t g, uint32_t i, PairBytes& b) {
-  if constexpr (T == QTYPE_MXFP4) {
-    b.h[0] = lds8(at), b.q = lds_8_bytes(at + 1u + 8u * (i & 1u));
-  } else if constexpr (T == QTYPE_Q4_0) {
-    b.h[0] = lds16(at), b.q = lds_8_bytes(at + 2u + 8u * (i & 1u));
-  } else {
-    const uint32_t qa = at + (T == QTYPE_Q5_K ? 48u : 16u) + 32u * g + 8u * i;
-#pragma unroll
-    for (int k = 0; k < 4; k++) b.h[k] = lds32(at + 4u * k);
-    b.q = make_uint2(lds32(qa), lds32(qa + 4u));
-    if constexpr (T == QTYPE_Q5_K) b.f = make_uint2(lds32(at + 16u + 8u * i), lds32(at + 20u + 8u * i));
-  }
-}
-template <uint32_t T>
-__device__ __forceinline__ void pair_chunks(const PairBytes& p, uint32_t g, uint4& lo, uint4& hi) {
-  const uint2 q = p.q;
+// the 32-value types: a step's two blocks at byte O of b (a Pieces); false: an odd scale, nothing put
+template <uint32_t T, int O, class B, class Put>
+__device__ __forceinline__ bool two_blocks(const B& b, const Put& put) {
+  constexpr int kNext = Fmt<T>::bytes;
   if constexpr (T == QTYPE_MXFP4) {
     // times 2^(e - 127): the f16 product by 2^(e - 113) is exact or rounds once, as the F32 value's conversion does - past
     // F16 infinite, below it zero. 2^(e - 113) is an F16 for e <= 128; below e = 99 every value is under half of F16's
-    // least (6 2^-29), so the factor may be zero; above 128 the rest of the power goes in two more exact products.
-    const uint32_t e = p.h[0], f = e >= 99u ? (min(e, 128u) - 98u) << 10 : 0u, f2 = f | f << 16;
-    const __half2 fh = *(const __half2*) &f2;
-    const uint2 l0 = e2m1_halves(((q.x << 1) & 0x0E0E0E0Eu) | ((q.x << 4) & kTops), fh), l1 = e2m1_halves(((q.y << 1) & 0x0E0E0E0Eu) | ((q.y << 4) & kTops), fh);
-    const uint2 h0 = e2m1_halves(((q.x >> 3) & 0x0E0E0E0Eu) | (q.x & kTops), fh), h1 = e2m1_halves(((q.y >> 3) & 0x0E0E0E0Eu) | (q.y & kTops), fh);
-    lo = make_uint4(l0.x, l0.y, l1.x, l1.y), hi = make_uint4(h0.x, h0.y, h1.x, h1.y);
-    if (e > 128u) {
-      const uint32_t a = (min(e, 143u) - 113u) << 10, b = (min(max(e, 143u), 158u) - 128u) << 10;  // 2^(e - 128) up to 2^15; the rest up to 2^15
-      scale_halves(lo, a | a << 16), scale_halves(hi, a | a << 16), scale_halves(lo, b | b << 16), scale_halves(hi, b | b << 16);
-    }
-  } else if constexpr (T == QTYPE_Q4_0) {
-    const float d = half_value(p.h[0]);
-    const uint64_t dd = pack2(d, d);
-    uint64_t v[8];
-    code_pairs(make_uint2(q.x & kLow4, q.y & kLow4), make_uint2((q.x >> 4) & kLow4, (q.y >> 4) & kLow4), -32776.0f, v);
+    // least (6 2^-29), so the factor may be zero; a larger exponent is odd.
+    const uint32_t e0 = b.byte(O), e1 = b.byte(O + kNext);
+    if (__any_sync(0xFFFFFFFFu, max(e0, e1) > 128u)) return false;
 #pragma unroll
-    for (int j = 0; j < 8; j++) v[j] = mul2(dd, v[j]);
-    store_pairs(v, lo, hi);
-  } else {  // Q4_K, Q5_K
+    for (int i = 0; i < 2; i++) {
+      const uint32_t e = i ? e1 : e0, f = e >= 99u ? (e - 98u) << 10 : 0u, f2 = f | f << 16;
+      const __half2 fh = *(const __half2*) &f2;
+      uint32_t lo[8], hi[8];
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const uint32_t q = b.word(O + kNext * i + 1 + 4 * k);
+        e2m1_halves(((q << 1) & 0x0E0E0E0Eu) | ((q << 4) & kTops), fh, lo[2 * k], lo[2 * k + 1]);
+        e2m1_halves(((q >> 3) & 0x0E0E0E0Eu) | (q & kTops), fh, hi[2 * k], hi[2 * k + 1]);
+      }
+      put(2u * i, lo), put(2u * i + 1u, hi);
+    }
+  } else {
+    const uint32_t h0 = b.half(O), h1 = b.half(O + kNext);
+    if (__any_sync(0xFFFFFFFFu, inf_or_nan(h0) || inf_or_nan(h1))) return false;
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+      const float d = half_value(i ? h1 : h0);
+      uint32_t lo[8], hi[8];
+      if constexpr (T == QTYPE_Q4_0) {  // (the high nibbles where they lie: 16 n under a sixteenth of the scale)
+        const Affine a(d, mul_rn(d, -8.0f)), b16(mul_rn(d, 0.0625f), mul_rn(d, -8.0f));
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          const uint32_t q = b.word(O + kNext * i + 2 + 4 * k), q8 = q >> 8;
+          a.halves(q & 0x000F000Fu, q8 & 0x000F000Fu, lo[2 * k], lo[2 * k + 1]);
+          b16.halves(q & 0x00F000F0u, q8 & 0x00F000F0u, hi[2 * k], hi[2 * k + 1]);
+        }
+      } else {  // Q8_0: the signed byte as q + 128
+        const Affine a(d, mul_rn(d, -128.0f));
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          a.bytes(b.word(O + kNext * i + 2 + 4 * k) ^ kTops, lo[2 * k], lo[2 * k + 1]);
+          a.bytes(b.word(O + kNext * i + 18 + 4 * k) ^ kTops, hi[2 * k], hi[2 * k + 1]);
+        }
+      }
+      put(2u * i, lo), put(2u * i + 1u, hi);
+    }
+  }
+  return true;
+}
+// ... of step SUB, whose K block starts A bytes (0 or 8) into a 16-byte piece
+template <uint32_t T, int SUB, int A, class Put>
+__device__ __forceinline__ bool two_blocks_at(uint32_t piece, const Put& put) {
+  constexpr int kFrom = A + SUB * 2 * Fmt<T>::bytes, kTo = kFrom + 2 * Fmt<T>::bytes, kPiece = kFrom / 16;
+  Pieces<(kTo + 15) / 16 - kPiece> b;
+  b.load(piece + 16u * kPiece);
+  return two_blocks<T, kFrom - 16 * kPiece>(b, put);
+}
+template <uint32_t T, int A, class Put>
+__device__ __forceinline__ bool two_blocks_in(uint32_t piece, uint32_t sub, const Put& put) {
+  if (sub == 0) return two_blocks_at<T, 0, A>(piece, put);
+  if constexpr (kRawK<T> == 256) {
+    if (sub == 2) return two_blocks_at<T, 2, A>(piece, put);
+    if (sub == 3) return two_blocks_at<T, 3, A>(piece, put);
+  }
+  return two_blocks_at<T, 1, A>(piece, put);
+}
+
+template <bool HI, class Put>  // Q6_K: HI, the step whose nibbles are the high ones
+__device__ __forceinline__ void q6_step(uint32_t at, uint32_t sub, float d, const Put& put) {
+  const uint32_t ql = at + 64u * (sub >> 1), qh = at + 128u + 32u * (sub >> 1);
+#pragma unroll
+  for (uint32_t i = 0; i < 2; i++) {
+    Moved<16> top;
+    top.load(qh + 16u * i);
+#pragma unroll
+    for (uint32_t b = 0; b < 2; b++) {  // sub-blocks 2 sub, 2 sub + 1: their top bit pairs at bits 4 HI + 2 b of the same bytes
+      Moved<16> low;
+      uint32_t r[8];
+      low.load(ql + 32u * b + 16u * i);
+      const float ds = mul_rn(d, (float) (int) (int8_t) lds8(at + 192u + 4u * sub + 2u * b + i));
+      const Affine a(ds, mul_rn(ds, -32.0f));
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const uint32_t n = HI ? low.w[k] >> 4 : low.w[k];
+        const uint32_t t = HI ? (b ? top.w[k] >> 2 : top.w[k]) : (b ? top.w[k] << 2 : top.w[k] << 4);
+        a.bytes((n & kLow4) | (t & 0x30303030u), r[2 * k], r[2 * k + 1]);
+      }
+      put(2u * b + i, r);
+    }
+  }
+}
+
+template <uint32_t T, class Put>
+__device__ __forceinline__ void decode_step(uint32_t at, const uint8_t* p, uint32_t sub, const Grids& g, const Put& put) {
+  if constexpr (T == QTYPE_Q4_K || T == QTYPE_Q5_K) {
+    // the step is groups 2 sub and 2 sub + 1: the low and the high nibbles of the same 32 bytes
+    const bool whole = __all_sync(0xFFFFFFFFu, (at & 15u) == 0);
+    uint4 h = make_uint4(0x7C00u, 0, 0, 0);
+    if (__all_sync(0xFFFFFFFFu, (at & 3u) == 0)) h = lds_16(at, whole);
+    if (__any_sync(0xFFFFFFFFu, inf_or_nan(h.x) || inf_or_nan(h.x >> 16))) return decode_step_any<T>(p, sub, g, put);
     uint32_t sc, mn;
-    k_scales(p.h[1], p.h[2], p.h[3], 16u * (g & 1u), g >= 2u, sc, mn);
-    const float d = half_value(p.h[0] & 0xFFFFu), m = -half_value(p.h[0] >> 16);
-    const uint64_t ds = mul2(pack2(d, d), pack2(byte_value<0>(sc), byte_value<1>(sc)));
-    const uint64_t dm = mul2(pack2(m, m), pack2(byte_value<0>(mn), byte_value<1>(mn)));  // (minus the minimum)
-    uint2 a = make_uint2(q.x & kLow4, q.y & kLow4), b = make_uint2((q.x >> 4) & kLow4, (q.y >> 4) & kLow4);
-    if constexpr (T == QTYPE_Q5_K) {  // the fifth bits: bits 2 g and 2 g + 1 of the 32 bytes at 16
-      const uint32_t f0 = p.f.x >> (2u * g), f1 = p.f.y >> (2u * g);
-      a.x |= (f0 & kOnes) << 4, a.y |= (f1 & kOnes) << 4, b.x |= (f0 << 3) & 0x10101010u, b.y |= (f1 << 3) & 0x10101010u;
-    }
-    uint64_t v[8];
-    code_pairs(a, b, -32768.0f, v);
+    k_scales(h.y, h.z, h.w, 16u * (sub & 1u), sub >= 2u, sc, mn);
+    const float d = half_value(h.x & 0xFFFFu), m = -half_value(h.x >> 16);
+    const float s0 = mul_rn(d, byte_value<0>(sc)), s1 = mul_rn(d, byte_value<1>(sc));
+    const float m0 = mul_rn(m, byte_value<0>(mn)), m1 = mul_rn(m, byte_value<1>(mn));  // (minus the minimum)
+    if constexpr (T == QTYPE_Q4_K) {  // (the high nibbles where they lie: 16 n under a sixteenth of the scale)
+      const Affine a(s0, m0), b(mul_rn(s1, 0.0625f), m1);
 #pragma unroll
-    for (int j = 0; j < 8; j++) v[j] = add2(mul2(ds, v[j]), dm);
-    store_pairs(v, lo, hi);
+      for (uint32_t i = 0; i < 2; i++) {
+        const uint4 q = lds_16(at + 16u + 32u * sub + 16u * i, whole);
+        const uint32_t qw[4] = {q.x, q.y, q.z, q.w};
+        uint32_t lo[8], hi[8];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          const uint32_t q8 = qw[k] >> 8;
+          a.halves(qw[k] & 0x000F000Fu, q8 & 0x000F000Fu, lo[2 * k], lo[2 * k + 1]);
+          b.halves(qw[k] & 0x00F000F0u, q8 & 0x00F000F0u, hi[2 * k], hi[2 * k + 1]);
+        }
+        put(i, lo), put(2u + i, hi);
+      }
+    } else {
+      const Affine a(s0, m0), b(s1, m1);
+#pragma unroll
+      for (uint32_t i = 0; i < 2; i++) {
+        const uint4 q = lds_16(at + 48u + 32u * sub + 16u * i, whole), f = lds_16(at + 16u + 16u * i, whole);
+        const uint32_t qw[4] = {q.x, q.y, q.z, q.w};  // the fifth bits: bits 2 sub and 2 sub + 1 of the 32 bytes at 16
+        const uint32_t fw[4] = {f.x >> (2u * sub), f.y >> (2u * sub), f.z >> (2u * sub), f.w >> (2u * sub)};
+        uint32_t lo[8], hi[8];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          a.bytes((qw[k] & kLow4) | ((fw[k] << 4) & 0x10101010u), lo[2 * k], lo[2 * k + 1]);
+          b.bytes(((qw[k] >> 4) & kLow4) | ((fw[k] << 3) & 0x10101010u), hi[2 * k], hi[2 * k + 1]);
+        }
+        put(i, lo), put(2u + i, hi);
+      }
+    }
+  } else if constexpr (T == QTYPE_Q4_0 || T == QTYPE_MXFP4 || T == QTYPE_Q8_0) {
+    // (rows of whole 16-byte pieces lie alike: the places of the step's bytes are then known when compiled)
+    bool done;
+    if (__all_sync(0xFFFFFFFFu, (at & 15u) == 0)) {
+      done = two_blocks_in<T, 0>(at, sub, put);
+    } else if (__all_sync(0xFFFFFFFFu, (at & 15u) == 8u)) {
+      done = two_blocks_in<T, 8>(at & ~15u, sub, put);
+    } else {
+      Moved<2 * Fmt<T>::bytes> b;
+      b.load(at + sub * 2u * Fmt<T>::bytes);
+      done = two_blocks<T, 0>(b, put);
+    }
+    if (!done) decode_step_any<T>(p, sub, g, put);
+  } else if constexpr (T == QTYPE_Q6_K) {
+    const uint32_t h = lds_half(at + 208u);
+    if (__any_sync(0xFFFFFFFFu, inf_or_nan(h))) return decode_step_any<T>(p, sub, g, put);
+    if (sub & 1u) q6_step<true>(at, sub, half_value(h), put);
+    else q6_step<false>(at, sub, half_value(h), put);
+  } else {
+    decode_step_any<T>(p, sub, g, put);
   }
 }
 
@@ -259,9 +368,9 @@ struct Args {
   const __half* x16;
   float* y;
   uint32_t rows, cols, n, xts, ys;
-  uint32_t accs;  // accumulators (128 tokens each) a block: 1, 2 or 4
+  uint32_t n_mat, row_tiles;
+  uint32_t span;     // the most tokens a tile takes
   uint32_t use_tma;  // the activations come by tensor-map copies (mm_run), else by 16-byte cp.async (mm_group)
-  uint32_t stages, stage_bytes, raw_off;  // the operand ring's depth, a stage's bytes; where the raw weight buffers start
   float scale;
   uint32_t* status;
   // the epilogue (the kernel's EPI): kStore y = scale sum; kSilu y = silu(scale sum), and its f16 into x16_out (rows wide, tiled);
@@ -271,360 +380,411 @@ struct Args {
   int32_t* overflow;
   const float* xn;
   float* out;
-  uint32_t hc, dim, per, out_row0;  // per: the dim values a block takes (hc per <= 128 rows of its tile are used)
+  uint32_t hc, dim, per, out_row0;  // per: the dim values a tile takes (hc per <= 128 of its rows are used)
+};
+struct Maps {  // the tokens' maps: of a grouped launch map t a box of t + 1 token tiles, else the one map's box is a.span tokens
+  CUtensorMap map[kMaxSpan / MM_TILE];
 };
 enum : uint32_t { kStore = 0, kSilu = 1, kGatedMean = 2 };
 
 struct Shared {
-  uint64_t full_a[kMaxStages], full_b[kMaxStages], empty[kMaxStages], done;
-  uint32_t tmem_base;
-  int fail;
+  // of a unit - one K step or two - full_a: their weights are in tensor memory; full_b: their tokens in shared memory; empty: their products
+  // have run (so the weights' stages, and the tokens' slot of the token ring, are free)
+  uint64_t full_a[kSteps], full_b[kSteps], empty[kSteps], full_raw[4], empty_raw[4], full_acc[2], empty_acc[2], drain;
+  uint32_t tmem_base, max_tok, warp_tiles[kThreads / kWarp], warp_tok[kThreads / kWarp];
+  int fail, epi_fail;
 };
+
+__host__ __device__ constexpr uint32_t whole16(uint32_t n) { return (n + 15u) & ~15u; }
+__host__ __device__ constexpr uint32_t parts_of(uint32_t n, uint32_t of) { return (n + of - 1u) / of; }
+
+// Tile number t of the launch: tiles go matrix by matrix, row tile by row tile, a row tile's token tiles side by side (they
+// share the weights' bytes in L2). first[m]: matrix m's first tile; m: where the last search ended (a role's tiles only
+// go up). A matrix's tokens are dealt in equal whole tiles of 16.
+struct Tile {
+  uint32_t m, rt, c0, n;  // its matrix and row tile; its first token and their number
+};
+__device__ __forceinline__ Tile tile_at(const Args& a, const uint32_t* first, uint32_t t, uint32_t& m, uint32_t lane) {
+  if (a.wt) {
+    for (;;) {
+      const uint32_t i = m + 1u + lane;
+      const uint32_t past = __popc(__ballot_sync(0xFFFFFFFFu, first[i < a.n_mat ? i : a.n_mat] <= t && i <= a.n_mat));
+      m += past;
+      if (past < 32u) break;
+    }
+  }
+  const uint32_t n = a.wt ? (uint32_t) a.cnt[m] : a.n, in = t - first[m], cols = parts_of(n, a.span);
+  const uint32_t each = whole16(parts_of(n, cols));
+  Tile r;
+  r.m = m, r.rt = in / cols, r.c0 = (in - r.rt * cols) * each;
+  r.n = r.c0 < n ? min(each, n - r.c0) : 0u;
+  return r;
+}
 
 // EPI: the epilogue (kStore / kSilu / kGatedMean), a compile-time choice so that the plain product carries none of
 // the others' code
 template <uint32_t T, uint32_t EPI>
-__global__ void __launch_bounds__(kThreads, 1) mm_tc_kernel(const Args a, const __grid_constant__ CUtensorMap tmap) {
+__global__ void __launch_bounds__(kThreads, 1) mm_tc_kernel(const Args a, const __grid_constant__ Maps maps) {
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ Shared sh;
   __shared__ __align__(16) uint8_t tables[grid_smem_bytes<T>() > 0 ? grid_smem_bytes<T>() : 16];
   const uint32_t tid = threadIdx.x, lane = tid % kWarp, warp = tid / kWarp;
-  const uint32_t m = blockIdx.y, row0 = blockIdx.x * kM, span = a.accs * kN, c0 = blockIdx.z * span;
-  const uint32_t n_tok = a.wt ? (uint32_t) (a.cnt[m] > 0 ? a.cnt[m] : 0) : a.n;
-  if (c0 >= n_tok) return;  // the whole block, before anything is allocated
-  const uint32_t n_valid = n_tok - c0 < span ? n_tok - c0 : span;
-  const uint32_t n_valid16 = (n_valid + 15u) & ~15u;  // x16 holds whole tiles of 16 tokens
-  const uint32_t n_acc = (n_valid + kN - 1) / kN;
   const uint32_t steps = a.cols / kStep;
   const uint64_t row_bytes = (uint64_t) (a.cols / Fmt<T>::values) * Fmt<T>::bytes;
-  const uint8_t* w = a.wt ? a.wt[m] : a.w;
-  // the weight row behind row r of the block's tile: the matrix's next 128 rows - or, for the gated mean, stream
-  // r / per's row of value d0 + r % per, so the hc sums of one output value lie in one block (a row past the matrix,
-  // or past the streams, repeats a valid one and is never stored)
-  const uint32_t d0 = blockIdx.x * a.per;
-  auto wrow = [&](uint32_t r) -> uint32_t {
-    if constexpr (EPI != kGatedMean) return row0 + r < a.rows ? row0 + r : a.rows - 1;
-    const uint32_t st = r / a.per, d = d0 + (r - st * a.per);
-    return (st < a.hc ? st : a.hc - 1) * a.dim + (d < a.dim ? d : a.dim - 1);
-  };
-  const __half* x16 = a.x16 + (a.wt ? a.xoff[m] : 0u);
-  float* y = a.y + (a.wt ? a.yoff[m] : 0u);
+  constexpr uint32_t kStepsRaw = kRawK<T> / kStep, kSlot = kRawSlot<T>;
+  const uint32_t kblocks = parts_of(steps, kStepsRaw);
+  uint32_t* const first = (uint32_t*) (smem + kFirstAt<T, EPI>);
+  uint8_t* const raw = smem + kRawAt<T, EPI>;
 
   if (tid == 0) {
-    for (int i = 0; i < kMaxStages; i++) bar_init(&sh.full_a[i], kProdWarps / kGroups), bar_init(&sh.full_b[i], a.use_tma ? 1u : (uint32_t) kLoaderThreads), bar_init(&sh.empty[i], 1);
-    bar_init(&sh.done, 1);
-    sh.fail = 0;
+    for (uint32_t i = 0; i < kSteps; i++) bar_init(&sh.full_b[i], 1), bar_init(&sh.empty[i], 1);
+    for (int i = 0; i < 4; i++)
+      bar_init(&sh.full_raw[i], kRawWarps * kWarp), bar_init(&sh.empty_raw[i], (kProdWarps / kTeams) * kStepsRaw);
+    for (int i = 0; i < 2; i++) bar_init(&sh.full_acc[i], 1), bar_init(&sh.empty_acc[i], kEpiWarps);
+    bar_init(&sh.drain, 1);
+    sh.fail = 0, sh.epi_fail = 0;
     bar_init_fence();
   }
   if (warp == (uint32_t) kIssuerWarp) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&sh.tmem_base)), "r"(512));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
+  // the matrices' first tiles, a thread each, and the most tokens a tile has
+  const uint32_t n_mat = a.wt ? a.n_mat : 1u;
+  static_assert(kMaxMats <= (uint32_t) kThreads, "a thread a matrix");
+  {
+    const uint32_t n = tid < n_mat ? (a.wt ? (uint32_t) max(a.cnt[tid], 0) : a.n) : 0u, cols = parts_of(n, a.span);
+    const uint32_t mine = cols * a.row_tiles, most = __reduce_max_sync(0xFFFFFFFFu, n ? whole16(parts_of(n, cols)) : 0u);
+    uint32_t sum = mine;
+#pragma unroll
+    for (int o = 1; o < kWarp; o <<= 1) {
+      const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, sum, o);
+      if (lane >= (uint32_t) o) sum += v;
+    }
+    if (lane == kWarp - 1u) sh.warp_tiles[warp] = sum, sh.warp_tok[warp] = most;
+    __syncthreads();
+    uint32_t before = lane < warp ? sh.warp_tiles[lane] : 0u;
+    before = __reduce_add_sync(0xFFFFFFFFu, before);
+    if (tid < n_mat) first[tid] = before + sum - mine;
+    if (tid == n_mat - 1u) first[n_mat] = before + sum;
+    const uint32_t tok = __reduce_max_sync(0xFFFFFFFFu, lane < (uint32_t) (kThreads / kWarp) ? sh.warp_tok[lane] : 0u);
+    // the issuer goes by units: two steps where a tile is small and their products run shorter than a look at the barriers
+    if (tid == 0) {
+      sh.max_tok = tok;
+      for (uint32_t i = 0; i < kSteps; i++) bar_init(&sh.full_a[i], (tok > (uint32_t) kN ? 1u : 2u) * kProdWarps / kTeams);
+      bar_init_fence();
+    }
+  }
   const Grids g = stage_grids<T>(tables);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = sh.tmem_base;
-  const uint32_t S = a.stages;
+  const uint32_t tiles = first[n_mat];
+  // the token ring: slots of a unit's K steps of the largest tile's tokens, as many as fit, at most one a barrier (the products of
+  // an odd number of token tiles read one past the last)
+  const uint32_t slot_tiles = sh.max_tok ? sh.max_tok / MM_TILE : 1u, two = slot_tiles * MM_TILE > (uint32_t) kN ? 0u : 1u;  // (log2 of a unit's steps)
+  const uint32_t units = kSteps >> two, unit_subs = kSubs << two;
+  const uint32_t slot_bytes = (slot_tiles * unit_subs + (slot_tiles & 1u)) * 512u, slots = min(units, kTokenRing<EPI> / slot_bytes);
+  uint32_t m_at = 0;  // (tile_at's)
 
-  if (producer_of((int) warp) >= 0) {
+  if (warp >= (uint32_t) kFirstProd && warp < (uint32_t) kIssuerWarp) {
     // ================= producers =================
-    // The rows' bytes come through shared memory kRawK values of K at a time: 16-byte cp.async pieces of the aligned
-    // span around each row's bytes (a block may start anywhere in a 16-byte piece), two buffers, the next block's values
-    // on their way while these are decoded - so the decoders' many narrow reads are shared-memory reads.
-    const uint32_t pt = (uint32_t) producer_of((int) warp) * kWarp + lane;
-    constexpr uint32_t kKb = kRawK<T>, kKbBytes = kRawBytes<T>, kSlot = kRawSlot<T>;
-    constexpr uint32_t kPieces = (kKbBytes + 30u + 15u) / 16u;  // (the slot may be one piece longer: an odd count)
-    uint8_t* raw = smem + a.raw_off;
-    const uint8_t* w_end = w + (uint64_t) a.rows * row_bytes;
-    const uint32_t kblocks = (a.cols + kKb - 1) / kKb;
-    // this thread's pieces: where their rows start, worked out once (a 64-bit product a row), and their place in a buffer
-    constexpr int kFetch = (int) ((kM * kPieces + kProdThreads - 1) / kProdThreads);
-    const uint8_t* fetch_row[kFetch];
-    uint32_t fetch_at[kFetch];  // (a piece past the rows' last: none)
-#pragma unroll
-    for (int j = 0; j < kFetch; j++) {
-      const uint32_t i = pt + (uint32_t) j * kProdThreads, r = i / kPieces, piece = i - r * kPieces;
-      fetch_row[j] = i < (uint32_t) kM * kPieces ? w + wrow(r) * row_bytes : nullptr;
-      fetch_at[j] = r * kSlot + piece * 16u;
-    }
-    auto fetch_raw = [&](uint32_t kb) {  // the rows' bytes of K block kb into buffer kb % 2
-      const uint32_t buf = smem_addr(raw) + (kb & 1u) * (kM * kSlot);
-#pragma unroll
-      for (int j = 0; j < kFetch; j++) {
-        if (!fetch_row[j]) continue;
-        const uint8_t* src = (const uint8_t*) ((uintptr_t) (fetch_row[j] + (uint64_t) (kb * kKbBytes)) & ~(uintptr_t) 15) + fetch_at[j] % kSlot;
-        const int64_t left = w_end - src;
-        const uint32_t have = left >= 16 ? 16u : left > 0 ? (uint32_t) left : 0u;  // (zero fill past the tensor)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(buf + fetch_at[j]), "l"(src), "r"(have) : "memory");
-      }
-      asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    // this thread's chunks of a step: chunk kc of rows 64 apart (eight neighbouring threads take one K piece of eight
-    // neighbouring rows - eight different 16-byte bank columns of the operand tile, and of the raw buffer, whose row
-    // slots are an odd number of 16-byte pieces); what does not change from step to step is worked out here
-    constexpr uint32_t kChunks = kPairChunk<T> ? kStep / 16 : kStep / 8;  // a row's of a step: pairs, or chunks
-    constexpr int kMine = kM * (int) kChunks / kTeamThreads;
-    static_assert(kMine * kTeamThreads == kM * (int) kChunks && kTeamThreads % (8 * kChunks) == 0, "every producer thread the same number of chunks");
-    const uint32_t team = pt / kTeamThreads, tt = pt % kTeamThreads;  // the thread's team and its place in it
-    const uint32_t kc = (tt >> 3) % kChunks;
-    // (a pair's first chunk; its second is two on in a 32-value block, four on where the pair is two groups of 32)
-    const uint32_t kc0 = !kPairChunk<T> || kPairOfGroups<T> ? kc : 4u * (kc >> 1) + (kc & 1u);
-    constexpr uint32_t kSecond = (kPairOfGroups<T> ? 2u : 1u) * kSubTile;
-    uint32_t slot_at[kMine], dst_at[kMine], base15[kMine];
-#pragma unroll
-    for (int u = 0; u < kMine; u++) {
-      const uint32_t task = tt + (uint32_t) u * kTeamThreads, r = task / (8 * kChunks) * 8u + (task & 7u);
-      const uint32_t row = wrow(r);  // (a row past the matrix repeats the last one)
-      slot_at[u] = r * kSlot, dst_at[u] = (kc0 >> 1) * kSubTile + (r >> 3) * 256 + (kc0 & 1u) * 128 + (r & 7u) * 16;
-      base15[u] = (uint32_t) ((uintptr_t) (w + row * row_bytes) & 15u);
-    }
-    bool dead = false;  // a wait ran out: no more work, but the producers' own barrier is still kept
-    fetch_raw(0);
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    static_assert((kKb / kStep) % kGroups == 0, "every team has steps in every K block");
-    uint32_t stage = team % S, use = team / S;  // step it's stage and how often it has been used before
-    for (uint32_t it = team; it < steps; it += kGroups, stage += kGroups) {
-      if (stage >= S) stage -= S, use++;  // (a ring is two stages at least)
-      const uint32_t kb = it / (kKb / kStep), sub = it % (kKb / kStep);
-      const bool first = sub == team;  // the team's first step of K block kb
-      if (first) {  // this thread's pieces of block kb have landed; after the barrier everyone's have, and block
-        asm volatile("cp.async.wait_group 0;" ::: "memory");  // kb - 1's buffer is free for kb + 1
-        asm volatile("bar.sync 1, %0;" ::"n"(kProdThreads) : "memory");
-      }
-      if (!dead && use > 0 && !bar_wait(&sh.empty[stage], (use - 1) & 1u)) sh.fail = 1, dead = true;
-      if (dead) continue;
-      if (first && kb + 1 < kblocks) fetch_raw(kb + 1);
-      // A: the chunk decoded to 8 halves, 16 bytes, to sub-tile kc / 2 of the stage
-      uint8_t* sa = smem + stage * a.stage_bytes;
-      const uint8_t* buf = raw + (kb & 1u) * (kM * kSlot);
-      const uint32_t kb15 = (kb * kKbBytes) & 15u;
-      if constexpr (kPairChunk<T>) {
-        const uint32_t in_blk = kPairOfGroups<T> ? 0u : (sub * (kStep / 32) + (kc >> 1)) * Fmt<T>::bytes;
-        uint32_t at[kMine];
-        bool whole = true;  // (of Q4_K and Q5_K: the thread's blocks start on words, as they do in a matrix that does)
-#pragma unroll
-        for (int u = 0; u < kMine; u++) {
-          at[u] = smem_addr(buf) + slot_at[u] + ((base15[u] + kb15) & 15u) + in_blk;
-          if (kPairOfGroups<T> && (at[u] & 3u)) whole = false;
-        }
-        uint4 lo[kMine], hi[kMine];
-        if (whole) {
-          PairBytes raw_pair[kMine];
-#pragma unroll
-          for (int u = 0; u < kMine; u++) load_pair<T>(at[u], sub, kc, raw_pair[u]);
-#pragma unroll
-          for (int u = 0; u < kMine; u++) pair_chunks<T>(raw_pair[u], sub, lo[u], hi[u]);
-        } else if constexpr (kPairOfGroups<T>) {
-#pragma unroll
-          for (int u = 0; u < kMine; u++) {
-            const uint8_t* blk = buf + (at[u] - smem_addr(buf));
-            float v[kChunk];
-            decode8<T>(blk, (int) (8u * sub + kc), v, g);
-            lo[u] = make_uint4(half2_bits(v[0], v[1]), half2_bits(v[2], v[3]), half2_bits(v[4], v[5]), half2_bits(v[6], v[7]));
-            decode8<T>(blk, (int) (8u * sub + 4u + kc), v, g);
-            hi[u] = make_uint4(half2_bits(v[0], v[1]), half2_bits(v[2], v[3]), half2_bits(v[4], v[5]), half2_bits(v[6], v[7]));
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < kMine; u++) *(uint4*) (sa + dst_at[u]) = lo[u], *(uint4*) (sa + dst_at[u] + kSecond) = hi[u];
+    const uint32_t team = (warp - kFirstProd) / 4u, r = 32u * (warp % 4u) + lane;
+    const uint32_t lane_cols = tmem + ((32u * (warp % 4u)) << 16) + kAccCols;
+    uint32_t s0 = 0, rb0 = 0;  // the steps and raw blocks before this tile
+    bool ok = true;
+    for (uint32_t t = blockIdx.x; t < tiles && ok; t += gridDim.x, s0 += steps, rb0 += kblocks) {
+      const Tile tl = tile_at(a, first, t, m_at, lane);
+      const uint8_t* w = a.wt ? a.wt[tl.m] : a.w;
+      // (the weight row behind row r of the tile: see the raw loaders; here only where it starts in its 16-byte piece)
+      uint32_t row;
+      if constexpr (EPI == kGatedMean) {
+        const uint32_t d0 = tl.rt * a.per, st = r / a.per, d = d0 + (r - st * a.per);
+        row = (st < a.hc ? st : a.hc - 1) * a.dim + (d < a.dim ? d : a.dim - 1);
       } else {
-        const uint32_t cl = sub * (kStep / kChunk) + kc;  // the chunk's index in its K block
-        const uint32_t in_blk = (cl / Fmt<T>::chunks) * Fmt<T>::bytes, k_in = cl % Fmt<T>::chunks;
-#pragma unroll
-        for (int u = 0; u < kMine; u++) {
-          const uint8_t* blk = buf + slot_at[u] + ((base15[u] + kb15) & 15u) + in_blk;
-          uint4 out;
-          if constexpr (kFastChunk<T>) {
-            out = fast_chunk<T>(blk, k_in);
-          } else {
-            float v[kChunk];
-            decode8<T>(blk, (int) k_in, v, g);
-            out.x = half2_bits(v[0], v[1]), out.y = half2_bits(v[2], v[3]);
-            out.z = half2_bits(v[4], v[5]), out.w = half2_bits(v[6], v[7]);
-          }
-          *(uint4*) (sa + dst_at[u]) = out;
-        }
+        row = min(tl.rt * kM + r, a.rows - 1u);
       }
-      fence_async_smem();  // these writes before the tensor core's reads
-      __syncwarp();
-      if (lane == 0) bar_arrive(&sh.full_a[stage]);  // (one arrival a warp: 512 would queue on the one word)
-    }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-  } else if (loader_of((int) warp) >= 0) {
-    // ================= the activations' loader =================
-    // token n's 8-value piece kc of step `it`, 16 bytes, to sub-tile (n / 128, kc / 2) of the step's stage; the warp
-    // never waits for its own copies: each thread's arrival on the stage's barrier is made by the hardware when that
-    // thread's copies have landed, so the loads run as far ahead of the tensor core as the ring is deep
-    const uint32_t lt = (uint32_t) loader_of((int) warp) * kWarp + lane;
-    if (a.use_tma) {
-      // One warp, a tensor-map copy a (128 tokens, 16 values of K) sub-tile: the tiled x16 seen as [token tile][K
-      // fragment][token in tile][value in fragment], a box of 8 tiles x 1 fragment written with the 32-byte swizzle the
-      // MMA reads (tiles past the last are filled with zeros); the stage's barrier counts the bytes.
-      if (lt < (uint32_t) kWarp) {
-        const uint32_t ops = n_acc * kSubs;
-        uint32_t stage = 0, use = 0;
-        for (uint32_t it = 0; it < steps; it++, stage++) {
-          if (stage == S) stage = 0, use++;
-          if (use > 0 && !bar_wait(&sh.empty[stage], (use - 1) & 1u)) {
-            sh.fail = 1;
-            break;
-          }
-          if (lt == 0) bar_expect(&sh.full_b[stage], ops * kSubTile);
-          __syncwarp();
-          if (lt < ops) {
-            const uint32_t acc = lt / kSubs, q = lt % kSubs;
-            const uint32_t dst = smem_addr(smem + stage * a.stage_bytes + kStageA) + (acc * kSubs + q) * kSubTile;
-            asm volatile(
-                "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(dst),
-                "l"(&tmap), "r"(0), "r"(0), "r"(it * kSubs + q), "r"(c0 / MM_TILE + acc * (kN / MM_TILE)), "r"(smem_addr(&sh.full_b[stage]))
-                : "memory");
-          }
-        }
-      }
-    } else {
-      // (eight neighbouring threads: one K piece of eight neighbouring tokens - eight different 16-byte bank columns of the
-      // operand tile, so a store takes no more passes than its bytes need.) A thread's pieces are one K piece of every
-      // sixteenth token: a tile of x16 on, 512 bytes on in the operand, to the next accumulator's part every 128 tokens.
-      const uint32_t kc = (lt >> 3) & 7u, n0 = (lt >> 6) * 8u + (lt & 7u);
-      static_assert(kLoaderThreads == 128 && MM_TILE == 16, "a round of pieces is sixteen tokens");
-      const __half* src0 = x16 + mm_x16_at(c0 + n0, kc * 8, a.xts);
-      const uint64_t step_halves = mm_x16_at(0, kStep, a.xts), tile_halves = mm_x16_at(MM_TILE, 0, a.xts);
-      const uint32_t dst0 = (kc >> 1) * kSubTile + (n0 >> 3) * 256 + (kc & 1u) * 128 + (n0 & 7u) * 16;
-      uint32_t stage = 0, use = 0;
-      for (uint32_t it = 0; it < steps; it++, stage++, src0 += step_halves) {
-        if (stage == S) stage = 0, use++;
-        if (use > 0 && !bar_wait(&sh.empty[stage], (use - 1) & 1u)) {
-          sh.fail = 1;
+      const uint32_t base15 = (uint32_t) ((uintptr_t) (w + (uint64_t) row * row_bytes) & 15u);
+      for (uint32_t it = (team - s0) % kTeams; it < steps; it += kTeams) {
+        const uint32_t s = s0 + it, stage = s % kSteps, unit = stage >> two, kb = it / kStepsRaw, sub = it % kStepsRaw, rb = rb0 + kb, slot = rb % kRawStages<T>;
+        if (!bar_wait_soon(&sh.full_raw[slot], (rb / kRawStages<T>) & 1u) ||
+            (s >= kSteps && !bar_wait_soon(&sh.empty[unit], (s / kSteps - 1u) & 1u))) {
+          ok = false;
           break;
         }
-        const uint32_t sb = smem_addr(smem + stage * a.stage_bytes + kStageA) + dst0;
-        const __half* src = src0;
-        for (uint32_t n = 0; n < n_valid16; n += 16, src += tile_halves)
-          cp_async16(sb + (n / kN) * (kSubs * kSubTile) + (n % kN) * 32, src);
-        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_addr(&sh.full_b[stage])) : "memory");
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t off = slot * (kM * kSlot) + r * kSlot + ((base15 + kb * kRawBytes<T>) & 15u);
+        const uint32_t col = lane_cols + stage * kStageCols;
+        decode_step<T>(smem_addr(raw) + off, raw + off, sub, g, [&](uint32_t q, const uint32_t (&v)[8]) {
+          asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(col + 8u * q), "r"(v[0]), "r"(v[1]),
+                       "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                       : "memory");
+        });
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) {
+          bar_arrive(&sh.full_a[unit]);
+          // (the raw block's last step arrives for those a row's end leaves out)
+          bar_arrive_n(&sh.empty_raw[slot], it == steps - 1u ? kStepsRaw - sub : 1u);
+        }
       }
     }
+    if (!ok) sh.fail = 1;
+  } else if (warp >= (uint32_t) kFirstRaw && warp < (uint32_t) kTokenWarp) {
+    // ================= the weights' loaders =================
+    // The 16-byte pieces of the aligned span around each row's bytes (a block may start anywhere in a piece; every piece
+    // asked for holds some of them). Where all rows start at the same place in a piece, 64 threads take the pieces of
+    // kTogether rows in kRounds rounds whose places do not change from block to block: three instructions a copy. (A
+    // loader that worked a row's address out a copy held a K step to 1,000 cycles.)
+    constexpr uint32_t kP = kRawPieces<T>, kLoaders = kRawWarps * kWarp;
+    constexpr uint32_t kTogether = kP % 64u == 0 ? 1u : kP % 32u == 0 ? 2u : kP % 16u == 0 ? 4u : kP % 8u == 0 ? 8u : kP % 4u == 0 ? 16u : kP % 2u == 0 ? 32u : 64u;
+    constexpr uint32_t kRounds = kTogether * kP / kLoaders;
+    static_assert(kP <= 16u && kP * 16u <= kSlot && kRounds * kLoaders == kTogether * kP && kM % kTogether == 0, "the rows' pieces");
+    const uint32_t lt = (warp - kFirstRaw) * kWarp + lane;
+    const bool alike = EPI != kGatedMean && row_bytes % 16u == 0 && row_bytes < (1u << 24);
+    uint32_t src_at[kRounds], dst_at[kRounds];
+#pragma unroll
+    for (uint32_t j = 0; j < kRounds; j++) {
+      const uint32_t i = lt + j * kLoaders, r = i / kP, piece = i - r * kP;
+      src_at[j] = r * (uint32_t) row_bytes + piece * 16u, dst_at[j] = r * kSlot + piece * 16u;
+    }
+    uint32_t rb = 0;
+    bool ok = true;
+    for (uint32_t t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
+      const Tile tl = tile_at(a, first, t, m_at, lane);
+      const uint8_t* w = a.wt ? a.wt[tl.m] : a.w;
+      for (uint32_t kb = 0; kb < kblocks; kb++, rb++) {
+        const uint32_t slot = rb % kRawStages<T>;
+        if (rb >= kRawStages<T> && !bar_wait_soon(&sh.empty_raw[slot], (rb / kRawStages<T> - 1u) & 1u)) {
+          ok = false;
+          break;
+        }
+        const uint32_t dst = smem_addr(raw) + slot * (kM * kSlot);
+        const uint64_t in_row = (uint64_t) kb * kRawBytes<T>;
+        const uint32_t bytes = row_bytes - in_row < kRawBytes<T> ? (uint32_t) (row_bytes - in_row) : kRawBytes<T>;
+        if (alike) {  // (rows past the matrix are left out: whatever their lanes hold is never stored)
+          const uint32_t row0 = tl.rt * kM, live = min(a.rows - row0, (uint32_t) kM);
+          const uint8_t* from = w + (uint64_t) row0 * row_bytes + in_row;
+          const uint32_t need = (((uint32_t) (uintptr_t) from & 15u) + bytes + 15u) / 16u * 16u;
+          const uint8_t* src = (const uint8_t*) ((uintptr_t) from & ~(uintptr_t) 15);
+          for (uint32_t r0 = 0; r0 < live; r0 += kTogether, src += kTogether * row_bytes) {
+#pragma unroll
+            for (uint32_t j = 0; j < kRounds; j++) {
+              const uint32_t to = dst_at[j];
+              if (to % kSlot < need && r0 + to / kSlot < live)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + r0 * kSlot + to), "l"(src + src_at[j]) : "memory");
+            }
+          }
+        } else {  // a half-warp a row, four rows a round
+          const uint32_t piece = lt % 16u;
+          for (uint32_t r = lt / 16u; r < (uint32_t) kM; r += kLoaders / 16u) {
+            // the weight row behind row r of the tile: the matrix's next 128 rows - or, for the gated mean, stream
+            // r / per's row of value d0 + r % per, so the hc sums of one output value lie in one tile (a row past the
+            // matrix, or past the streams, repeats a valid one and is never stored)
+            uint32_t row;
+            if constexpr (EPI == kGatedMean) {
+              const uint32_t d0 = tl.rt * a.per, st = r / a.per, d = d0 + (r - st * a.per);
+              row = (st < a.hc ? st : a.hc - 1) * a.dim + (d < a.dim ? d : a.dim - 1);
+            } else {
+              row = min(tl.rt * kM + r, a.rows - 1u);
+            }
+            const uint8_t* from = w + (uint64_t) row * row_bytes + in_row;
+            const uint8_t* src = (const uint8_t*) ((uintptr_t) from & ~(uintptr_t) 15) + piece * 16u;
+            if (piece < (((uint32_t) (uintptr_t) from & 15u) + bytes + 15u) / 16u)
+              asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + r * kSlot + piece * 16u), "l"(src) : "memory");
+          }
+        }
+        arrive_when_copied(&sh.full_raw[slot]);
+      }
+    }
+    if (!ok) sh.fail = 1;
     asm volatile("cp.async.wait_all;" ::: "memory");
+  } else if (warp == (uint32_t) kTokenWarp) {
+    // ================= the activations' loader =================
+    uint32_t s = 0, slot = 0;
+    bool ok = true;
+    for (uint32_t t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
+      const Tile tl = tile_at(a, first, t, m_at, lane);
+      const uint32_t tok_tiles = whole16(tl.n) / MM_TILE;  // x16 holds whole tiles of 16 tokens
+      const uint32_t sub_bytes = (a.wt ? tok_tiles : slot_tiles) * 512u;
+      const uint32_t xoff = a.wt ? a.xoff[tl.m] : 0u, tile_halves = MM_TILE * a.xts;
+      const uint32_t tile0 = xoff / tile_halves + tl.c0 / MM_TILE;
+      const CUtensorMap* const map = &maps.map[a.wt ? tok_tiles - 1u : 0u];
+      const bool mapped = a.use_tma && tile0 * tile_halves == xoff + (tl.c0 / MM_TILE) * tile_halves;
+      const uint8_t* src0 = (const uint8_t*) (a.x16 + xoff + mm_x16_at(tl.c0, 0, a.xts)) + lane * 16u;
+      const uint32_t dst0 = (lane >> 2) * 64u + (((lane & 3u) ^ ((lane >> 3) & 3u)) * 16u);
+      for (uint32_t it = 0; it < steps; it += 1u << two, s++, src0 += MM_TILE * unit_subs * MM_TILE * 2u) {  // (s: units)
+        if (s >= slots && !bar_wait_soon(&sh.empty[(s - slots) & (units - 1u)], ((s - slots) >> (3u - two)) & 1u)) {
+          ok = false;
+          break;
+        }
+        const uint32_t dst = smem_addr(smem) + slot * slot_bytes;
+        uint64_t* const bar = &sh.full_b[s & (units - 1u)];
+        if (mapped) {
+          // the tiled x16 seen as [K fragment][token tile][two tokens][value]: one box is a step's four sub-tiles, swizzled as
+          // the products read it (tiles past the last are filled with zeros); the barrier counts the bytes
+          if (lane == 0) {
+            bar_expect(bar, sub_bytes * unit_subs);
+            for (uint32_t q = 0; q < unit_subs; q += kSubs)
+              asm volatile(
+                  "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(
+                      dst + q * sub_bytes),
+                  "l"(map), "r"(0), "r"(0), "r"(tile0), "r"(it * kSubs + q), "r"(smem_addr(bar))
+                  : "memory");
+          }
+          __syncwarp();
+        } else {
+          // tokens that start inside a tile of x16: a fragment a round, 512 bytes as they lie - lane = (two tokens, a quarter of
+          // their 64 bytes), the quarter swizzled - waited for here and made visible to the tensor core
+          const uint8_t* src = src0;
+          uint32_t to = dst + dst0;
+          for (uint32_t i = 0; i < tok_tiles; i++, src += tile_halves * 2u, to += 512u) {
+            for (uint32_t q = 0; q < unit_subs; q++)
+              asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + q * sub_bytes), "l"(src + q * 512u) : "memory");
+          }
+          asm volatile("cp.async.wait_all;" ::: "memory");
+          fence_async_smem();
+          __syncwarp();
+          if (lane == 0) bar_arrive(bar);
+        }
+        if (++slot == slots) slot = 0;
+      }
+    }
+    if (!ok) {  // (the copies in flight land before the block's shared memory is another's)
+      sh.fail = 1;
+      for (uint32_t i = s > slots ? s - slots : 0u; i < s; i++) bar_wait_warp(&sh.full_b[i & (units - 1u)], (i >> (3u - two)) & 1u);
+    }
   } else if (warp == (uint32_t) kIssuerWarp) {
     // ================= issuer =================
+    const uint32_t issuer = elect_one();
+    uint32_t s = 0, slot = 0, acc = 0;  // acc: accumulators taken so far
     bool ok = true;
-    uint32_t stage = 0, use = 0;
-    for (uint32_t it = 0; it < steps && !sh.fail; it++, stage++) {
-      if (stage == S) stage = 0, use++;
-      if (!bar_wait(&sh.full_a[stage], use & 1u) || !bar_wait(&sh.full_b[stage], use & 1u)) {
-        sh.fail = 1, ok = false;
-        break;
+    for (uint32_t t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
+      const Tile tl = tile_at(a, first, t, m_at, lane);
+      // a tile of up to 128 tokens has its even tokens' sums in an accumulator's first 64 columns, its odd ones' in the rest; a
+      // larger one an accumulator of each
+      const uint32_t uses = tl.n > (uint32_t) kN ? 2u : 1u, sub16 = (a.wt ? whole16(tl.n) / MM_TILE : slot_tiles) * (512u >> 4);
+      for (uint32_t u = 0; u < uses && ok; u++)
+        if (acc + u >= 2u && !bar_wait_soon(&sh.empty_acc[(acc + u) & 1u], ((acc + u) / 2u - 1u) & 1u)) ok = false;
+      if (!ok) break;
+      const uint32_t d0 = tmem + (acc & 1u) * kN, d1 = uses == 2u ? tmem + ((acc + 1u) & 1u) * kN : d0 + kN / 2;
+      const uint32_t id = idesc(whole16((tl.n + 1u) / 2u));
+      for (uint32_t it = 0; it < steps; it += 1u << two, s++) {  // (s: units)
+        const uint32_t unit = s & (units - 1u), parity = (s >> (3u - two)) & 1u;
+        if (!bar_wait_soon(&sh.full_b[unit], parity) || !bar_wait_soon(&sh.full_a[unit], parity)) {
+          ok = false;
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t at = tmem + kAccCols + unit * (kStageCols << two);
+        const uint64_t b0 = tile_desc_sw64(smem_addr(smem) + slot * slot_bytes);
+        mma_f16_ts_k64(issuer, d0, d1, at, b0, sub16, id, it);
+        if (two) mma_f16_ts_k64(issuer, d0, d1, at + kStageCols, b0 + 4u * sub16, sub16, id, 1u);
+        mma_commit(issuer, &sh.empty[unit]);
+        if (++slot == slots) slot = 0;
       }
-      fence_async_smem();  // the loader's copies (seen through the barrier) before the tensor core's reads
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      if (lane == 0) {
-        const uint32_t sa = smem_addr(smem + stage * a.stage_bytes), sb = sa + kStageA;
-        for (uint32_t acc = 0; acc < n_acc; acc++)
-          for (uint32_t q = 0; q < (uint32_t) kSubs; q++) {
-            const uint64_t da = tile_desc(sa + q * kSubTile);
-            const uint64_t db = a.use_tma ? tile_desc_sw32(sb + (acc * kSubs + q) * kSubTile) : tile_desc(sb + (acc * kSubs + q) * kSubTile);
-            const uint32_t accumulate = (it | q) != 0 ? 1u : 0u;
-            asm volatile(
-                "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(
-                    tmem + acc * kN),
-                "l"(da), "l"(db), "r"(kIdesc), "r"(accumulate)
-                : "memory");
-          }
-        // the stage's operands are free once these have run
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(&sh.empty[stage]))
-                     : "memory");
-      }
-      __syncwarp();
+      if (!ok) break;
+      mma_commit(issuer, &sh.full_acc[acc & 1u]);
+      if (uses == 2u) mma_commit(issuer, &sh.full_acc[(acc + 1u) & 1u]);
+      acc += uses;
     }
-    if (ok && !sh.fail && lane == 0)
-      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(&sh.done)) : "memory");
-    __syncwarp();
-  }
-  // ================= epilogue =================
-  // Every warp, once its own role is done: a warp reads the tensor-memory lanes of its quarter (its index mod 4: the
-  // hardware's rule), so the six or seven warps of a quarter share its rows' 32-token chunks - twenty-five warps
-  // storing instead of four. (The gated mean's exchange through shared memory stays with the first four warps.)
-  if (EPI != kGatedMean || warp < (uint32_t) kEpiWarps) {
-    const uint32_t quarter = warp % 4u, part = EPI == kGatedMean ? 0u : warp / 4u;
-    const uint32_t parts = EPI == kGatedMean ? 1u : ((uint32_t) (kThreads / kWarp) - quarter + 3u) / 4u;  // the quarter's warps
-    const uint32_t row = 32u * quarter + lane;  // this thread's weight row of the tile = its TMEM lane
-    const uint32_t lane_base = tmem + ((32u * quarter) << 16);
-    if (!bar_wait_long(&sh.done, 0)) {
-      // (the K loop's own waits are 0.2 s each and can queue up: look again while nobody has given up)
-      bool landed = false;
-      for (uint32_t tries = 0; tries < 25u && !__any_sync(0xFFFFFFFFu, sh.fail) && !landed; tries++) landed = bar_wait_long(&sh.done, 0);
-      if (!landed) sh.fail = 1;
+    if (!ok) {  // (what has been issued ends before tensor memory is released)
+      sh.fail = 1;
+      mma_commit(issuer, &sh.drain);
+      bar_wait_warp(&sh.drain, 0);
     }
-    // (nobody else writes the word once the last product has landed or been given up: after this barrier every
-    // epilogue thread reads the same value, so all of them or none take the barriers below)
-    if constexpr (EPI == kGatedMean) asm volatile("bar.sync 2, %0;" ::"n"(kEpiWarps * kWarp) : "memory");
-    if (!__any_sync(0xFFFFFFFFu, sh.fail)) {  // (one answer a warp: tensor memory is read by whole warps)
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      for (uint32_t acc = 0; acc < n_acc; acc++) {
+  } else {
+    // ================= epilogue =================
+    const uint32_t row = 32u * warp + lane;  // this thread's weight row of the tile = its TMEM lane
+    uint32_t acc = 0;
+    bool ok = true;
+    for (uint32_t t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
+      const Tile tl = tile_at(a, first, t, m_at, lane);
+      const uint32_t row0 = tl.rt * kM;
+      const bool live = row0 + row < a.rows;
+      const uint32_t uses = tl.n > (uint32_t) kN ? 2u : 1u;
+      for (uint32_t u = 0; u < uses; u++, acc++) {  // the tile's accumulators
+        const uint32_t buf = acc & 1u;
+        ok = false;  // (a K loop's own waits are 0.2 s each and can queue up: look again while nobody has given up)
+        for (uint32_t tries = 0; tries < 25u && !ok; tries++) {
+          ok = bar_wait_long(&sh.full_acc[buf], (acc / 2u) & 1u);
+          if (!ok && __any_sync(0xFFFFFFFFu, *(volatile int*) &sh.fail)) break;
+        }
+        if (!ok) sh.epi_fail = 1;
+        // (the gated mean's warps meet below: all of them or none. Nobody writes the word between this barrier and the next.)
+        if constexpr (EPI == kGatedMean) {
+          asm volatile("bar.sync 2, %0;" ::"n"(kEpiWarps * kWarp) : "memory");
+          ok = *(volatile int*) &sh.epi_fail == 0;
+        }
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        float* const y0 = a.y + (a.wt ? a.yoff[tl.m] : 0u) + (uint64_t) tl.c0 * a.ys + row0 + row;
 #pragma unroll 1
-        for (uint32_t c32 = 0; c32 < (uint32_t) kN; c32 += 32) {
-          if (acc * kN + c32 >= n_valid) break;
-          if ((acc * (uint32_t) (kN / 32) + c32 / 32u) % parts != part) continue;  // (a chunk of another warp of the quarter)
-          uint32_t r[32];
+        for (uint32_t c = 0; c < (uint32_t) kN; c += kChunkTok) {
+          // column c of the accumulator is token 2 c + u, or (both halves in one) token 2 (c % 64) + c / 64
+          const uint32_t t0 = uses == 2u ? 2u * c + u : 2u * (c % (kN / 2)) + c / (kN / 2);
+          if (t0 >= tl.n) continue;
+          uint32_t r[kChunkTok];
           asm volatile(
-              "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-              "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+              "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-                "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-                "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-                "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-              : "r"(lane_base + acc * kN + c32)
+                "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+              : "r"(tmem + ((32u * warp) << 16) + buf * kN + c)
               : "memory");
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
           if constexpr (EPI == kGatedMean) {
-            // each thread gates its row's sums into the idle operand ring ([token of the 32][tile row]); then thread e
-            // adds value e % per's streams in order for the tokens e / per, e / per + 128 / per, ...
-            float* ex = (float*) smem;
-            const uint32_t st = row / a.per, d = d0 + (row - st * a.per);
+            // each thread gates its row's sums into the exchange ([token of the chunk][tile row]); then thread e adds value
+            // e % per's streams in order for the tokens e / per, e / per + 128 / per, ...
+            float* ex = (float*) (smem + kExAt<T, EPI>);
+            const uint32_t d0 = tl.rt * a.per, st = row / a.per, d = d0 + (row - st * a.per);
             const bool mine = st < a.hc && d < a.dim;
 #pragma unroll
-            for (int i = 0; i < 32; i++) {
-              const uint32_t t = acc * kN + c32 + i;
+            for (uint32_t i = 0; i < kChunkTok; i++) {
               float p = 0.0f;
-              if (mine && t < n_valid)
-                p = mul_rn(a.xn[((uint64_t) (c0 + t) * a.hc + st) * a.dim + d], sigmoidf(__uint_as_float(r[i])));
+              if (mine && t0 + 2u * i < tl.n)
+                p = mul_rn(a.xn[((uint64_t) (tl.c0 + t0 + 2u * i) * a.hc + st) * a.dim + d], sigmoidf(__uint_as_float(r[i])));
               ex[i * kM + row] = p;
             }
             asm volatile("bar.sync 2, %0;" ::"n"(kEpiWarps * kWarp) : "memory");
             const uint32_t j = row % a.per, tg = row / a.per, groups = (uint32_t) kM / a.per;
             if (tg < groups && d0 + j < a.dim) {
-              for (uint32_t i = tg; i < 32u; i += groups) {
-                const uint32_t t = acc * kN + c32 + i;
-                if (t >= n_valid) break;
+              for (uint32_t i = tg; i < kChunkTok && t0 + 2u * i < tl.n; i += groups) {
+                const uint32_t tk = tl.c0 + t0 + 2u * i;
                 float sum = 0.0f;
                 for (uint32_t q = 0; q < a.hc; q++) sum = __fadd_rn(sum, ex[i * kM + q * a.per + j]);
                 const float v = __fdiv_rn(sum, (float) a.hc);
-                a.out[(uint64_t) (c0 + t) * a.dim + d0 + j] = v;
-                if (a.x16_out) x16_store(a.x16_out, a.overflow, a.out_row0 + c0 + t, d0 + j, a.dim, v);
+                a.out[(uint64_t) tk * a.dim + d0 + j] = v;
+                if (a.x16_out) x16_store(a.x16_out, a.overflow, a.out_row0 + tk, d0 + j, a.dim, v);
               }
             }
-            asm volatile("bar.sync 2, %0;" ::"n"(kEpiWarps * kWarp) : "memory");  // (the next 32 tokens reuse ex)
-          } else if (row0 + row < a.rows) {
+            asm volatile("bar.sync 2, %0;" ::"n"(kEpiWarps * kWarp) : "memory");  // (the next tokens reuse ex)
+          } else if (live) {
+            float* y = y0 + (uint64_t) t0 * a.ys;
 #pragma unroll
-            for (int i = 0; i < 32; i++) {
-              const uint32_t t = acc * kN + c32 + i;
-              if (t < n_valid) {
-                float v = __uint_as_float(r[i]);
-                if (a.scale != 1.0f) v = mul_rn(v, a.scale);
+            for (uint32_t i = 0; i < kChunkTok; i++) {
+              if (t0 + 2u * i < tl.n) {
+                float v = mul_rn(__uint_as_float(r[i]), a.scale);
                 if constexpr (EPI == kSilu) {
                   v = siluf(v);
-                  x16_store(a.x16_out, a.overflow, c0 + t, row0 + row, a.rows, v);
+                  x16_store(a.x16_out, a.overflow, tl.c0 + t0 + 2u * i, row0 + row, a.rows, v);
                 }
-                y[(uint64_t) (c0 + t) * a.ys + row0 + row] = v;
+                *y = v;
               }
+              y += 2u * (uint64_t) a.ys;
             }
           }
         }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) bar_arrive(&sh.empty_acc[buf]);
       }
     }
+    if (!ok) sh.fail = 1;
   }
   // ================= common exit =================
+  __syncwarp();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == (uint32_t) kIssuerWarp) {
@@ -661,49 +821,63 @@ EncodeTiled encoder() {
   return fn;
 }
 
-// the tiled x16 of n tokens (rows xts values long) as [token tile][K fragment][token in tile][value in fragment]
-bool x16_map(const void* x16, uint32_t n, uint32_t xts, CUtensorMap* tm) {
+// the tiled x16 of `tiles` token tiles (rows xts values long) as [K fragment][token tile][two tokens][value in
+// fragment]; a box: a K step's fragments of `tok` tokens
+bool x16_map(const void* x16, uint32_t tiles, uint32_t xts, uint32_t tok, CUtensorMap* tm) {
   const EncodeTiled enc = encoder();
   if (!enc) return false;
-  const cuuint64_t dims[4] = {MM_TILE, MM_TILE, xts / MM_TILE, (n + MM_TILE - 1) / MM_TILE};
-  const cuuint64_t strides[3] = {MM_TILE * 2, MM_TILE * MM_TILE * 2, (cuuint64_t) MM_TILE * xts * 2};
-  const cuuint32_t box[4] = {MM_TILE, MM_TILE, 1, kN / MM_TILE}, unit[4] = {1, 1, 1, 1};
+  const cuuint64_t dims[4] = {2 * MM_TILE, MM_TILE / 2, tiles, xts / MM_TILE};
+  const cuuint64_t strides[3] = {MM_TILE * 4, (cuuint64_t) MM_TILE * xts * 2, MM_TILE * MM_TILE * 2};
+  const cuuint32_t box[4] = {2 * MM_TILE, MM_TILE / 2, tok / MM_TILE, kSubs}, unit[4] = {1, 1, 1, 1};
   return enc(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<void*>(x16), dims, strides, box, unit, CU_TENSOR_MAP_INTERLEAVE_NONE,
-             CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+             CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 template <uint32_t T, uint32_t EPI = kStore>
 bool launch(Args a, uint32_t n_mat, uint32_t max_cnt, cudaStream_t s) {
-  alignas(64) CUtensorMap tmap;
-  memset(&tmap, 0, sizeof tmap);
-  a.use_tma = 0;
-  if (!a.wt && x16_map(a.x16, a.n, a.xts, &tmap)) a.use_tma = 1;
+  constexpr int kBytes = (int) kSmem<T, EPI>;
+  static_assert(kBytes + grid_smem_bytes<T>() + (int) sizeof(Shared) + 64 <= 227 * 1024, "a block's shared memory");
   a.status = status_word();
   if (!a.status) return false;
   int sms = 0, dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     return false;
-  constexpr uint32_t kSlot = kRawSlot<T>, kLimit = 224u * 1024u - (uint32_t) ((grid_smem_bytes<T>() + 1023) / 1024 * 1024);
-  const uint32_t row_tiles = EPI == kGatedMean ? (a.dim + a.per - 1) / a.per : (a.rows + kM - 1) / kM;
-  auto stages_for = [&](uint32_t k) { return k >= 4 ? 2u : k == 2 ? 3u : 4u; };  // a deeper ring where a stage is small
-  auto smem_for = [&](uint32_t k) { return stages_for(k) * (kStageA + k * kSubs * kSubTile) + 2u * kM * kSlot; };
-  // tokens a block: the accumulator count (1, 2 or 4 of 128 tokens; a weight is decoded once a block) with the least
-  // estimated time - waves of blocks over the SMs times a block's time, which measured ~0.85 + 0.45 k a step with the
-  // activations copied 16 bytes at a time and ~0.95 + 0.12 k with tensor-map copies
-  a.accs = 1;
-  float best = 0.0f;
-  for (uint32_t k = 1; k <= (uint32_t) kMaxAcc; k <<= 1) {
-    if (smem_for(k) > kLimit) break;
-    const uint64_t blocks = (uint64_t) row_tiles * n_mat * ((max_cnt + k * kN - 1) / (k * kN));
-    const float cost = (float) ((blocks + sms - 1) / sms) * (a.use_tma ? 0.95f + 0.12f * (float) k : 0.85f + 0.45f * (float) k);
-    if (k == 1 || cost < best) best = cost, a.accs = k;
-  }
-  a.stages = stages_for(a.accs), a.stage_bytes = kStageA + a.accs * kSubs * kSubTile, a.raw_off = a.stages * a.stage_bytes;
-  const int smem_bytes = (int) smem_for(a.accs);
+  a.row_tiles = EPI == kGatedMean ? parts_of(a.dim, a.per) : parts_of(a.rows, kM);
   static bool sized[64] = {};  // (one record a template instance, one flag a device)
-  if (!allow_dynamic_smem(mm_tc_kernel<T, EPI>, (int) kLimit, sized)) return false;
-  const dim3 grid(row_tiles, n_mat, (max_cnt + a.accs * kN - 1) / (a.accs * kN));
-  mm_tc_kernel<T, EPI><<<grid, kThreads, smem_bytes, s>>>(a, tmap);
+  if (!allow_dynamic_smem(mm_tc_kernel<T, EPI>, kBytes, sized)) return false;
+  alignas(64) Maps maps;
+  memset(&maps, 0, sizeof maps);
+  if (a.wt) {
+    a.span = max_cnt < kMaxSpan ? whole16(max_cnt) : kMaxSpan;
+    // (where in x16 a matrix's tokens lie is on the device: the maps reach as far as its 32-bit offsets do, and a box has no
+    // tile but the tokens')
+    a.use_tma = 1;
+    for (uint32_t t = 0; t < a.span / MM_TILE && a.use_tma; t++)
+      if (!x16_map(a.x16, (uint32_t) (0xFFFFFFFFull / (MM_TILE * (uint64_t) a.xts)) + 1u + MM_MAX_TOKENS / MM_TILE, a.xts, (t + 1u) * MM_TILE, &maps.map[t])) a.use_tma = 0;
+    for (uint32_t m0 = 0; m0 < n_mat; m0 += kMaxMats) {
+      Args c = a;
+      c.n_mat = n_mat - m0 < kMaxMats ? n_mat - m0 : kMaxMats;
+      c.wt += m0, c.cnt += m0, c.xoff += m0, c.yoff += m0;
+      const uint64_t tiles = (uint64_t) a.row_tiles * c.n_mat * parts_of(max_cnt, a.span);
+      mm_tc_kernel<T, EPI><<<(unsigned) (tiles < (uint64_t) sms ? tiles : (uint64_t) sms), kThreads, kBytes, s>>>(c, maps);
+      if (!launched()) return false;
+    }
+    return true;
+  }
+  // tokens a tile: the split with the least estimated time - rounds of tiles over the SMs times a K step's cycles, which are
+  // the decoders' or the products' (2 a token, and reading their operands), whichever is more
+  uint64_t best = 0;
+  constexpr uint32_t kMost = EPI == kGatedMean ? 192u : kMaxSpan;  // (two slots of the token ring)
+  for (uint32_t cols = parts_of(a.n, kMost); cols <= parts_of(a.n, MM_TILE); cols++) {
+    const uint32_t tok = whole16(parts_of(a.n, cols)), step = 60u + 9u * tok / 4u;
+    const uint64_t rounds = ((uint64_t) a.row_tiles * parts_of(a.n, tok) + (uint32_t) sms - 1u) / (uint32_t) sms;
+    const uint64_t cost = rounds * (step > 320u ? step : 320u);
+    if (!best || cost < best) best = cost, a.span = tok;
+  }
+  a.use_tma = x16_map(a.x16, parts_of(a.n, MM_TILE), a.xts, a.span, &maps.map[0]) ? 1u : 0u, a.n_mat = 1;
+  const uint64_t tiles = (uint64_t) a.row_tiles * parts_of(a.n, a.span);
+  if (tiles > 0xFFFFFFFFull) return false;
+  mm_tc_kernel<T, EPI><<<(unsigned) (tiles < (uint64_t) sms ? tiles : (uint64_t) sms), kThreads, kBytes, s>>>(a, maps);
   return launched();
 }
 
