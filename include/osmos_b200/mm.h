@@ -122,6 +122,11 @@ bool mm_tokens_scaled(uint32_t type, const void *w0, uint32_t rows0, float *y0, 
 bool mm_group(uint32_t type, const void *const *w, const int32_t *cnt, uint32_t n_mat, uint32_t max_cnt, uint32_t rows,
               uint32_t cols, const void *x16, const uint32_t *xoff, uint32_t xts, float *y, const uint32_t *yoff,
               uint32_t ys, void *stream);
+/* Not in the reference: mm_group where every w[m] is one of the n_base matrices of one tensor, `bytes` apart from `base` on (an
+   expert tensor): known to the host, its rows can be read through a tensor map. base NULL: mm_group. */
+bool mm_group_of(uint32_t type, const void *base, uint64_t bytes, uint32_t n_base, const void *const *w, const int32_t *cnt,
+                 uint32_t n_mat, uint32_t max_cnt, uint32_t rows, uint32_t cols, const void *x16, const uint32_t *xoff,
+                 uint32_t xts, float *y, const uint32_t *yoff, uint32_t ys, void *stream);
 /* NVFP4 weights times NVFP4 activations, W4A4 (reference: include/osmos/gpu/mm.h:45-61, kernels/mm_fp4.hip).
    mm_fp4_ok: whether this device runs the path (the reference's answers true on sm_120a only; this one on sm_100a).
    mm_fp4_quant: x's n rows (F32, or (bf16) BF16 as 16-bit words; stride xs elements) quantized under the input scale gs

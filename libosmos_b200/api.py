@@ -149,6 +149,7 @@ SIGNATURES = {
     "mm_tokens": (B, [U32, P, U32, P, U32, P, U32, P, U32, U32, P, U32, U32, P, P, C.c_bool, P]),
     "mm_tokens_scaled": (B, [U32, P, U32, P, U32, C.c_float, P, U32, P, U32, C.c_float, U32, P, U32, U32, P, P, C.c_bool, P]),
     "mm_group": (B, [U32, P, P, U32, U32, U32, U32, P, P, U32, P, P, U32, P]),
+    "mm_group_of": (B, [U32, P, U64, U32, P, P, U32, U32, U32, U32, P, P, U32, P, P, U32, P]),
     "mm_status": (U32, []),
     "mm_fp4_ok": (B, []),
     "mm_fp4_act": (B, [P, U32, U32, U32, C.c_float, P, P, P]),

@@ -90,6 +90,10 @@ __device__ __forceinline__ void arrive_when_copied(uint64_t* bar) {
 template <uint32_t T> constexpr uint32_t kRawK = (T == QTYPE_Q8_0 || T == QTYPE_MXFP8) ? 128u : 256u;
 template <uint32_t T> constexpr uint32_t kRawBytes = kRawK<T> / Fmt<T>::values * Fmt<T>::bytes;
 template <uint32_t T> constexpr uint32_t kRawSlot = ((kRawBytes<T> + 30u + 15u) & ~15u) | 16u;
+// a matrix whose rows all start on 16 bytes comes by tensor-map copies: a window of each row that starts on 16 bytes and holds the
+// block's, again of an odd number of pieces
+template <uint32_t T> constexpr uint32_t kLead = kRawBytes<T> % 16u == 0 ? 0u : kRawBytes<T> % 8u == 0 ? 8u : kRawBytes<T> % 4u == 0 ? 12u : 14u;
+template <uint32_t T> constexpr uint32_t kWindow = ((kRawBytes<T> + kLead<T> + 15u) & ~15u) | 16u;
 template <uint32_t T> constexpr uint32_t kRawPieces = (kRawBytes<T> + 30u) / 16u;  // of a row that starts anywhere in its first piece
 template <uint32_t T> constexpr uint32_t kRawStages = (92u * 1024u) / (kM * kRawSlot<T>) < 4u ? (92u * 1024u) / (kM * kRawSlot<T>) : 4u;
 // shared memory: the tokens' ring (1024-byte aligned), the raw ring, the gated mean's exchange, the matrices' first tiles
@@ -370,7 +374,11 @@ struct Args {
   uint32_t rows, cols, n, xts, ys;
   uint32_t n_mat, row_tiles;
   uint32_t span;     // the most tokens a tile takes
-  uint32_t use_tma;  // the activations come by tensor-map copies (mm_run), else by 16-byte cp.async (mm_group)
+  uint32_t use_tma;  // the activations come by tensor-map copies, else by 16-byte cp.async
+  uint32_t raw_map;  // the weights too (Maps::raw); grouped: the matrices are those of one tensor, `bytes` apart from `base` on
+  const uint8_t* base;
+  uint64_t bytes;
+  uint32_t n_base;
   float scale;
   uint32_t* status;
   // the epilogue (the kernel's EPI): kStore y = scale sum; kSilu y = silu(scale sum), and its f16 into x16_out (rows wide, tiled);
@@ -384,6 +392,7 @@ struct Args {
 };
 struct Maps {  // the tokens' maps: of a grouped launch map t a box of t + 1 token tiles, else the one map's box is a.span tokens
   CUtensorMap map[kMaxSpan / MM_TILE];
+  CUtensorMap raw;  // the weights' bytes as [matrix][row][byte]
 };
 enum : uint32_t { kStore = 0, kSilu = 1, kGatedMean = 2 };
 
@@ -435,11 +444,13 @@ __global__ void __launch_bounds__(kThreads, 1) mm_tc_kernel(const Args a, const 
   const uint32_t kblocks = parts_of(steps, kStepsRaw);
   uint32_t* const first = (uint32_t*) (smem + kFirstAt<T, EPI>);
   uint8_t* const raw = smem + kRawAt<T, EPI>;
+  const uint32_t pitch = a.raw_map ? kWindow<T> : kSlot;  // a row's bytes in the raw ring
+  static_assert(kWindow<T> <= kSlot, "either fits");
 
   if (tid == 0) {
     for (uint32_t i = 0; i < kSteps; i++) bar_init(&sh.full_b[i], 1), bar_init(&sh.empty[i], 1);
     for (int i = 0; i < 4; i++)
-      bar_init(&sh.full_raw[i], kRawWarps * kWarp), bar_init(&sh.empty_raw[i], (kProdWarps / kTeams) * kStepsRaw);
+      bar_init(&sh.full_raw[i], a.raw_map ? 1 : kRawWarps * kWarp), bar_init(&sh.empty_raw[i], (kProdWarps / kTeams) * kStepsRaw);
     for (int i = 0; i < 2; i++) bar_init(&sh.full_acc[i], 1), bar_init(&sh.empty_acc[i], kEpiWarps);
     bar_init(&sh.drain, 1);
     sh.fail = 0, sh.epi_fail = 0;
@@ -514,7 +525,7 @@ __global__ void __launch_bounds__(kThreads, 1) mm_tc_kernel(const Args a, const 
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t off = slot * (kM * kSlot) + r * kSlot + ((base15 + kb * kRawBytes<T>) & 15u);
+        const uint32_t off = slot * (kM * kSlot) + r * pitch + ((base15 + kb * kRawBytes<T>) & 15u);
         const uint32_t col = lane_cols + stage * kStageCols;
         decode_step<T>(smem_addr(raw) + off, raw + off, sub, g, [&](uint32_t q, const uint32_t (&v)[8]) {
           asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(col + 8u * q), "r"(v[0]), "r"(v[1]),
@@ -535,15 +546,13 @@ __global__ void __launch_bounds__(kThreads, 1) mm_tc_kernel(const Args a, const 
   } else if (warp >= (uint32_t) kFirstRaw && warp < (uint32_t) kTokenWarp) {
     // ================= the weights' loaders =================
     // The 16-byte pieces of the aligned span around each row's bytes (a block may start anywhere in a piece; every piece
-    // asked for holds some of them). Where all rows start at the same place in a piece, 64 threads take the pieces of
-    // kTogether rows in kRounds rounds whose places do not change from block to block: three instructions a copy. (A
-    // loader that worked a row's address out a copy held a K step to 1,000 cycles.)
+    // asked for holds some of them): 64 threads take the pieces of kTogether rows in kRounds rounds whose places do not change
+    // from block to block. (A loader that worked a row's address out for each copy held a K step to 1,000 cycles.)
     constexpr uint32_t kP = kRawPieces<T>, kLoaders = kRawWarps * kWarp;
     constexpr uint32_t kTogether = kP % 64u == 0 ? 1u : kP % 32u == 0 ? 2u : kP % 16u == 0 ? 4u : kP % 8u == 0 ? 8u : kP % 4u == 0 ? 16u : kP % 2u == 0 ? 32u : 64u;
     constexpr uint32_t kRounds = kTogether * kP / kLoaders;
     static_assert(kP <= 16u && kP * 16u <= kSlot && kRounds * kLoaders == kTogether * kP && kM % kTogether == 0, "the rows' pieces");
     const uint32_t lt = (warp - kFirstRaw) * kWarp + lane;
-    const bool alike = EPI != kGatedMean && row_bytes % 16u == 0 && row_bytes < (1u << 24);
     uint32_t src_at[kRounds], dst_at[kRounds];
 #pragma unroll
     for (uint32_t j = 0; j < kRounds; j++) {
@@ -552,7 +561,31 @@ __global__ void __launch_bounds__(kThreads, 1) mm_tc_kernel(const Args a, const 
     }
     uint32_t rb = 0;
     bool ok = true;
-    for (uint32_t t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
+    if (a.raw_map) {  // a copy a block: the second warp has nothing to do
+      for (uint32_t t = blockIdx.x; t < tiles && ok && warp == (uint32_t) kFirstRaw; t += gridDim.x) {
+        const Tile tl = tile_at(a, first, t, m_at, lane);
+        const uint32_t mat = a.wt ? (uint32_t) ((uint64_t) (a.wt[tl.m] - a.base) / a.bytes) : 0u;
+        for (uint32_t kb = 0; kb < kblocks; kb++, rb++) {
+          const uint32_t slot = rb % kRawStages<T>;
+          if (rb >= kRawStages<T> && !bar_wait_soon(&sh.empty_raw[slot], (rb / kRawStages<T> - 1u) & 1u)) {
+            ok = false;
+            break;
+          }
+          if (lane == 0) {  // (rows past the matrix, and bytes past a row's, are filled with zeros)
+            bar_expect(&sh.full_raw[slot], kM * kWindow<T>);
+            asm volatile(
+                "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
+                    smem_addr(raw) + slot * (kM * kSlot)),
+                "l"(&maps.raw), "r"((kb * kRawBytes<T>) & ~15u), "r"(tl.rt * kM), "r"(mat), "r"(smem_addr(&sh.full_raw[slot]))
+                : "memory");
+          }
+          __syncwarp();
+        }
+      }
+      if (!ok)  // (the copies in flight land before the block's shared memory is another's)
+        for (uint32_t i = rb > kRawStages<T> ? rb - kRawStages<T> : 0u; i < rb; i++) bar_wait_warp(&sh.full_raw[i % kRawStages<T>], (i / kRawStages<T>) & 1u);
+    }
+    for (uint32_t t = blockIdx.x; t < tiles && ok && !a.raw_map; t += gridDim.x) {
       const Tile tl = tile_at(a, first, t, m_at, lane);
       const uint8_t* w = a.wt ? a.wt[tl.m] : a.w;
       for (uint32_t kb = 0; kb < kblocks; kb++, rb++) {
@@ -564,36 +597,35 @@ __global__ void __launch_bounds__(kThreads, 1) mm_tc_kernel(const Args a, const 
         const uint32_t dst = smem_addr(raw) + slot * (kM * kSlot);
         const uint64_t in_row = (uint64_t) kb * kRawBytes<T>;
         const uint32_t bytes = row_bytes - in_row < kRawBytes<T> ? (uint32_t) (row_bytes - in_row) : kRawBytes<T>;
-        if (alike) {  // (rows past the matrix are left out: whatever their lanes hold is never stored)
-          const uint32_t row0 = tl.rt * kM, live = min(a.rows - row0, (uint32_t) kM);
+        const uint32_t row0 = tl.rt * kM;
+        auto copy = [&](uint32_t to, const uint8_t* from) {  // the piece `to` of a slot whose bytes start where `from` lies in its piece
+          const uint32_t lead = (uint32_t) (uintptr_t) from & 15u;
+          if (to % kSlot < lead + bytes)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + to), "l"(from - lead) : "memory");
+        };
+        if (EPI != kGatedMean && a.rows - row0 >= (uint32_t) kM && row_bytes < (1u << 24)) {
           const uint8_t* from = w + (uint64_t) row0 * row_bytes + in_row;
-          const uint32_t need = (((uint32_t) (uintptr_t) from & 15u) + bytes + 15u) / 16u * 16u;
-          const uint8_t* src = (const uint8_t*) ((uintptr_t) from & ~(uintptr_t) 15);
-          for (uint32_t r0 = 0; r0 < live; r0 += kTogether, src += kTogether * row_bytes) {
+          for (uint32_t r0 = 0; r0 < (uint32_t) kM; r0 += kTogether, from += kTogether * row_bytes) {
+#pragma unroll
+            for (uint32_t j = 0; j < kRounds; j++) copy(r0 * kSlot + dst_at[j], from + src_at[j]);
+          }
+        } else {
+          for (uint32_t r0 = 0; r0 < (uint32_t) kM; r0 += kTogether) {
 #pragma unroll
             for (uint32_t j = 0; j < kRounds; j++) {
-              const uint32_t to = dst_at[j];
-              if (to % kSlot < need && r0 + to / kSlot < live)
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + r0 * kSlot + to), "l"(src + src_at[j]) : "memory");
+              // the weight row behind row r of the tile: the matrix's next 128 rows - or, for the gated mean, stream
+              // r / per's row of value d0 + r % per, so the hc sums of one output value lie in one tile (a row past the
+              // matrix, or past the streams, repeats a valid one and is never stored)
+              const uint32_t to = r0 * kSlot + dst_at[j], r = to / kSlot;
+              uint32_t row;
+              if constexpr (EPI == kGatedMean) {
+                const uint32_t d0 = tl.rt * a.per, st = r / a.per, d = d0 + (r - st * a.per);
+                row = (st < a.hc ? st : a.hc - 1) * a.dim + (d < a.dim ? d : a.dim - 1);
+              } else {
+                row = min(row0 + r, a.rows - 1u);
+              }
+              copy(to, w + (uint64_t) row * row_bytes + in_row + to % kSlot);
             }
-          }
-        } else {  // a half-warp a row, four rows a round
-          const uint32_t piece = lt % 16u;
-          for (uint32_t r = lt / 16u; r < (uint32_t) kM; r += kLoaders / 16u) {
-            // the weight row behind row r of the tile: the matrix's next 128 rows - or, for the gated mean, stream
-            // r / per's row of value d0 + r % per, so the hc sums of one output value lie in one tile (a row past the
-            // matrix, or past the streams, repeats a valid one and is never stored)
-            uint32_t row;
-            if constexpr (EPI == kGatedMean) {
-              const uint32_t d0 = tl.rt * a.per, st = r / a.per, d = d0 + (r - st * a.per);
-              row = (st < a.hc ? st : a.hc - 1) * a.dim + (d < a.dim ? d : a.dim - 1);
-            } else {
-              row = min(tl.rt * kM + r, a.rows - 1u);
-            }
-            const uint8_t* from = w + (uint64_t) row * row_bytes + in_row;
-            const uint8_t* src = (const uint8_t*) ((uintptr_t) from & ~(uintptr_t) 15) + piece * 16u;
-            if (piece < (((uint32_t) (uintptr_t) from & 15u) + bytes + 15u) / 16u)
-              asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + r * kSlot + piece * 16u), "l"(src) : "memory");
           }
         }
         arrive_when_copied(&sh.full_raw[slot]);
@@ -833,6 +865,16 @@ bool x16_map(const void* x16, uint32_t tiles, uint32_t xts, uint32_t tok, CUtens
              CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// n_mat matrices of rows x row_bytes, `bytes` apart: a box is the block of a row tile's rows
+bool raw_map(const void* w, uint64_t row_bytes, uint32_t rows, uint32_t n_mat, uint64_t bytes, uint32_t window, CUtensorMap* tm) {
+  const EncodeTiled enc = encoder();
+  if (!enc || ((uintptr_t) w | row_bytes | bytes) % 16 || row_bytes >> 32 || bytes >> 40 || row_bytes < window) return false;
+  const cuuint64_t dims[3] = {row_bytes, rows, n_mat}, strides[2] = {row_bytes, bytes};
+  const cuuint32_t box[3] = {window, kM, 1}, unit[3] = {1, 1, 1};
+  return enc(tm, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(w), dims, strides, box, unit, CU_TENSOR_MAP_INTERLEAVE_NONE,
+             CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 template <uint32_t T, uint32_t EPI = kStore>
 bool launch(Args a, uint32_t n_mat, uint32_t max_cnt, cudaStream_t s) {
   constexpr int kBytes = (int) kSmem<T, EPI>;
@@ -847,6 +889,10 @@ bool launch(Args a, uint32_t n_mat, uint32_t max_cnt, cudaStream_t s) {
   if (!allow_dynamic_smem(mm_tc_kernel<T, EPI>, kBytes, sized)) return false;
   alignas(64) Maps maps;
   memset(&maps, 0, sizeof maps);
+  const uint64_t row_bytes = (uint64_t) (a.cols / Fmt<T>::values) * Fmt<T>::bytes;
+  if (EPI != kGatedMean && (!a.wt || (a.base && a.bytes >= a.rows * row_bytes)))
+    a.raw_map = a.wt ? raw_map(a.base, row_bytes, a.rows, a.n_base, a.bytes, kWindow<T>, &maps.raw)
+                     : raw_map(a.w, row_bytes, a.rows, 1, a.rows * row_bytes, kWindow<T>, &maps.raw);
   if (a.wt) {
     a.span = max_cnt < kMaxSpan ? whole16(max_cnt) : kMaxSpan;
     // (where in x16 a matrix's tokens lie is on the device: the maps reach as far as its 32-bit offsets do, and a box has no
@@ -1000,16 +1046,23 @@ extern "C" bool mm_tokens(uint32_t type, const void* w0, uint32_t rows0, float* 
   return mm_tokens_scaled(type, w0, rows0, y0, ys0, 1.0f, w1, rows1, y1, ys1, 1.0f, cols, x, xs, n, x16, overflow, ready, stream);
 }
 
-extern "C" bool mm_group(uint32_t type, const void* const* w, const int32_t* cnt, uint32_t n_mat, uint32_t max_cnt,
-                         uint32_t rows, uint32_t cols, const void* x16, const uint32_t* xoff, uint32_t xts, float* y,
-                         const uint32_t* yoff, uint32_t ys, void* stream) {
+extern "C" bool mm_group_of(uint32_t type, const void* base, uint64_t bytes, uint32_t n_base, const void* const* w, const int32_t* cnt, uint32_t n_mat,
+                            uint32_t max_cnt, uint32_t rows, uint32_t cols, const void* x16, const uint32_t* xoff, uint32_t xts, float* y,
+                            const uint32_t* yoff, uint32_t ys, void* stream) {
   if (!w || !cnt || !x16 || !xoff || !y || !yoff || !n_mat || n_mat > 65535 || !max_cnt || max_cnt > MM_MAX_TOKENS ||
       !mm_tc::shape_ok(type, rows, cols) || xts < cols || xts % MM_TILE || ys < rows || ((uintptr_t) x16 & 15u))
     return false;
   mm_tc::Args a{};
   a.wt = (const uint8_t* const*) w, a.cnt = cnt, a.xoff = xoff, a.yoff = yoff, a.x16 = (const __half*) x16, a.y = y;
   a.rows = rows, a.cols = cols, a.xts = xts, a.ys = ys, a.scale = 1.0f;
+  a.base = (const uint8_t*) base, a.bytes = bytes, a.n_base = n_base;
 #define CASE(T) return mm_tc::launch<T>(a, n_mat, max_cnt, stream_of(stream));
   OSMOS_SWITCH_QUANT(type, CASE, return false)
 #undef CASE
+}
+
+extern "C" bool mm_group(uint32_t type, const void* const* w, const int32_t* cnt, uint32_t n_mat, uint32_t max_cnt,
+                         uint32_t rows, uint32_t cols, const void* x16, const uint32_t* xoff, uint32_t xts, float* y,
+                         const uint32_t* yoff, uint32_t ys, void* stream) {
+  return mm_group_of(type, nullptr, 0, 0, w, cnt, n_mat, max_cnt, rows, cols, x16, xoff, xts, y, yoff, ys, stream);
 }

@@ -220,14 +220,14 @@ bool q4x_moe_scratch_bind(const Q4xMoeLayer *l, uint32_t max_tok, void *mem, uin
 
 /* one expert tensor over all the tables' entries in one launch: every run of tile counts holds at most 128 tokens an entry,
    one block's, so a launch a run (hip_layers.c:317-329) would give the same blocks with a thin last wave a run */
-static bool experts(uint32_t type, const void *const *ptr, const Q4xMoeScratch *s, const Q4xExpertBounds *bd, uint32_t rows,
+static bool experts(const Q4xMoeLayer *l, int j, const void *const *ptr, const Q4xMoeScratch *s, const Q4xExpertBounds *bd, uint32_t rows,
                     uint32_t cols, const uint32_t *xo, float *y, const uint32_t *yo, void *stream)
 {
   bool ok = true;
   for (uint32_t at = 0; ok && at < bd->entries; at += MV_MAX_GROUP)
   {
     const uint32_t left = bd->entries - at, n = left < MV_MAX_GROUP ? left : MV_MAX_GROUP;
-    ok = mm_group(type, ptr + at, s->cnt + at, n, (uint32_t)MM_TILE << (Q4X_TILE_RUNS - 1), rows, cols, s->xe16, xo + at, cols, y,
+    ok = mm_group_of(l->type[j], l->tab[j] ? NULL : l->base[j], l->bytes[j], l->n_exp, ptr + at, s->cnt + at, n, (uint32_t)MM_TILE << (Q4X_TILE_RUNS - 1), rows, cols, s->xe16, xo + at, cols, y,
                   yo + at, rows, stream);
   }
   return ok;
@@ -255,9 +255,9 @@ bool q4x_moe(const Q4xMoeLayer *l, const Q4xMoeScratch *s, const float *x, const
   return q4x_route(logits, n, l->n_exp, l->k, s->ids, s->w, s->rows, stream) &&
          q4x_expert_tiles(s->ids, picks, l->k, l->n_exp, D, FF, &et, stream) &&
          mm_x16_rows(x, D, s->gidx, bd.slots, D, s->xe16, s->overflow, stream) &&
-         experts(l->type[0], et.ptr[0], s, &bd, FF, D, s->xg, s->ga, s->yg, stream) &&
-         experts(l->type[1], et.ptr[1], s, &bd, FF, D, s->xg, s->up, s->yg, stream) &&
+         experts(l, 0, et.ptr[0], s, &bd, FF, D, s->xg, s->ga, s->yg, stream) &&
+         experts(l, 1, et.ptr[1], s, &bd, FF, D, s->xg, s->up, s->yg, stream) &&
          q4x_swiglu_rows(s->ga, s->up, FF, s->hidx, bd.slots, s->xe16, s->overflow, stream) &&
-         experts(l->type[2], et.ptr[2], s, &bd, D, FF, s->xd, s->y, s->yd, stream) &&
+         experts(l, 2, et.ptr[2], s, &bd, D, FF, s->xd, s->y, s->yd, stream) &&
          q4x_moe_sum(s->y, s->where, s->w, n, l->k, D, shared, shared_logit, out, stream);
 }
