@@ -5,22 +5,27 @@
 //   MXFP4 (kind::mxf4, a UE8M0 scale every 32 values): ggml type 39 weights against ops_fp4_round's packed activations.
 // E2M1 x E2M1 products are exact and so is a product of two scale factors; the sums are the tensor core's, in F32.
 //
-// A block computes 128 weight rows x up to 256 tokens; K in steps of 256 values through a ring of four stages.
-//   producers (8 warps)  the rows' blocks as the GGUF holds them -> the tensor core's operand layout: the nibbles
+// A block computes 128 weight rows x up to 256 tokens; K in steps of 256 values through a ring of three stages.
+//   producers (16 warps, two teams on alternate stages)
+//                        the rows' blocks as the GGUF holds them -> the tensor core's operand layout: the nibbles
 //                        reordered from ggml's "low nibbles first, then high" to K order (two values a byte, the lower K
-//                        in the low nibble) into K-major core matrices of 8 rows x 16 bytes, and the block scales into
+//                        in the low nibble) under the 128-byte swizzle, and the block scales into
 //                        the scale-factor chunk layout (128 rows x 4 factors: byte (r % 32) * 16 + (r / 32) * 4 + f).
 //                        The raw bytes reach shared memory by the loader's tensor-map copies (a ring of its own, three
-//                        stages ahead), so a producer only ever waits on shared memory. The tokens' scale bytes go to
-//                        the chunk layout by 4-byte cp.async that nobody waits for (the stage's barrier counts them).
+//                        stages ahead), so a producer only ever waits on shared memory. The tokens' scale bytes they
+//                        read a team's stage ahead and store to the chunk layout.
 //   loaders (2 warps)    one the rows' raw bytes (a box of 128 rows x 144 bytes a stage), one the tokens' codes, already in
 //                        K order: one tensor-map copy a stage, a box of 256 tokens x 128 bytes written with the 128-byte
 //                        swizzle, which the MMA's B descriptor names (an MMA's 32 bytes of K 32 bytes along the row).
 //   issuer (1 warp)      per 64 values of K: tcgen05.cp of the scale-factor chunks into tensor memory (32 lanes x 16
 //                        bytes, broadcast to the four lane quarters), then one tcgen05.mma M128 N(16 .. 256) K64 with
 //                        the chunks' addresses; tcgen05.commit onto the stage's "empty" barrier after a stage's four,
-//                        onto the accumulator's barrier after the last.
-//   epilogue (4 warps)   thread = one weight row (its TMEM lane): tcgen05.ld the sums, times the tensors' scale, stored.
+//                        onto the accumulator's barrier after the last. The whole warp runs this, one elected lane issues.
+//   epilogue (all warps, their roles done) thread = one weight row (its TMEM lane): tcgen05.ld the sums, times the tensors'
+//                        scale, stored.
+// 17408 x 5120, 2048 tokens, with the tokens' quantization: 183 -> 164 us with the teams, the elected issuer, the shorter
+// repacking and the shared epilogue. What is left: a stage brings 54 KB to the SM in about 1,100 cycles (over 11 TB/s in all),
+// the tensor pipe needs 700 of them; 3,000 cycles of a tile's 34,000 are its start, 4,300 its stores.
 // The descriptors follow the layouts CUTLASS documents in cute/arch/mma_sm100_desc.hpp (InstrDescriptorBlockScaled),
 // cute/atom/mma_traits_sm100.hpp (the scale factors' tensor-memory fragment) and cutlass/detail/sm100_blockscaled_layout.hpp
 // (the chunk layout); tests/test_fp4_desc.py holds the instruction descriptor to CUTLASS's own encoder.
@@ -41,26 +46,13 @@ namespace fp4_tc {
 namespace {
 
 constexpr int kM = 128, kNMax = 256;
-constexpr int kEpiWarps = 4, kProdWarps = 8;
-// Who does what goes by the warp scheduler a warp lives on (its index mod 4). Scheduler 0 has the issuer and the two
-// loaders, which issue little and wait much, and an epilogue warp that sleeps until the end - so the issuer, whose
-// chain of tcgen05 instructions a stage is the kernel's critical path (35 cycles a scale-factor copy, 75 an MMA, measured
-// by leaving them out), never waits for an issue slot behind a producer. The eight producers share schedulers 1, 2 and 3
-// with the other three epilogue warps. (A second issuing warp for the scale factors' copies, a stage ahead with two sets
-// of tensor-memory columns, was slower: what the hand-over costs exceeds what the copies' issue saved.)
-constexpr int kIssuerWarp = 4;   // scheduler 0
-constexpr int kRawWarp = 8;      // scheduler 0: the rows' raw bytes by tensor-map copies
-constexpr int kLoaderWarp = 12;  // scheduler 0: the tokens' codes by tensor-map copies
-// producer p's warp: 5, 6, 7, 9, 10, 11, 13, 14
-__host__ __device__ constexpr int producer_of(int warp) {  // 0 .. 7, or -1
-  return (warp < 5 || warp > 14 || warp % 4 == 0) ? -1 : (warp / 4 - 1) * 3 + warp % 4 - 1;
-}
-static_assert(producer_of(5) == 0 && producer_of(7) == 2 && producer_of(9) == 3 && producer_of(11) == 5 && producer_of(13) == 6 &&
-                  producer_of(14) == 7 && producer_of(8) == -1 && producer_of(12) == -1 && producer_of(4) == -1,
-              "eight producers on schedulers 1 to 3");
+// Sixteen producers in two teams on alternate stages: a stage's chain (raw bytes out of shared memory, repacking, stores, proxy
+// fence, arrival) took one team of eight 1,300 to 1,500 cycles, and was what the kernel waited for.
+constexpr int kProdWarps = 8, kTeams = 2;  // (warps a team)
+constexpr int kIssuerWarp = kTeams * kProdWarps, kRawWarp = kIssuerWarp + 1, kLoaderWarp = kIssuerWarp + 2;
 constexpr int kProdThreads = kProdWarps * kWarp;
 constexpr int kTasks = kM * 4 / kProdThreads;  // (row, MMA) tasks a producer thread takes a stage: 2
-constexpr int kThreads = 15 * kWarp;
+constexpr int kThreads = (kLoaderWarp + 1) * kWarp;
 constexpr int kStages = 3, kRawStages = 3;
 constexpr int kStepValues = 256, kMmaK = 64, kMmas = kStepValues / kMmaK;  // a stage: 256 values of K, four MMAs
 constexpr int kABytes = kM * kStepValues / 2;                              // 16 KB: 128 rows of 128 bytes, the tokens' layout
@@ -71,53 +63,12 @@ constexpr int kStageBytes = kABytes + kBBytes + kSfaBytes + kSfbBytes;     // 54
 static_assert(kABytes % 1024 == 0 && kStageBytes % 1024 == 0, "both tiles start on 1024 bytes: the swizzle's period");
 constexpr int kRawRow = 144;                // a row's raw bytes of one stage: 4 x 36 (NVFP4), or 8 x 17 = 136 and the 8 a
 constexpr int kRawBytes = kM * kRawRow;     // 16-byte window may start before them (MXFP4)
-constexpr uint64_t kWaitLimitNs = 200ull * 1000 * 1000;
 // tensor memory: the accumulator's 256 columns, then the scale factors of one stage (a column = 4 factors of 32 rows)
 constexpr uint32_t kSfaCol = 256, kSfbCol = kSfaCol + 16, kTmemCols = 512;
 
 __device__ uint32_t g_status;
 
-__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t) __cvta_generic_to_shared(p); }
-__device__ __forceinline__ uint64_t global_ns() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-__device__ __forceinline__ void bar_init(uint64_t* bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count));
-}
-__device__ __forceinline__ void bar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
-}
-__device__ __forceinline__ bool bar_wait(uint64_t* bar, uint32_t parity) {
-  const uint32_t a = smem_addr(bar);
-  uint64_t t0 = 0;
-  for (uint32_t spin = 0;; spin++) {
-    uint32_t done;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(done)
-        : "r"(a), "r"(parity)
-        : "memory");
-    if (done) return true;
-    if (spin == 0) t0 = global_ns();
-    else if (global_ns() - t0 > kWaitLimitNs) return false;
-  }
-}
-
-// shared-memory matrix descriptor: K-major, no swizzle, core matrices of 8 rows x 16 bytes; lbo: to the next 16 bytes of
-// K, sbo: to the next 8 rows (cute/arch/mma_sm100_desc.hpp: start >> 4, leading >> 4 at bit 16, stride >> 4 at bit 32,
-// version 1 at bit 46, layout type 0)
-__device__ __forceinline__ uint64_t tile_desc(uint32_t addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
-  return (uint64_t) ((addr >> 4) & 0x3FFFu) | (uint64_t) (lbo_bytes >> 4) << 16 | (uint64_t) (sbo_bytes >> 4) << 32 |
-         (uint64_t) 1 << 46;
-}
-
-// the same for the tokens' tile as the tensor-map copy writes it with the 128-byte swizzle: rows of 128 bytes (a stage's K of
-// a token), 8 rows 1024 bytes on; an MMA's 32 bytes of K start 32 bytes further into the row (layout type 2 at bit 61)
-__device__ __forceinline__ uint64_t tile_desc_sw128(uint32_t addr) {
-  return (uint64_t) ((addr >> 4) & 0x3FFFu) | (uint64_t) 1 << 16 | (uint64_t) (1024u >> 4) << 32 | (uint64_t) 1 << 46 | (uint64_t) 2 << 61;
-}
+using namespace tma;
 
 // where the 16 bytes j (0 .. 7) of row r's 128 bytes of K lie in a tile under the 128-byte swizzle: rows of 128 bytes, a
 // row's 16-byte pieces permuted by its place among its eight (what a tensor-map copy with that swizzle writes)
@@ -126,12 +77,14 @@ __device__ __forceinline__ uint32_t tile_at(uint32_t r, uint32_t j) { return r *
 __device__ __forceinline__ uint32_t chunk_at(uint32_t r) { return (r & 31u) * 16u + (r >> 5) * 4u; }
 
 // 16 values' nibbles to K order: `lo`, `hi` hold 8 bytes whose low nibbles are values 0 .. 7 and high nibbles values
-// 8 .. 15 (ggml's order); returns values 0 .. 7 and 8 .. 15 as two words, value j at bits 4 (j % 8)
+// 8 .. 15 (ggml's order); returns values 0 .. 7 and 8 .. 15 as two words, value j at bits 4 (j % 8). A byte of the result is
+// a nibble of an even byte and the same one of the next: a shift or two and one bitwise choice put them together in the even
+// bytes (ten instructions; the repacking is most of what the producers do).
 __device__ __forceinline__ uint2 k_order16(uint32_t lo, uint32_t hi) {
   const uint32_t m = 0x0F0F0F0Fu;
-  const uint32_t a0 = lo & m, a1 = hi & m, b0 = (lo >> 4) & m, b1 = (hi >> 4) & m;
-  // n | n' << 4 of neighbouring bytes lands in the even bytes; the two words' even bytes make one word
-  return make_uint2(__byte_perm(a0 | a0 >> 4, a1 | a1 >> 4, 0x6420), __byte_perm(b0 | b0 >> 4, b1 | b1 >> 4, 0x6420));
+  const uint32_t a0 = (lo & m) | ((lo >> 4) & ~m), a1 = (hi & m) | ((hi >> 4) & ~m);    // in the even bytes
+  const uint32_t b0 = ((lo >> 4) & m) | ((lo >> 8) & ~m), b1 = ((hi >> 4) & m) | ((hi >> 8) & ~m);
+  return make_uint2(__byte_perm(a0, a1, 0x6420), __byte_perm(b0, b1, 0x6420));
 }
 
 struct Args {
@@ -163,7 +116,6 @@ __global__ void __launch_bounds__(kThreads, 1) fp4_tc_kernel(const Args a, const
   const uint32_t n_mma = (n_valid + 15u) & ~15u;  // the MMA's N: whole 16s
   const uint32_t steps = a.cols / kStepValues;
   constexpr uint32_t kSfChunks = MX ? 2 : 4;  // chunks of 4 factors a stage: 256 values / (4 x 32) or / (4 x 16)
-  const uint64_t row_bytes = MX ? (uint64_t) (a.cols / 32) * 17 : (uint64_t) (a.cols / 64) * 36;
 
   if (tid == 0) {
     // a stage is full when every producer has stored its part of A (an arrival each), every producer's scale-byte copies
@@ -185,13 +137,13 @@ __global__ void __launch_bounds__(kThreads, 1) fp4_tc_kernel(const Args a, const
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = sh.tmem_base;
 
-  if (producer_of((int) warp) >= 0) {
+  if (warp < (uint32_t) kIssuerWarp) {
     // ================= producers =================
-    const uint32_t pt = (uint32_t) producer_of((int) warp) * kWarp + lane;
+    const uint32_t team = warp / kProdWarps, pt = tid % kProdThreads;
     const uint32_t raw0 = smem_addr(smem + kStages * kStageBytes);
     // this thread's token of the block: a warp takes tokens 8 b .. 8 b + 7 of each of a half's four 32-token groups,
     // whose words lie side by side in a chunk (32 lanes on 32 banks). A stage's scale bytes of a token are 16 (8)
-    // bytes in a row: one load.
+    // bytes in a row: one load. (Four warps of their own for this, two stages ahead, were slower: 164 -> 169 us.)
     const uint32_t sf_j = pt & 127u, sf_t128 = ((sf_j >> 3) & 3u) * 32u + (sf_j >> 5) * 8u + (sf_j & 7u);
     const uint32_t sf_t = (pt >> 7) * 128u + sf_t128, sf_at = chunk_at(sf_t128);
     const uint8_t* sf_row = a.as + (uint64_t) (c0 + (sf_t < n_valid ? sf_t : n_valid - 1)) * a.as_stride;
@@ -204,26 +156,25 @@ __global__ void __launch_bounds__(kThreads, 1) fp4_tc_kernel(const Args a, const
                      : "=r"(sfw[0]), "=r"(sfw[1]), "=r"(sfw[2]), "=r"(sfw[3])
                      : "l"(sf_row + (uint64_t) it * 16u));
     };
-    if (sf_t < n_mma) read_sf(0);
-    for (uint32_t it = 0; it < steps; it++) {
+    if (sf_t < n_mma && team < steps) read_sf(team);
+    for (uint32_t it = team; it < steps; it += kTeams) {
       const uint32_t stage = it % kStages, use = it / kStages;
-      if (use > 0 && !bar_wait(&sh.empty[stage], (use - 1) & 1u)) {
+      if (use > 0 && !bar_wait_soon(&sh.empty[stage], (use - 1) & 1u)) {
         sh.fail = 1;
         break;
       }
       const uint32_t st = smem_addr(smem + stage * kStageBytes);
       const uint32_t sa = st, sfa = st + kABytes + kBBytes, sfb = sfa + kSfaBytes;
-      // the tokens' scale bytes of the stage (read a stage ahead), a word into each chunk
+      // the tokens' scale bytes of the stage (read a team's stage ahead), a word into each chunk
       if (sf_t < n_mma) {
 #pragma unroll
         for (uint32_t ch = 0; ch < kSfChunks; ch++)
           asm volatile("st.shared.u32 [%0], %1;" ::"r"(sfb + (ch * 2u + (sf_t >> 7)) * kChunk + sf_at), "r"(sfw[ch]) : "memory");
-        if (it + 1 < steps) read_sf(it + 1);
       }
       // the stage's raw rows have landed (the loader's tensor-map copy): a task = (row, 64 values of K = one MMA's 32
       // bytes of the row), its raw bytes nine aligned words of the row's 144-byte window
       const uint32_t rs = it % kRawStages;
-      if (!bar_wait(&sh.raw_full[rs], (it / kRawStages) & 1u)) {
+      if (!bar_wait_soon(&sh.raw_full[rs], (it / kRawStages) & 1u)) {
         sh.fail = 1;
         break;
       }
@@ -277,6 +228,7 @@ __global__ void __launch_bounds__(kThreads, 1) fp4_tc_kernel(const Args a, const
         bar_arrive(&sh.full[stage]);
         bar_arrive(&sh.raw_empty[rs]);  // (the warp has read its part of the raw rows)
       }
+      if (sf_t < n_mma && it + kTeams < steps) read_sf(it + kTeams);
     }
   } else if (warp == (uint32_t) kRawWarp) {
     // ================= the rows' raw bytes =================
@@ -321,11 +273,11 @@ __global__ void __launch_bounds__(kThreads, 1) fp4_tc_kernel(const Args a, const
     // ================= issuer =================
     // instruction descriptor (block scaled): A and B E2M1 (format 1), both K-major, N, the scale format, M = 128
     const uint32_t idesc = (1u << 7) | (1u << 10) | ((n_mma >> 3) << 17) | ((MX ? 1u : 0u) << 23) | ((uint32_t) (kM >> 4) << 24);
-    // (one lane runs the whole loop: nothing here is the warp's, and the other lanes' polling and the meeting after
-    // every stage only stood in its way)
-    for (uint32_t it = 0; lane == 0 && it < steps && !sh.fail; it++) {
+    // (the whole warp runs the loop and one elected lane issues: see tma.cuh)
+    const uint32_t issuer = elect_one();
+    for (uint32_t it = 0; it < steps; it++) {
       const uint32_t stage = it % kStages, use = it / kStages;
-      if (!bar_wait(&sh.full[stage], use & 1u)) {
+      if (!bar_wait_soon(&sh.full[stage], use & 1u)) {
         sh.fail = 1;
         break;
       }
@@ -340,13 +292,13 @@ __global__ void __launch_bounds__(kThreads, 1) fp4_tc_kernel(const Args a, const
         const uint64_t sfa0 = kSfDesc | ((st + kABytes + kBBytes) >> 4), sfb0 = kSfDesc | ((st + kABytes + kBBytes + kSfaBytes) >> 4);
         // a chunk of scale factors (32 lanes x 16 bytes = 4 columns of tensor memory) for the rows and two for the tokens,
         // then the MMAs that read them: the first MMA of a stage starts after three copies, not twelve
+        auto copy = [&](uint32_t to, uint64_t from) {
+          asm volatile("{\n .reg .pred e;\n setp.ne.b32 e, %2, 0;\n @e tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;\n}\n" ::"r"(to), "l"(from), "r"(issuer) : "memory");
+        };
         auto copy_chunk = [&](uint32_t ch) {
-          asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(tmem + kSfaCol + 4u * ch), "l"(sfa0 + ch * (kChunk >> 4)) : "memory");
-          asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(tmem + kSfbCol + 8u * ch), "l"(sfb0 + 2u * ch * (kChunk >> 4)) : "memory");
-          if (n_mma > 128u)
-            asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(tmem + kSfbCol + 8u * ch + 4u),
-                         "l"(sfb0 + (2u * ch + 1u) * (kChunk >> 4))
-                         : "memory");
+          copy(tmem + kSfaCol + 4u * ch, sfa0 + ch * (kChunk >> 4));
+          copy(tmem + kSfbCol + 8u * ch, sfb0 + 2u * ch * (kChunk >> 4));
+          if (n_mma > 128u) copy(tmem + kSfbCol + 8u * ch + 4u, sfb0 + (2u * ch + 1u) * (kChunk >> 4));
         };
 #pragma unroll
         for (uint32_t mm = 0; mm < (uint32_t) kMmas; mm++) {
@@ -357,35 +309,40 @@ __global__ void __launch_bounds__(kThreads, 1) fp4_tc_kernel(const Args a, const
           if constexpr (!MX) {  // a chunk a MMA: its four factors are the MMA's four 16s
             copy_chunk(mm);
             asm volatile(
-                "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                " tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.block16 [%0], %1, %2, %3, [%5], [%6], p;\n}\n" ::"r"(tmem),
-                "l"(da), "l"(db), "r"(idesc), "r"(accumulate), "r"(tmem + kSfaCol + 4u * mm), "r"(tmem + kSfbCol + 8u * mm)
+                "{\n .reg .pred e, p;\n setp.ne.b32 e, %7, 0;\n setp.ne.b32 p, %4, 0;\n"
+                " @e tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.block16 [%0], %1, %2, %3, [%5], [%6], p;\n}\n" ::"r"(tmem),
+                "l"(da), "l"(db), "r"(idesc), "r"(accumulate), "r"(tmem + kSfaCol + 4u * mm), "r"(tmem + kSfbCol + 8u * mm), "r"(issuer)
                 : "memory");
           } else {  // a chunk two MMAs: factors 0, 1 then 2, 3 (the factor id in the descriptor is the first's byte)
             if ((mm & 1u) == 0) copy_chunk(mm >> 1);
             const uint32_t id = 2u * (mm & 1u), idesc_mm = idesc | (id << 4) | (id << 29);
             asm volatile(
-                "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                " tcgen05.mma.cta_group::1.kind::mxf4.block_scale.block32 [%0], %1, %2, %3, [%5], [%6], p;\n}\n" ::"r"(tmem),
+                "{\n .reg .pred e, p;\n setp.ne.b32 e, %7, 0;\n setp.ne.b32 p, %4, 0;\n"
+                " @e tcgen05.mma.cta_group::1.kind::mxf4.block_scale.block32 [%0], %1, %2, %3, [%5], [%6], p;\n}\n" ::"r"(tmem),
                 "l"(da), "l"(db), "r"(idesc_mm), "r"(accumulate), "r"(tmem + kSfaCol + 4u * (mm >> 1)),
-                "r"(tmem + kSfbCol + 8u * (mm >> 1))
+                "r"(tmem + kSfbCol + 8u * (mm >> 1)), "r"(issuer)
                 : "memory");
           }
         }
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(&sh.empty[stage])) : "memory");
-        if (it + 1 == steps)
-          asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(&sh.acc_full)) : "memory");
+        mma_commit(issuer, &sh.empty[stage]);
+        if (it + 1 == steps) mma_commit(issuer, &sh.acc_full);
       }
     }
-    __syncwarp();
-  } else {
-    // ================= epilogue =================
-    const uint32_t row = 32u * warp + lane;  // this thread's weight row of the tile = its TMEM lane
-    const uint32_t lane_base = tmem + ((32u * warp) << 16);
-    float* y = a.y + (uint64_t) c0 * a.ys + row0 + row;
-    if (tma::bar_wait_warp(&sh.acc_full, 0)) {
+  }
+  // ================= epilogue =================
+  // Every warp, once its own role is done: a warp reads the tensor-memory lanes of its quarter (its index mod 4: the hardware's
+  // rule), so the three or four warps of a quarter share its rows' 32-token chunks.
+  __syncwarp();
+  {
+    const uint32_t quarter = warp % 4u, part = warp / 4u, parts = ((uint32_t) (kThreads / kWarp) - quarter + 3u) / 4u;
+    const uint32_t row = 32u * quarter + lane;  // this thread's weight row of the tile = its TMEM lane
+    const uint32_t lane_base = tmem + ((32u * quarter) << 16);
+    bool landed = false;  // (the K loop's own waits are 0.2 s each and can queue up: look again while nobody has given up)
+    for (uint32_t tries = 0; tries < 25u && !landed && !__any_sync(0xFFFFFFFFu, *(volatile int*) &sh.fail); tries++)
+      landed = bar_wait_long(&sh.acc_full, 0);
+    if (landed) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      for (uint32_t col = 0; col < n_mma; col += 32) {
+      for (uint32_t col = 32u * part; col < n_mma; col += 32u * parts) {
         uint32_t r[32];
         asm volatile(
             "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
@@ -397,9 +354,10 @@ __global__ void __launch_bounds__(kThreads, 1) fp4_tc_kernel(const Args a, const
             : "r"(lane_base + col)
             : "memory");
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        float* y = a.y + (uint64_t) (c0 + col) * a.ys + row0 + row;
 #pragma unroll
-        for (int i = 0; i < 32; i++)
-          if (col + i < n_valid) y[(uint64_t) (col + i) * a.ys] = mul_rn(__uint_as_float(r[i]), a.scale);
+        for (int i = 0; i < 32; i++, y += a.ys)
+          if (col + i < n_valid) *y = mul_rn(__uint_as_float(r[i]), a.scale);
       }
     } else {
       sh.fail = 1;
