@@ -163,8 +163,6 @@ __device__ __forceinline__ uint4 lds_16(uint32_t at, bool whole) {  // 16 bytes 
 // with the integer fields included) has at most 24 significant bits, as in all of these types, fma(d, n, c) is the product
 // rounded, exactly, and then the sum, rounded: decode8's two operations. An infinite or NaN scale is not exact times 2^24 or an
 // integer, so such a step goes through decode8 (`odd`: the warp's, as tcgen05.st is the whole warp's).
-__device__ __forceinline__ float low_half(uint32_t h) { return __half2float(__ushort_as_half((unsigned short) (h & 0xFFFFu))); }
-__device__ __forceinline__ float high_half(uint32_t h) { return __half2float(__ushort_as_half((unsigned short) (h >> 16))); }
 struct Affine {  // n 2^-24 -> d n + c
   uint64_t d, c;
   __device__ __forceinline__ Affine(float scale, float plus) : d(pack2(mul_rn(scale, 16777216.0f), mul_rn(scale, 16777216.0f))), c(pack2(plus, plus)) {}

@@ -86,7 +86,7 @@ template <uint32_t T> __host__ __device__ constexpr uint32_t stretch_bytes() { r
 // the 136 of MXFP4 and IQ4_XS, where an odd stretch starts 8 bytes into a piece)
 template <uint32_t T> constexpr bool kWhole = stretch_bytes<T>() % 16 == 0;
 // types whose two nibbles go through a table of 256 (low, high) value pairs, two bf16 (the values are exact in it)
-template <uint32_t T> constexpr bool kPairTable = (T == QTYPE_MXFP4 || T == QTYPE_IQ4_XS);
+template <uint32_t T> constexpr bool kPairTable = (T == QTYPE_IQ4_XS);
 constexpr uint32_t kTableBytes = 256u * 128u;  // a copy a lane: every lookup its own bank
 struct Table {
   const uint8_t* at;
@@ -138,12 +138,28 @@ template <> struct Pair<QTYPE_MXFP4> {
   uint32_t off, sh, eoff;
   __device__ __forceinline__ explicit Pair(uint32_t p) : off((p >> 1) * 17u + 1u + 8u * (p & 1u)), sh(off % 4u * 8u), eoff((p >> 1) * 17u) { off &= ~3u; }
   static __device__ __forceinline__ uint32_t lane(uint32_t p) { return (p >> 1) * 4u + (p & 1u); }
-  static __device__ __forceinline__ float entry(uint32_t n) { return (float) osmos_e2m1_doubled[n]; }
-  __device__ __forceinline__ void values(uint32_t at, const Table& tbl, uint64_t* v) const {
+  // An E2M1 code's bits as an F16's sign, exponent's low two bits and mantissa's top one are its value times 2^-14 (a subnormal
+  // code is a subnormal F16); to F32 exactly, times 2^(e - 113): one rounding, of the value itself, as decode8's product. Past
+  // e = 240 that factor is no F32: half the scale times the doubled code, as there. (Against a table of 256 pairs in shared memory, a copy
+  // a lane, which took most of its passes.)
+  __device__ __forceinline__ void values(uint32_t at, const Table&, uint64_t* v) const {
     const uint2 q = lds_8_bytes(at + off, sh);
-    const float d = e8m0_value(lds8(at + eoff), 128);  // half the block's scale: the table holds the codes' values doubled
+    const uint32_t e = lds8(at + eoff);
+    const bool large = e > 240u;
+    const float d = e8m0_value(e, large ? 128 : 113), one = large ? 32768.0f : 1.0f;
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+      const uint32_t w = i ? q.y : q.x;
+      const uint32_t lo = ((w << 1) & 0x0E0E0E0Eu) | ((w << 4) & kTops), hi = ((w >> 3) & 0x0E0E0E0Eu) | (w & kTops);
+      const uint32_t le = (lo << 8) & 0xFF00FF00u, lp = lo & 0xFF00FF00u, he = (hi << 8) & 0xFF00FF00u, hp = hi & 0xFF00FF00u;
+      v[4 * i] = pack2(low_half(le), low_half(he)), v[4 * i + 1] = pack2(low_half(lp), low_half(hp));
+      v[4 * i + 2] = pack2(high_half(le), high_half(he)), v[4 * i + 3] = pack2(high_half(lp), high_half(hp));
+    }
     const uint64_t dd = pack2(d, d);
-    table_pairs(q, tbl, v);
+    if (large) {
+#pragma unroll
+      for (int j = 0; j < kChunk; j++) v[j] = mul2(v[j], pack2(one, one));
+    }
 #pragma unroll
     for (int j = 0; j < kChunk; j++) v[j] = mul2(dd, v[j]);
   }

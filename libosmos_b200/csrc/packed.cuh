@@ -34,6 +34,12 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
   return r;
 }
 
+// An integer n < 1024 in the low bits of a half IS the subnormal F16 n 2^-24, and F16 to F32 is exact: codes masked in place, two
+// to a word, reach F32 (times 2^-24, which a scale taken 2^24 times larger gives back) without a byte permute each, and the
+// conversion runs beside the integer pipe.
+__device__ __forceinline__ float low_half(uint32_t h) { return __half2float(__ushort_as_half((unsigned short) (h & 0xFFFFu))); }
+__device__ __forceinline__ float high_half(uint32_t h) { return __half2float(__ushort_as_half((unsigned short) (h >> 16))); }
+
 // byte J of `bytes` (n < 256) as the F32 32768 + n: bits 8 .. 15 of 0x47000000, one byte permute
 template <int J> __device__ __forceinline__ uint32_t biased_byte(uint32_t bytes) { return __byte_perm(bytes, 0x47000000u, 0x7404 | (J << 4)); }
 // a byte of a word as F32, exactly
