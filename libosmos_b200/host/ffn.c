@@ -185,7 +185,8 @@ static uint64_t carve_q4x(const Q4xMoeLayer *l, uint32_t max_tok, uint8_t *mem, 
   PART(yg, uint32_t, b.entries);
   PART(xd, uint32_t, b.entries);
   PART(yd, uint32_t, b.entries);
-  PART(xe16, uint16_t, (uint64_t)b.slots * widest);
+  /* (whole tiles of 16 slots: a tile's slots are interleaved, so the last one's live slots reach to its end) */
+  PART(xe16, uint16_t, ((uint64_t)b.slots + MM_TILE - 1) / MM_TILE * MM_TILE * widest);
   PART(ga, float, (uint64_t)picks * l->ff);
   PART(up, float, (uint64_t)picks * l->ff);
   PART(y, float, (uint64_t)picks * l->dim);
