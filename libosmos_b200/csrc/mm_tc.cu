@@ -373,6 +373,7 @@ struct Args {
   uint32_t n_mat, row_tiles;
   uint32_t span;     // the most tokens a tile takes
   uint32_t use_tma;  // the activations come by tensor-map copies, else by 16-byte cp.async
+  uint32_t early;    // the kernel ahead made x16 (mm_tokens): what does not need it starts before it has ended
   uint32_t raw_map;  // the weights too (Maps::raw); grouped: the matrices are those of one tensor, `bytes` apart from `base` on
   const uint8_t* base;
   uint64_t bytes;
@@ -458,6 +459,12 @@ __global__ void __launch_bounds__(kThreads, 1) mm_tc_kernel(const Args a, const 
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&sh.tmem_base)), "r"(512));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
+  // (a dependent launch: the counts, x16 and the readers of y may be the kernel ahead's. Where that kernel is this call's own
+  // conversion - launched the ordinary way, so that whatever wrote the weights is over - the weights' loads and their
+  // decoding need not wait for it, only the tokens' loads and the stores. Q4_K 4096 x 4096, 777 tokens: 37.1 -> 34.5 us; MXFP4
+  // 2560 x 1536, 126 tokens: 16.4 -> 14.4.)
+  if (!a.early) pdl_wait();
+  pdl_launch_next();
   // the matrices' first tiles, a thread each, and the most tokens a tile has
   const uint32_t n_mat = a.wt ? a.n_mat : 1u;
   static_assert(kMaxMats <= (uint32_t) kThreads, "a thread a matrix");
@@ -633,6 +640,7 @@ __global__ void __launch_bounds__(kThreads, 1) mm_tc_kernel(const Args a, const 
     asm volatile("cp.async.wait_all;" ::: "memory");
   } else if (warp == (uint32_t) kTokenWarp) {
     // ================= the activations' loader =================
+    if (a.early) pdl_wait();
     uint32_t s = 0, slot = 0;
     bool ok = true;
     for (uint32_t t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
@@ -727,6 +735,7 @@ __global__ void __launch_bounds__(kThreads, 1) mm_tc_kernel(const Args a, const 
     }
   } else {
     // ================= epilogue =================
+    if (a.early) pdl_wait();
     const uint32_t row = 32u * warp + lane;  // this thread's weight row of the tile = its TMEM lane
     uint32_t acc = 0;
     bool ok = true;
@@ -903,8 +912,8 @@ bool launch(Args a, uint32_t n_mat, uint32_t max_cnt, cudaStream_t s) {
       c.n_mat = n_mat - m0 < kMaxMats ? n_mat - m0 : kMaxMats;
       c.wt += m0, c.cnt += m0, c.xoff += m0, c.yoff += m0;
       const uint64_t tiles = (uint64_t) a.row_tiles * c.n_mat * parts_of(max_cnt, a.span);
-      mm_tc_kernel<T, EPI><<<(unsigned) (tiles < (uint64_t) sms ? tiles : (uint64_t) sms), kThreads, kBytes, s>>>(c, maps);
-      if (!launched()) return false;
+      const dim3 grid((unsigned) (tiles < (uint64_t) sms ? tiles : (uint64_t) sms));
+      if (launch_dependent(mm_tc_kernel<T, EPI>, grid, dim3(kThreads), kBytes, s, c, maps) != cudaSuccess) return false;
     }
     return true;
   }
@@ -921,8 +930,8 @@ bool launch(Args a, uint32_t n_mat, uint32_t max_cnt, cudaStream_t s) {
   a.use_tma = x16_map(a.x16, parts_of(a.n, MM_TILE), a.xts, a.span, &maps.map[0]) ? 1u : 0u, a.n_mat = 1;
   const uint64_t tiles = (uint64_t) a.row_tiles * parts_of(a.n, a.span);
   if (tiles > 0xFFFFFFFFull) return false;
-  mm_tc_kernel<T, EPI><<<(unsigned) (tiles < (uint64_t) sms ? tiles : (uint64_t) sms), kThreads, kBytes, s>>>(a, maps);
-  return launched();
+  const dim3 grid((unsigned) (tiles < (uint64_t) sms ? tiles : (uint64_t) sms));
+  return launch_dependent(mm_tc_kernel<T, EPI>, grid, dim3(kThreads), kBytes, s, a, maps) == cudaSuccess;
 }
 
 }  // namespace
@@ -942,12 +951,12 @@ bool run_with(uint32_t type, const Args& a, void* stream) {
 }  // namespace
 
 bool run(uint32_t type, const void* w, uint32_t rows, uint32_t cols, const void* x16, uint32_t n, float* y, uint32_t ys,
-         float scale, void* stream) {
+         float scale, void* stream, bool early) {
   if (!w || !x16 || !y || !n || n > MM_MAX_TOKENS || !shape_ok(type, rows, cols) || (n > 1 && ys < rows)) return false;
   if ((uintptr_t) x16 & 15u) return false;
   Args a{};
   a.w = (const uint8_t*) w, a.x16 = (const __half*) x16, a.y = y, a.rows = rows, a.cols = cols, a.n = n, a.xts = cols;
-  a.ys = ys, a.scale = scale;
+  a.ys = ys, a.scale = scale, a.early = early ? 1u : 0u;
   return run_with<kStore>(type, a, stream);
 }
 
@@ -1031,8 +1040,9 @@ extern "C" bool mm_tokens_scaled(uint32_t type, const void* w0, uint32_t rows0, 
   if ((uintptr_t) x16 & 15u) return false;
   for (uint32_t t0 = 0; t0 < n; t0 += MM_MAX_TOKENS) {  // MM_MAX_TOKENS a time through the one x16
     const uint32_t c = n - t0 < MM_MAX_TOKENS ? n - t0 : MM_MAX_TOKENS;
-    if (!(ready && n <= MM_MAX_TOKENS) && !mm_x16(x + (uint64_t) t0 * xs, xs, c, cols, x16, overflow, stream)) return false;
-    if (!mm_tc::run(type, w0, rows0, cols, x16, c, y0 + (uint64_t) t0 * ys0, ys0, s0, stream)) return false;
+    const bool convert = !(ready && n <= MM_MAX_TOKENS);
+    if (convert && !mm_x16(x + (uint64_t) t0 * xs, xs, c, cols, x16, overflow, stream)) return false;
+    if (!mm_tc::run(type, w0, rows0, cols, x16, c, y0 + (uint64_t) t0 * ys0, ys0, s0, stream, convert)) return false;
     if (w1 && !mm_tc::run(type, w1, rows1, cols, x16, c, y1 + (uint64_t) t0 * ys1, ys1, s1, stream)) return false;
   }
   return true;

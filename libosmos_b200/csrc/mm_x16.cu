@@ -25,6 +25,7 @@ struct X16Args {
 
 template <bool VEC>
 __global__ void __launch_bounds__(kThreads) x16_kernel(const X16Args a) {
+  pdl_launch_next();  // (the product behind this may set itself up and bring its first weights; it waits for x16)
   const uint64_t run = (uint64_t) blockIdx.x * kThreads + threadIdx.x;  // over heads x tiled runs
   const uint64_t per_head = (uint64_t) a.slots16 * a.cols / kRun;
   if (run >= per_head * a.heads) return;
