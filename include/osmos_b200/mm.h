@@ -74,10 +74,10 @@ bool mm_x16_attn(const float *x, uint32_t xs, uint32_t n, uint32_t cols, uint32_
    tiles: rows a multiple of 16, cols a multiple of 128 and whole blocks (reference: mm.h:10-11) */
 bool mm_known(uint32_t type);
 bool mm_fits(uint32_t type, uint32_t rows, uint32_t cols);
-/* the launch class of a matrix with n tokens - how many 128-token accumulators a block carries at most: 1, 2 or 4; 0
+/* the launch class of a matrix with n tokens - by 128 tokens: 1, 2 or 4; 0
    for a type without a kernel (reference: mm.h:12, kernels/mm.hip:161-167, 455-465, where it is the column tiles a
-   block takes). A caller sorts mm_group's matrices by count and makes one launch a run of equal classes
-   (src/run/hip_ffn.c:110-127), so that a matrix of few tokens is not run in a kernel sized for many. */
+   block takes). The reference's callers sort mm_group's matrices by count and make one launch a run of equal classes
+   (src/run/hip_ffn.c:110-127); here one launch takes them all, its tiles sized by each matrix's own count. */
 uint32_t mm_col_tiles(uint32_t type, uint32_t n);
 /* y[t * ys + r] = sum_c W[r, c] x16[t][c], t < n <= MM_MAX_TOKENS; x16 as mm_x16 lays it (rows of cols values)
    (reference: mm.h:15). false for a type without a kernel, a shape that does not tile, n 0 or past MM_MAX_TOKENS,

@@ -20,14 +20,19 @@
 //                        mm_run_gated_mean the block's rows are hc streams' rows of the same dim values (row map
 //                        below), each thread gates its sum, and the streams are added in order through shared memory
 //   producers (16 warps, four teams of four on every fourth K step) decode the rows' bytes out of shared memory
-//   issuer (1 warp)      a K step's tcgen05.mma M128 N<=128 K16 (four an accumulator; the first of a tile overwrites, the
-//                        rest accumulate), then tcgen05.commit onto the step's "empty" mbarrier; after a tile's last step a
-//                        commit onto its accumulators' "full" ones
-//   raw loaders (2 warps) cp.async of the rows' bytes, 256 values of K at a time (128 of the widest types), a ring of
-//                        three or four
-//   token loader (1 warp) the tokens' x16, a K step at a time: one tensor-map copy (mm_run), or 16-byte cp.async pieces
-//                        (mm_group: an expert's tokens start anywhere in x16, and a copy of a 512-byte fragment each costs ~45
-//                        cycles to issue), its arrivals on the stage's mbarrier made by the hardware when the copies land
+//   issuer (1 warp)      a unit of one or two K steps: tcgen05.mma M128 N<=128 K16, eight a step (the even and the odd tokens; the
+//                        first of a tile overwrite, the rest accumulate), then tcgen05.commit onto the unit's "empty" mbarrier; after
+//                        a tile's last step a commit onto its accumulators' "full" ones. The whole warp runs this, one elected
+//                        lane issues.
+//   raw loaders (2 warps) the rows' bytes, 256 values of K at a time (128 of the widest types), a ring of three or four: one
+//                        tensor-map copy where rows start on 16 bytes, else 16-byte cp.async pieces
+//   token loader (1 warp) the tokens' x16, a K step a tensor-map copy; grouped tokens that start inside a tile of x16 by 16-byte
+//                        cp.async pieces
+// Bound by the decoders' integer and F32 pipes up to about 128 tokens a tile (a 64-value step of 128 rows is some 330 instructions
+// a thread, 300 to 400 cycles; its products are 128 cycles at 64 tokens), past that by the tokens' copies, 32 KB a step at 256 tokens
+// where the products take 512 cycles. Measured, against decoded tiles in shared memory, a tile a block (with the tokens' rounding):
+// Q4_K 4096 x 4096 at 777 / 2048 tokens 62.8 / 106 us -> 40.7 / 71; 128 MXFP4 experts of 1536 x 4096 over 2048 tokens, the
+// layer, 1827 -> 769.
 // Every mbarrier wait is bounded (%globaltimer) with one outcome a warp; a wait that runs out raises the status word, every
 // role falls through to the common exit and tensor memory is released.
 #include <cuda.h>

@@ -1,0 +1,101 @@
+"""GPU parity of the f16 product at the edges of its tiles and of its ways to bring operands: row tiles and token tiles of every
+shape (one accumulator, both, an odd number of 16-token tiles), matrices whose rows start on 16 bytes (tensor-map copies) and
+not (16-byte copies), K of half a raw block, tokens that start inside a tile of the grouped x16, more matrices than a launch
+takes, and an expert tensor by its base. Bounds and the oracle as in test_gpu_mm.py."""
+import numpy as np
+import pytest
+import torch
+
+from helpers import ptr, same_bits, sync, to_dev
+from libosmos_b200 import synth
+from oracle.oracle import TYPES
+from test_gpu_mm import _exact, _within, _x16
+
+pytestmark = pytest.mark.gpu
+
+
+# cols: 128 and 384 leave half a 256-value block; MXFP4 at 256 / 768 / 1280 columns and Q6_K at 256 have rows that do not start on
+# 16 bytes; off: where in its allocation the matrix starts
+@pytest.mark.parametrize("name,rows,cols,off", [
+    ("MXFP4", 16, 128, 0), ("MXFP4", 272, 512, 0), ("MXFP4", 272, 512, 8), ("MXFP4", 144, 1280, 0), ("MXFP4", 128, 384, 1),
+    ("Q4_K", 16, 256, 0), ("Q4_K", 400, 512, 0), ("Q4_K", 144, 768, 4), ("Q4_K", 144, 256, 2), ("Q5_K", 272, 512, 0), ("Q5_K", 144, 512, 4),
+    ("Q6_K", 144, 256, 0), ("Q6_K", 272, 2048, 0), ("Q8_0", 144, 128, 0), ("Q8_0", 272, 512, 0), ("Q8_0", 144, 512, 2),
+    ("Q4_0", 144, 384, 0), ("Q4_0", 272, 512, 2), ("IQ3_XXS", 144, 2048, 0), ("IQ1_M", 144, 512, 0), ("MXFP8", 144, 384, 0)])
+def test_tiles(lib, dev, oracle, name, rows, cols, off):
+    tid = TYPES[name]
+    rng = synth.rng_for(61, tid * 10000 + rows + cols + off)
+    w = synth.random_tensor(tid, rows, cols, rng)
+    mem = torch.zeros(w.size + 64, dtype=torch.uint8, device=dev)
+    mem[off:off + w.size] = to_dev(w.reshape(-1).view(np.uint8), dev)
+    lib.mm_status()
+    first = None
+    for n in (1, 16, 17, 33, 48, 127, 128, 129, 144, 255, 256, 257, 400):
+        x = synth.rng_for(62, 7).standard_normal((n, cols)).astype(np.float32)  # (the same leading tokens at every count)
+        exact, mag = _exact(oracle, tid, w, rows, cols, x)
+        y = torch.full((n, rows + 1), -7.0, dtype=torch.float32, device=dev)
+        assert lib.mm_run(tid, mem.data_ptr() + off, rows, cols, ptr(_x16(lib, dev, x, cols)), n, ptr(y), rows + 1, None)
+        sync()
+        got = y.cpu().numpy()
+        assert (got[:, rows] == -7.0).all() and _within(got[:, :rows], exact, mag, cols), n
+        first = got[0, :rows].copy() if first is None else first
+        assert same_bits(got[0, :rows], first), n  # (a token's bits do not depend on the count)
+    assert lib.mm_status() == 0
+
+
+@pytest.mark.parametrize("shift", [0, 8, 24])
+def test_group_tokens_anywhere(lib, dev, shift):
+    """matrices of 1 .. 260 tokens whose x16 starts on a tile or (shift halves on) inside one, by pointers and by their tensor's
+    base: the bits mm_run gives"""
+    tid = TYPES["MXFP4"]
+    rows, cols, cnt = 144, 512, [5, 0, 129, 260, 1, 64]
+    rng = synth.rng_for(63)
+    nb = synth.tensor_bytes(tid, rows, cols)
+    w = np.concatenate([synth.random_tensor(tid, rows, cols, rng).reshape(-1).view(np.uint8) for _ in cnt])
+    wd = to_dev(w, dev)
+    xs = [rng.standard_normal((max(c, 1), cols)).astype(np.float32) for c in cnt]
+    tiles = [(c + 15) // 16 for c in cnt]
+    x16 = torch.zeros(sum(tiles) * 16 * cols + shift, dtype=torch.float16, device=dev)
+    xoff, yoff, at, ya = [], [], shift, 0
+    for x, c, t in zip(xs, cnt, tiles):
+        xoff.append(at), yoff.append(ya)
+        if c:
+            x16[at:at + t * 16 * cols] = _x16(lib, dev, x[:c], cols)
+        at, ya = at + t * 16 * cols, ya + c * rows
+    table = torch.tensor([wd.data_ptr() + m * nb for m in range(len(cnt))], dtype=torch.int64, device=dev)
+    args = [to_dev(np.array(a, t), dev) for a, t in ((cnt, np.int32), (xoff, np.uint32), (yoff, np.uint32))]
+    lib.mm_status()
+    for by_base in (False, True):
+        y = torch.full((ya + 1,), -3.0, dtype=torch.float32, device=dev)
+        base = (ptr(wd), nb, len(cnt)) if by_base else (0, 0, 0)
+        assert lib.mm_group_of(tid, *base, ptr(table), ptr(args[0]), len(cnt), 260, rows, cols, ptr(x16), ptr(args[1]), cols, ptr(y), ptr(args[2]),
+                               rows, None)
+        sync()
+        got = y.cpu().numpy()
+        assert got[-1] == -3.0
+        for m, c in enumerate(cnt):
+            if c:
+                one = torch.empty((c, rows), dtype=torch.float32, device=dev)
+                assert lib.mm_run(tid, wd.data_ptr() + m * nb, rows, cols, ptr(_x16(lib, dev, xs[m][:c], cols)), c, ptr(one), rows, None)
+                sync()
+                assert same_bits(got[yoff[m]:yoff[m] + c * rows].reshape(c, rows), one.cpu().numpy())
+    assert lib.mm_status() == 0
+
+
+def test_group_of_many(lib, dev):
+    """more matrices than one launch keeps (768): entries of one token each, every seventh without"""
+    tid, rows, cols, n_mat = TYPES["Q4_0"], 16, 128, 1600
+    rng = synth.rng_for(64)
+    w = to_dev(synth.random_tensor(tid, rows, cols, rng), dev)
+    x = rng.standard_normal((1, cols)).astype(np.float32)
+    x16 = _x16(lib, dev, x, cols)
+    cnt = np.array([0 if m % 7 == 3 else 1 for m in range(n_mat)], np.int32)
+    table = torch.full((n_mat,), w.data_ptr(), dtype=torch.int64, device=dev)
+    y = torch.full((n_mat, rows), -3.0, dtype=torch.float32, device=dev)
+    one = torch.empty((1, rows), dtype=torch.float32, device=dev)
+    assert lib.mm_run(tid, ptr(w), rows, cols, ptr(x16), 1, ptr(one), rows, None)
+    assert lib.mm_group(tid, ptr(table), ptr(to_dev(cnt, dev)), n_mat, 1, rows, cols, ptr(x16), ptr(to_dev(np.zeros(n_mat, np.uint32), dev)), cols,
+                        ptr(y), ptr(to_dev(np.arange(n_mat, dtype=np.uint32) * rows, dev)), rows, None)
+    sync()
+    got = y.cpu().numpy()
+    assert same_bits(got[cnt == 1], np.repeat(one.cpu().numpy(), int(cnt.sum()), 0)) and (got[cnt == 0] == -3.0).all()
+    assert lib.mm_status() == 0
