@@ -376,6 +376,12 @@ struct Args {
   float* y;
   uint32_t rows, cols, n, xts, ys;
   uint32_t n_mat, row_tiles;
+  // a second matrix over the same tokens (w1 NULL: none), its row tiles after the first one's in the same launch: the shared
+  // expert's gate and up, 16 row tiles each, 32 us one after the other
+  const uint8_t* w1;
+  float* y1;
+  uint32_t rows1, ys1, row_tiles1;
+  float scale1;
   uint32_t span;     // the most tokens a tile takes
   uint32_t use_tma;  // the activations come by tensor-map copies, else by 16-byte cp.async
   uint32_t early;    // the kernel ahead made x16 (mm_tokens): what does not need it starts before it has ended
@@ -396,7 +402,7 @@ struct Args {
 };
 struct Maps {  // the tokens' maps: of a grouped launch map t a box of t + 1 token tiles, else the one map's box is a.span tokens
   CUtensorMap map[kMaxSpan / MM_TILE];
-  CUtensorMap raw;  // the weights' bytes as [matrix][row][byte]
+  CUtensorMap raw, raw1;  // the weights' bytes as [matrix][row][byte]; the second matrix's
 };
 enum : uint32_t { kStore = 0, kSilu = 1, kGatedMean = 2 };
 
@@ -416,6 +422,7 @@ __host__ __device__ constexpr uint32_t parts_of(uint32_t n, uint32_t of) { retur
 // go up). A matrix's tokens are dealt in equal whole tiles of 16.
 struct Tile {
   uint32_t m, rt, c0, n;  // its matrix and row tile; its first token and their number
+  bool second;            // the second matrix's
 };
 __device__ __forceinline__ Tile tile_at(const Args& a, const uint32_t* first, uint32_t t, uint32_t& m, uint32_t lane) {
   if (a.wt) {
@@ -430,6 +437,8 @@ __device__ __forceinline__ Tile tile_at(const Args& a, const uint32_t* first, ui
   const uint32_t each = whole16(parts_of(n, cols));
   Tile r;
   r.m = m, r.rt = in / cols, r.c0 = (in - r.rt * cols) * each;
+  r.second = r.rt >= a.row_tiles;
+  if (r.second) r.rt -= a.row_tiles;
   r.n = r.c0 < n ? min(each, n - r.c0) : 0u;
   return r;
 }
@@ -475,7 +484,7 @@ __global__ void __launch_bounds__(kThreads, 1) mm_tc_kernel(const Args a, const 
   static_assert(kMaxMats <= (uint32_t) kThreads, "a thread a matrix");
   {
     const uint32_t n = tid < n_mat ? (a.wt ? (uint32_t) max(a.cnt[tid], 0) : a.n) : 0u, cols = parts_of(n, a.span);
-    const uint32_t mine = cols * a.row_tiles, most = __reduce_max_sync(0xFFFFFFFFu, n ? whole16(parts_of(n, cols)) : 0u);
+    const uint32_t mine = cols * (a.row_tiles + a.row_tiles1), most = __reduce_max_sync(0xFFFFFFFFu, n ? whole16(parts_of(n, cols)) : 0u);
     uint32_t sum = mine;
 #pragma unroll
     for (int o = 1; o < kWarp; o <<= 1) {
@@ -517,14 +526,15 @@ __global__ void __launch_bounds__(kThreads, 1) mm_tc_kernel(const Args a, const 
     bool ok = true;
     for (uint32_t t = blockIdx.x; t < tiles && ok; t += gridDim.x, s0 += steps, rb0 += kblocks) {
       const Tile tl = tile_at(a, first, t, m_at, lane);
-      const uint8_t* w = a.wt ? a.wt[tl.m] : a.w;
+      const uint8_t* w = a.wt ? a.wt[tl.m] : tl.second ? a.w1 : a.w;
+      const uint32_t rows = tl.second ? a.rows1 : a.rows;
       // (the weight row behind row r of the tile: see the raw loaders; here only where it starts in its 16-byte piece)
       uint32_t row;
       if constexpr (EPI == kGatedMean) {
         const uint32_t d0 = tl.rt * a.per, st = r / a.per, d = d0 + (r - st * a.per);
         row = (st < a.hc ? st : a.hc - 1) * a.dim + (d < a.dim ? d : a.dim - 1);
       } else {
-        row = min(tl.rt * kM + r, a.rows - 1u);
+        row = min(tl.rt * kM + r, rows - 1u);
       }
       const uint32_t base15 = (uint32_t) ((uintptr_t) (w + (uint64_t) row * row_bytes) & 15u);
       for (uint32_t it = (team - s0) % kTeams; it < steps; it += kTeams) {
@@ -586,7 +596,7 @@ __global__ void __launch_bounds__(kThreads, 1) mm_tc_kernel(const Args a, const 
             asm volatile(
                 "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
                     smem_addr(raw) + slot * (kM * kSlot)),
-                "l"(&maps.raw), "r"((kb * kRawBytes<T>) & ~15u), "r"(tl.rt * kM), "r"(mat), "r"(smem_addr(&sh.full_raw[slot]))
+                "l"(tl.second ? &maps.raw1 : &maps.raw), "r"((kb * kRawBytes<T>) & ~15u), "r"(tl.rt * kM), "r"(mat), "r"(smem_addr(&sh.full_raw[slot]))
                 : "memory");
           }
           __syncwarp();
@@ -597,7 +607,8 @@ __global__ void __launch_bounds__(kThreads, 1) mm_tc_kernel(const Args a, const 
     }
     for (uint32_t t = blockIdx.x; t < tiles && ok && !a.raw_map; t += gridDim.x) {
       const Tile tl = tile_at(a, first, t, m_at, lane);
-      const uint8_t* w = a.wt ? a.wt[tl.m] : a.w;
+      const uint8_t* w = a.wt ? a.wt[tl.m] : tl.second ? a.w1 : a.w;
+      const uint32_t rows = tl.second ? a.rows1 : a.rows;
       for (uint32_t kb = 0; kb < kblocks; kb++, rb++) {
         const uint32_t slot = rb % kRawStages<T>;
         if (rb >= kRawStages<T> && !bar_wait_soon(&sh.empty_raw[slot], (rb / kRawStages<T> - 1u) & 1u)) {
@@ -613,7 +624,7 @@ __global__ void __launch_bounds__(kThreads, 1) mm_tc_kernel(const Args a, const 
           if (to % kSlot < lead + bytes)
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + to), "l"(from - lead) : "memory");
         };
-        if (EPI != kGatedMean && a.rows - row0 >= (uint32_t) kM && row_bytes < (1u << 24)) {
+        if (EPI != kGatedMean && rows - row0 >= (uint32_t) kM && row_bytes < (1u << 24)) {
           const uint8_t* from = w + (uint64_t) row0 * row_bytes + in_row;
           for (uint32_t r0 = 0; r0 < (uint32_t) kM; r0 += kTogether, from += kTogether * row_bytes) {
 #pragma unroll
@@ -632,7 +643,7 @@ __global__ void __launch_bounds__(kThreads, 1) mm_tc_kernel(const Args a, const 
                 const uint32_t d0 = tl.rt * a.per, st = r / a.per, d = d0 + (r - st * a.per);
                 row = (st < a.hc ? st : a.hc - 1) * a.dim + (d < a.dim ? d : a.dim - 1);
               } else {
-                row = min(row0 + r, a.rows - 1u);
+                row = min(row0 + r, rows - 1u);
               }
               copy(to, w + (uint64_t) row * row_bytes + in_row + to % kSlot);
             }
@@ -747,7 +758,9 @@ __global__ void __launch_bounds__(kThreads, 1) mm_tc_kernel(const Args a, const 
     for (uint32_t t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
       const Tile tl = tile_at(a, first, t, m_at, lane);
       const uint32_t row0 = tl.rt * kM;
-      const bool live = row0 + row < a.rows;
+      const bool live = row0 + row < (tl.second ? a.rows1 : a.rows);
+      const uint32_t ys = tl.second ? a.ys1 : a.ys;
+      const float scale = tl.second ? a.scale1 : a.scale;
       const uint32_t uses = tl.n > (uint32_t) kN ? 2u : 1u;
       for (uint32_t u = 0; u < uses; u++, acc++) {  // the tile's accumulators
         const uint32_t buf = acc & 1u;
@@ -764,7 +777,7 @@ __global__ void __launch_bounds__(kThreads, 1) mm_tc_kernel(const Args a, const 
         }
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        float* const y0 = a.y + (a.wt ? a.yoff[tl.m] : 0u) + (uint64_t) tl.c0 * a.ys + row0 + row;
+        float* const y0 = (tl.second ? a.y1 : a.y) + (a.wt ? a.yoff[tl.m] : 0u) + (uint64_t) tl.c0 * ys + row0 + row;
 #pragma unroll 1
         for (uint32_t c = 0; c < (uint32_t) kN; c += kChunkTok) {
           // column c of the accumulator is token 2 c + u, or (both halves in one) token 2 (c % 64) + c / 64
@@ -805,18 +818,18 @@ __global__ void __launch_bounds__(kThreads, 1) mm_tc_kernel(const Args a, const 
             }
             asm volatile("bar.sync 2, %0;" ::"n"(kEpiWarps * kWarp) : "memory");  // (the next tokens reuse ex)
           } else if (live) {
-            float* y = y0 + (uint64_t) t0 * a.ys;
+            float* y = y0 + (uint64_t) t0 * ys;
 #pragma unroll
             for (uint32_t i = 0; i < kChunkTok; i++) {
               if (t0 + 2u * i < tl.n) {
-                float v = mul_rn(__uint_as_float(r[i]), a.scale);
+                float v = mul_rn(__uint_as_float(r[i]), scale);
                 if constexpr (EPI == kSilu) {
                   v = siluf(v);
                   x16_store(a.x16_out, a.overflow, tl.c0 + t0 + 2u * i, row0 + row, a.rows, v);
                 }
                 *y = v;
               }
-              y += 2u * (uint64_t) a.ys;
+              y += 2u * (uint64_t) ys;
             }
           }
         }
@@ -897,6 +910,7 @@ bool launch(Args a, uint32_t n_mat, uint32_t max_cnt, cudaStream_t s) {
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     return false;
   a.row_tiles = EPI == kGatedMean ? parts_of(a.dim, a.per) : parts_of(a.rows, kM);
+  a.row_tiles1 = a.w1 ? parts_of(a.rows1, kM) : 0u;
   static bool sized[64] = {};  // (one record a template instance, one flag a device)
   if (!allow_dynamic_smem(mm_tc_kernel<T, EPI>, kBytes, sized)) return false;
   alignas(64) Maps maps;
@@ -904,7 +918,9 @@ bool launch(Args a, uint32_t n_mat, uint32_t max_cnt, cudaStream_t s) {
   const uint64_t row_bytes = (uint64_t) (a.cols / Fmt<T>::values) * Fmt<T>::bytes;
   if (EPI != kGatedMean && (!a.wt || (a.base && a.bytes >= a.rows * row_bytes)))
     a.raw_map = a.wt ? raw_map(a.base, row_bytes, a.rows, a.n_base, a.bytes, kWindow<T>, &maps.raw)
-                     : raw_map(a.w, row_bytes, a.rows, 1, a.rows * row_bytes, kWindow<T>, &maps.raw);
+                     : raw_map(a.w, row_bytes, a.rows, 1, a.rows * row_bytes, kWindow<T>, &maps.raw) &&
+                           (!a.w1 || raw_map(a.w1, row_bytes, a.rows1, 1, a.rows1 * row_bytes, kWindow<T>, &maps.raw1));
+  const uint64_t row_tiles = (uint64_t) a.row_tiles + a.row_tiles1;  // (of one matrix or two)
   if (a.wt) {
     a.span = max_cnt < kMaxSpan ? whole16(max_cnt) : kMaxSpan;
     // (where in x16 a matrix's tokens lie is on the device: the maps reach as far as its 32-bit offsets do, and a box has no
@@ -928,12 +944,12 @@ bool launch(Args a, uint32_t n_mat, uint32_t max_cnt, cudaStream_t s) {
   constexpr uint32_t kMost = EPI == kGatedMean ? 192u : kMaxSpan;  // (two slots of the token ring)
   for (uint32_t cols = parts_of(a.n, kMost); cols <= parts_of(a.n, MM_TILE); cols++) {
     const uint32_t tok = whole16(parts_of(a.n, cols)), step = 60u + 9u * tok / 4u;
-    const uint64_t rounds = ((uint64_t) a.row_tiles * parts_of(a.n, tok) + (uint32_t) sms - 1u) / (uint32_t) sms;
+    const uint64_t rounds = (row_tiles * parts_of(a.n, tok) + (uint32_t) sms - 1u) / (uint32_t) sms;
     const uint64_t cost = rounds * (step > 320u ? step : 320u);
     if (!best || cost < best) best = cost, a.span = tok;
   }
   a.use_tma = x16_map(a.x16, parts_of(a.n, MM_TILE), a.xts, a.span, &maps.map[0]) ? 1u : 0u, a.n_mat = 1;
-  const uint64_t tiles = (uint64_t) a.row_tiles * parts_of(a.n, a.span);
+  const uint64_t tiles = row_tiles * parts_of(a.n, a.span);
   if (tiles > 0xFFFFFFFFull) return false;
   const dim3 grid((unsigned) (tiles < (uint64_t) sms ? tiles : (uint64_t) sms));
   return launch_dependent(mm_tc_kernel<T, EPI>, grid, dim3(kThreads), kBytes, s, a, maps) == cudaSuccess;
@@ -962,6 +978,16 @@ bool run(uint32_t type, const void* w, uint32_t rows, uint32_t cols, const void*
   Args a{};
   a.w = (const uint8_t*) w, a.x16 = (const __half*) x16, a.y = y, a.rows = rows, a.cols = cols, a.n = n, a.xts = cols;
   a.ys = ys, a.scale = scale, a.early = early ? 1u : 0u;
+  return run_with<kStore>(type, a, stream);
+}
+
+// two matrices of a type and width over the same tokens in one launch, each the bits `run` gives it alone; both have been checked
+bool run_pair(uint32_t type, const void* w0, uint32_t rows0, float* y0, uint32_t ys0, float s0, const void* w1, uint32_t rows1, float* y1,
+              uint32_t ys1, float s1, uint32_t cols, const void* x16, uint32_t n, void* stream, bool early) {
+  Args a{};
+  a.w = (const uint8_t*) w0, a.x16 = (const __half*) x16, a.y = y0, a.rows = rows0, a.cols = cols, a.n = n, a.xts = cols;
+  a.ys = ys0, a.scale = s0, a.early = early ? 1u : 0u;
+  a.w1 = (const uint8_t*) w1, a.y1 = y1, a.rows1 = rows1, a.ys1 = ys1, a.scale1 = s1;
   return run_with<kStore>(type, a, stream);
 }
 
@@ -1031,8 +1057,7 @@ extern "C" bool mm_run2(uint32_t type, const void* w0, uint32_t rows0, float* y0
   if (!w0 || !w1 || !y0 || !y1 || !x16 || !n || n > MM_MAX_TOKENS || !mm_tc::shape_ok(type, rows0, cols) ||
       !mm_tc::shape_ok(type, rows1, cols) || (n > 1 && (ys0 < rows0 || ys1 < rows1)) || ((uintptr_t) x16 & 15u))
     return false;  // (decided for both before either is queued)
-  return mm_tc::run(type, w0, rows0, cols, x16, n, y0, ys0, 1.0f, stream) &&
-         mm_tc::run(type, w1, rows1, cols, x16, n, y1, ys1, 1.0f, stream);
+  return mm_tc::run_pair(type, w0, rows0, y0, ys0, 1.0f, w1, rows1, y1, ys1, 1.0f, cols, x16, n, stream, false);
 }
 
 extern "C" bool mm_tokens_scaled(uint32_t type, const void* w0, uint32_t rows0, float* y0, uint32_t ys0, float s0,
@@ -1047,8 +1072,10 @@ extern "C" bool mm_tokens_scaled(uint32_t type, const void* w0, uint32_t rows0, 
     const uint32_t c = n - t0 < MM_MAX_TOKENS ? n - t0 : MM_MAX_TOKENS;
     const bool convert = !(ready && n <= MM_MAX_TOKENS);
     if (convert && !mm_x16(x + (uint64_t) t0 * xs, xs, c, cols, x16, overflow, stream)) return false;
-    if (!mm_tc::run(type, w0, rows0, cols, x16, c, y0 + (uint64_t) t0 * ys0, ys0, s0, stream, convert)) return false;
-    if (w1 && !mm_tc::run(type, w1, rows1, cols, x16, c, y1 + (uint64_t) t0 * ys1, ys1, s1, stream)) return false;
+    float* const to0 = y0 + (uint64_t) t0 * ys0;
+    if (w1 ? !mm_tc::run_pair(type, w0, rows0, to0, ys0, s0, w1, rows1, y1 + (uint64_t) t0 * ys1, ys1, s1, cols, x16, c, stream, convert)
+           : !mm_tc::run(type, w0, rows0, cols, x16, c, to0, ys0, s0, stream, convert))
+      return false;
   }
   return true;
 }

@@ -99,3 +99,27 @@ def test_group_of_many(lib, dev):
     got = y.cpu().numpy()
     assert same_bits(got[cnt == 1], np.repeat(one.cpu().numpy(), int(cnt.sum()), 0)) and (got[cnt == 0] == -3.0).all()
     assert lib.mm_status() == 0
+
+
+@pytest.mark.parametrize("name,rows0,rows1,cols,off", [("Q4_K", 256, 256, 512, 0), ("Q4_K", 144, 400, 512, 0), ("Q8_0", 16, 272, 384, 0),
+                                                       ("Q6_K", 144, 16, 256, 0), ("Q4_0", 144, 144, 512, 2)])
+def test_two_matrices(lib, dev, name, rows0, rows1, cols, off):
+    """two matrices in one launch (both, one or none of them on 16 bytes): each the bits mm_run gives it alone"""
+    tid = TYPES[name]
+    rng = synth.rng_for(65, tid)
+    w0, w1 = synth.random_tensor(tid, rows0, cols, rng), synth.random_tensor(tid, rows1, cols, rng)
+    d0 = to_dev(w0, dev)
+    mem = torch.zeros(w1.size + 64, dtype=torch.uint8, device=dev)
+    mem[off:off + w1.size] = to_dev(w1.reshape(-1).view(np.uint8), dev)
+    lib.mm_status()
+    for n in (1, 40, 129, 300):
+        xb = _x16(lib, dev, rng.standard_normal((n, cols)).astype(np.float32), cols)
+        a, b = torch.empty((n, rows0), device=dev), torch.empty((n, rows1), device=dev)
+        y0, y1 = torch.full((n, rows0 + 3), -7.0, device=dev), torch.full((n, rows1 + 5), -7.0, device=dev)
+        assert lib.mm_run(tid, ptr(d0), rows0, cols, ptr(xb), n, ptr(a), rows0, None)
+        assert lib.mm_run(tid, mem.data_ptr() + off, rows1, cols, ptr(xb), n, ptr(b), rows1, None)
+        assert lib.mm_run2(tid, ptr(d0), rows0, ptr(y0), rows0 + 3, mem.data_ptr() + off, rows1, ptr(y1), rows1 + 5, cols, ptr(xb), n, None)
+        sync()
+        assert same_bits(y0[:, :rows0].cpu().numpy(), a.cpu().numpy()) and same_bits(y1[:, :rows1].cpu().numpy(), b.cpu().numpy())
+        assert (y0[:, rows0:] == -7.0).all() and (y1[:, rows1:] == -7.0).all()
+    assert lib.mm_status() == 0
