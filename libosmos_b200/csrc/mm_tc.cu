@@ -82,9 +82,6 @@ __device__ __forceinline__ uint64_t tile_desc_sw64(uint32_t addr) {
 // instruction descriptor: D F32, A and B f16, both K-major, M = 128, N = n
 __device__ __forceinline__ uint32_t idesc(uint32_t n) { return (1u << 4) | (n >> 3) << 17 | (uint32_t) (kM >> 4) << 24; }
 
-__device__ __forceinline__ void bar_arrive_n(uint64_t* bar, uint32_t n) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(n) : "memory");
-}
 __device__ __forceinline__ void arrive_when_copied(uint64_t* bar) {
   asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_addr(bar)) : "memory");
 }
@@ -417,6 +414,28 @@ struct Shared {
 __host__ __device__ constexpr uint32_t whole16(uint32_t n) { return (n + 15u) & ~15u; }
 __host__ __device__ constexpr uint32_t parts_of(uint32_t n, uint32_t of) { return (n + of - 1u) / of; }
 
+// The steps a producer team walks of a tile of `steps`: those of its whole raw blocks. A row of an odd multiple of 128 values
+// ends in half a block of 256, which has a step for two of the four teams; the other two wait for it and hand it back all the
+// same. A wait on a raw slot names its phase by a parity, and so holds only for a team that has seen the phase before: a team
+// that left a block out could, three slots deep, take the phase before it for its own and decode bytes that had not landed.
+__host__ __device__ constexpr uint32_t walked(uint32_t steps, uint32_t steps_raw) { return parts_of(steps, steps_raw) * steps_raw; }
+// whether each team meets every phase, from the first, of every slot it uses: over rows of all lengths mod a block and enough tiles
+constexpr bool every_phase_seen(uint32_t slots, uint32_t steps_raw) {
+  for (uint32_t steps = 2; steps <= 4 * steps_raw; steps += 2) {
+    for (uint32_t team = 0; team < (uint32_t) kTeams; team++) {
+      uint32_t next[8] = {}, s0 = 0, rb0 = 0;  // next[slot]: the phase to be met next
+      for (uint32_t tile = 0; tile < 4 * slots; tile++, s0 += steps, rb0 += parts_of(steps, steps_raw)) {
+        for (uint32_t it = (team - s0) % (uint32_t) kTeams; it < walked(steps, steps_raw); it += (uint32_t) kTeams) {
+          const uint32_t rb = rb0 + it / steps_raw, slot = rb % slots, phase = rb / slots;
+          if (phase != next[slot]) return false;
+          next[slot] = phase + 1;
+        }
+      }
+    }
+  }
+  return true;
+}
+
 // Tile number t of the launch: tiles go matrix by matrix, row tile by row tile, a row tile's token tiles side by side (they
 // share the weights' bytes in L2). first[m]: matrix m's first tile; m: where the last search ended (a role's tiles only
 // go up). A matrix's tokens are dealt in equal whole tiles of 16.
@@ -537,12 +556,17 @@ __global__ void __launch_bounds__(kThreads, 1) mm_tc_kernel(const Args a, const 
         row = min(tl.rt * kM + r, rows - 1u);
       }
       const uint32_t base15 = (uint32_t) ((uintptr_t) (w + (uint64_t) row * row_bytes) & 15u);
-      for (uint32_t it = (team - s0) % kTeams; it < steps; it += kTeams) {
+      for (uint32_t it = (team - s0) % kTeams; it < walked(steps, kStepsRaw); it += kTeams) {
         const uint32_t s = s0 + it, stage = s % kSteps, unit = stage >> two, kb = it / kStepsRaw, sub = it % kStepsRaw, rb = rb0 + kb, slot = rb % kRawStages<T>;
+        const bool past = it >= steps;  // (no step of the row's: the block is waited for and handed back)
         if (!bar_wait_soon(&sh.full_raw[slot], (rb / kRawStages<T>) & 1u) ||
-            (s >= kSteps && !bar_wait_soon(&sh.empty[unit], (s / kSteps - 1u) & 1u))) {
+            (!past && s >= kSteps && !bar_wait_soon(&sh.empty[unit], (s / kSteps - 1u) & 1u))) {
           ok = false;
           break;
+        }
+        if (past) {
+          if (lane == 0) bar_arrive(&sh.empty_raw[slot]);
+          break;  // (the tile's last block)
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t off = slot * (kM * kSlot) + r * pitch + ((base15 + kb * kRawBytes<T>) & 15u);
@@ -557,8 +581,7 @@ __global__ void __launch_bounds__(kThreads, 1) mm_tc_kernel(const Args a, const 
         __syncwarp();
         if (lane == 0) {
           bar_arrive(&sh.full_a[unit]);
-          // (the raw block's last step arrives for those a row's end leaves out)
-          bar_arrive_n(&sh.empty_raw[slot], it == steps - 1u ? kStepsRaw - sub : 1u);
+          bar_arrive(&sh.empty_raw[slot]);
         }
       }
     }
@@ -904,6 +927,7 @@ template <uint32_t T, uint32_t EPI = kStore>
 bool launch(Args a, uint32_t n_mat, uint32_t max_cnt, cudaStream_t s) {
   constexpr int kBytes = (int) kSmem<T, EPI>;
   static_assert(kBytes + grid_smem_bytes<T>() + (int) sizeof(Shared) + 64 <= 227 * 1024, "a block's shared memory");
+  static_assert(every_phase_seen(kRawStages<T>, kRawK<T> / kStep), "a producer's wait on a raw slot");
   a.status = status_word();
   if (!a.status) return false;
   int sms = 0, dev = 0;

@@ -123,3 +123,38 @@ def test_two_matrices(lib, dev, name, rows0, rows1, cols, off):
         assert same_bits(y0[:, :rows0].cpu().numpy(), a.cpu().numpy()) and same_bits(y1[:, :rows1].cpu().numpy(), b.cpu().numpy())
         assert (y0[:, rows0:] == -7.0).all() and (y1[:, rows1:] == -7.0).all()
     assert lib.mm_status() == 0
+
+
+def _f16_weights_on(oracle, dev, tid, w, rows, cols):
+    """the weights as the product takes them, F16, as float64 on the device"""
+    with np.errstate(over="ignore"):
+        return torch.from_numpy(oracle.dequant(tid, w, rows * cols).reshape(rows, cols).astype(np.float16)).to(dev).to(torch.float64)
+
+
+# more tiles than a block takes at once (75 row tiles over the tokens' tiles on 148 SMs), so that every ring, parity and accumulator goes
+# on from one tile to the next. cols: 128, 384, 640 and 896 end a row in half a raw block - of Q5_1 in a ring of three such blocks, of
+# the others in one of four; 512 does not
+@pytest.mark.parametrize("name,cols", [("Q5_1", 128), ("Q5_1", 384), ("Q5_1", 640), ("Q5_1", 896), ("Q5_1", 512), ("MXFP4", 384), ("MXFP4", 512), ("Q4_0", 640),
+                                       ("NVFP4", 896), ("Q8_0", 384), ("Q4_K", 512), ("Q5_K", 256), ("Q6_K", 512), ("IQ3_XXS", 512)])
+def test_many_tiles_a_block(lib, dev, oracle, name, cols):
+    tid, rows = TYPES[name], 9600
+    rng = synth.rng_for(66, tid * 10000 + cols)
+    w = synth.random_tensor(tid, rows, cols, rng)
+    wd, w16 = to_dev(w, dev), _f16_weights_on(oracle, dev, tid, w, rows, cols)
+    lib.mm_status()
+    for n in (1000, 130, 97):
+        x = rng.standard_normal((n, cols)).astype(np.float32)
+        y = torch.full((n, rows), float("nan"), dtype=torch.float32, device=dev)
+        for _ in range(3):
+            y.fill_(float("nan"))
+            assert lib.mm_run(tid, ptr(wd), rows, cols, ptr(_x16(lib, dev, x, cols)), n, ptr(y), rows, None)
+            sync()
+            x16 = torch.from_numpy(x.astype(np.float16)).to(dev).to(torch.float64)
+            bound = (cols / 16 + 20) * 2.0 ** -24 * (x16.abs() @ w16.abs().T) + 1e-30  # (test_gpu_mm.py's)
+            assert bool(((y.to(torch.float64) - x16 @ w16.T).abs() <= bound).all()), n
+        one = torch.empty((1, rows), dtype=torch.float32, device=dev)
+        for t in (0, n // 2, n - 1):  # a token alone - a tile a block, for the most part: the bits it has among the others
+            assert lib.mm_run(tid, ptr(wd), rows, cols, ptr(_x16(lib, dev, x[t:t + 1], cols)), 1, ptr(one), rows, None)
+            sync()
+            assert same_bits(one.cpu().numpy()[0], y[t].cpu().numpy()), (n, t)
+    assert lib.mm_status() == 0
