@@ -123,7 +123,8 @@ bool mm_group(uint32_t type, const void *const *w, const int32_t *cnt, uint32_t 
               uint32_t cols, const void *x16, const uint32_t *xoff, uint32_t xts, float *y, const uint32_t *yoff,
               uint32_t ys, void *stream);
 /* Not in the reference: mm_group where every w[m] is one of the n_base matrices of one tensor, `bytes` apart from `base` on (an
-   expert tensor): known to the host, its rows can be read through a tensor map. base NULL: mm_group. */
+   expert tensor): known to the host, its rows can be read through a tensor map. base NULL: mm_group. A w[m] with tokens that
+   is not one of them raises mm_status's bit 1 where the map is used, and its rows of y are not valid. */
 bool mm_group_of(uint32_t type, const void *base, uint64_t bytes, uint32_t n_base, const void *const *w, const int32_t *cnt,
                  uint32_t n_mat, uint32_t max_cnt, uint32_t rows, uint32_t cols, const void *x16, const uint32_t *xoff,
                  uint32_t xts, float *y, const uint32_t *yoff, uint32_t ys, void *stream);
@@ -167,7 +168,8 @@ bool mm_mxfp4(const void *w, uint32_t rows, uint32_t cols, const void *packed, u
    CUTLASS's encoder */
 uint32_t mm_fp4_desc(uint32_t mx, uint32_t n, uint32_t sf_id);
 /* Not in the reference: the products' kernel never waits without a bound; reads and clears the current device's
-   record (synchronizes): bit 0 a wait ran out, the launch's outputs are not valid */
+   record (synchronizes): bit 0 a wait ran out, bit 1 mm_group_of met a matrix that is not one of its tensor's; the
+   launch's outputs are not valid */
 uint32_t mm_status(void);
 
 #ifdef __cplusplus

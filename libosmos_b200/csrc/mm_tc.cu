@@ -71,6 +71,7 @@ constexpr uint32_t kMaxSpan = 2 * kN;      // tokens a tile
 constexpr uint32_t kMaxMats = 768;        // matrices a launch: their first tiles are kept in shared memory
 
 __device__ uint32_t g_status;
+enum : uint32_t { kWaitRanOut = 1, kNotOfTensor = 2 };  // (mm_status's bits)
 
 // shared-memory matrix descriptor of one K = 16 sub-tile of tokens: x16's fragments as they lie - a token's 16 values 32 bytes - as
 // rows of 64 bytes, two tokens each, with the 64-byte swizzle; 8 rows are 512 bytes. A product takes the first 32 bytes of
@@ -607,7 +608,13 @@ __global__ void __launch_bounds__(kThreads, 1) mm_tc_kernel(const Args a, const 
     if (a.raw_map) {  // a copy a block: the second warp has nothing to do
       for (uint32_t t = blockIdx.x; t < tiles && ok && warp == (uint32_t) kFirstRaw; t += gridDim.x) {
         const Tile tl = tile_at(a, first, t, m_at, lane);
-        const uint32_t mat = a.wt ? (uint32_t) ((uint64_t) (a.wt[tl.m] - a.base) / a.bytes) : 0u;
+        uint32_t mat = 0;
+        if (a.wt) {
+          // (the pointers are the device's: one that is no matrix of the tensor would be another's rows, or rows of zeros)
+          const uint64_t at = (uint64_t) (a.wt[tl.m] - a.base), index = at / a.bytes;
+          if (index < a.n_base && index * a.bytes == at) mat = (uint32_t) index;
+          else if (lane == 0) atomicOr(a.status, kNotOfTensor);
+        }
         for (uint32_t kb = 0; kb < kblocks; kb++, rb++) {
           const uint32_t slot = rb % kRawStages<T>;
           if (rb >= kRawStages<T> && !bar_wait_soon(&sh.empty_raw[slot], (rb / kRawStages<T> - 1u) & 1u)) {
@@ -871,7 +878,7 @@ __global__ void __launch_bounds__(kThreads, 1) mm_tc_kernel(const Args a, const 
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
   }
-  if (tid == 0 && sh.fail) atomicOr(a.status, 1u);
+  if (tid == 0 && sh.fail) atomicOr(a.status, kWaitRanOut);
 }
 
 uint32_t* status_word() {

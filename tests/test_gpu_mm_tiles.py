@@ -158,3 +158,29 @@ def test_many_tiles_a_block(lib, dev, oracle, name, cols):
             sync()
             assert same_bits(one.cpu().numpy()[0], y[t].cpu().numpy()), (n, t)
     assert lib.mm_status() == 0
+
+
+def test_group_not_of_the_tensor(lib, dev):
+    """pointers that are no matrix of the tensor they are said to be of (one past the count given, one before the base, one inside a
+    matrix; all of them in the allocation): reported, the other matrices' results as ever, and no report without tokens"""
+    tid, rows, cols, n = TYPES["MXFP4"], 144, 512, 20
+    rng = synth.rng_for(67)
+    nb = synth.tensor_bytes(tid, rows, cols)
+    wd = to_dev(np.concatenate([synth.random_tensor(tid, rows, cols, rng).reshape(-1).view(np.uint8) for _ in range(4)]), dev)
+    xb = _x16(lib, dev, rng.standard_normal((n, cols)).astype(np.float32), cols)
+    want = torch.empty((n, rows), dtype=torch.float32, device=dev)
+    assert lib.mm_run(tid, wd.data_ptr() + nb, rows, cols, ptr(xb), n, ptr(want), rows, None)
+    lib.mm_status()
+    zeros, offs = to_dev(np.zeros(2, np.uint32), dev), to_dev(np.array([0, n * rows], np.uint32), dev)
+    for base, n_base, second, cnt, bits in ((0, 4, 3 * nb, n, 0), (0, 3, 3 * nb, n, 2), (0, 3, 3 * nb, 0, 0), (nb, 3, 0, n, 2),
+                                            (0, 4, 2 * nb + 272, n, 2)):
+        table = torch.tensor([wd.data_ptr() + nb, wd.data_ptr() + second], dtype=torch.int64, device=dev)
+        y = torch.full((2 * n, rows), -3.0, dtype=torch.float32, device=dev)
+        assert lib.mm_group_of(tid, wd.data_ptr() + base, nb, n_base, ptr(table), ptr(to_dev(np.array([n, cnt], np.int32), dev)), 2, n, rows, cols,
+                               ptr(xb), ptr(zeros), cols, ptr(y), ptr(offs), rows, None)
+        assert lib.mm_status() == bits and lib.mm_status() == 0
+        assert same_bits(y[:n].cpu().numpy(), want.cpu().numpy())
+        # by the pointers alone: any address is a matrix
+        assert lib.mm_group(tid, ptr(table), ptr(to_dev(np.array([n, cnt], np.int32), dev)), 2, n, rows, cols, ptr(xb), ptr(zeros), cols, ptr(y),
+                            ptr(offs), rows, None)
+        assert lib.mm_status() == 0
