@@ -1,7 +1,8 @@
 """GPU parity of the f16 product at the edges of its tiles and of its ways to bring operands: row tiles and token tiles of every
 shape (one accumulator, both, an odd number of 16-token tiles), matrices whose rows start on 16 bytes (tensor-map copies) and
 not (16-byte copies), K of half a raw block, tokens that start inside a tile of the grouped x16, more matrices than a launch
-takes, and an expert tensor by its base. Bounds and the oracle as in test_gpu_mm.py."""
+takes, an expert tensor by its base, many tiles a block, and the product beside its own tokens' conversion. Bounds and the
+oracle as in test_gpu_mm.py."""
 import numpy as np
 import pytest
 import torch
@@ -184,3 +185,97 @@ def test_group_not_of_the_tensor(lib, dev):
         assert lib.mm_group(tid, ptr(table), ptr(to_dev(np.array([n, cnt], np.int32), dev)), 2, n, rows, cols, ptr(xb), ptr(zeros), cols, ptr(y),
                             ptr(offs), rows, None)
         assert lib.mm_status() == 0
+
+
+@pytest.mark.parametrize("capture", [False, True])
+def test_mm_tokens_queued(lib, dev, capture):
+    """the product starts while the conversion of its own tokens runs: calls in a row through one x16 (NaN before the first) without
+    a wait between, each with another x - a large conversion, a small one, more tokens than one x16 holds, the one before's x16
+    again (`ready`), one matrix and two: every output the bits of mm_x16, a wait, mm_run"""
+    tid, rows, rows1, cols = TYPES["Q4_K"], 1040, 144, 4096
+    rng = synth.rng_for(68)
+    d0, d1 = (to_dev(synth.random_tensor(tid, r, cols, rng), dev) for r in (rows, rows1))
+    calls = [(2048, False, False), (33, True, False), (2048 + 37, False, False), (200, True, False), (200, False, True), (2048 + 300, True, False),
+             (2048, True, False), (1, False, False)]
+    gen = torch.Generator(device=dev)
+    gen.manual_seed(68)
+    xs, outs, want = [], [], []
+    for n, two, ready in calls:
+        xs.append(xs[-1] if ready else torch.randn((n, cols), generator=gen, device=dev))
+        outs.append([torch.empty((n, r), device=dev) for r in ((rows, rows1) if two else (rows,))])
+        want.append([torch.empty_like(o) for o in outs[-1]])
+        for t in range(0, n, 2048):
+            c = min(2048, n - t)
+            xb = _x16(lib, dev, xs[-1][t:t + c].cpu().numpy(), cols)
+            for o, d, r in zip(want[-1], (d0, d1), (rows, rows1)):
+                assert lib.mm_run(tid, ptr(d), r, cols, ptr(xb), c, ptr(o) + 4 * t * r, r, None)
+            sync()
+    x16 = torch.empty(2048 * cols, dtype=torch.float16, device=dev)
+    flag = torch.zeros(1, dtype=torch.int32, device=dev)
+    lib.mm_status()
+
+    def queue(stream):
+        for (n, two, ready), x, o in zip(calls, xs, outs):
+            assert lib.mm_tokens(tid, ptr(d0), rows, ptr(o[0]), rows, ptr(d1) if two else None, rows1 if two else 0, ptr(o[1]) if two else None,
+                                 rows1 if two else 0, cols, ptr(x), cols, n, ptr(x16), ptr(flag), ready, stream)
+
+    side = torch.cuda.Stream(dev)
+    graph = torch.cuda.CUDAGraph()
+    if capture:
+        queue(None)  # (what a first call sets up is set up before the capture)
+        sync()
+        with torch.cuda.graph(graph, stream=side):
+            queue(side.cuda_stream)
+    for _ in range(5):
+        x16.fill_(float("nan"))
+        for o in outs:
+            for a in o:
+                a.fill_(float("nan"))
+        sync()
+        graph.replay() if capture else queue(None)
+        sync()
+        for o, w in zip(outs, want):
+            for a, b in zip(o, w):
+                assert torch.equal(a.view(torch.int32), b.view(torch.int32))
+    assert lib.mm_status() == 0 and int(flag.item()) == 0
+
+
+@pytest.mark.parametrize("name,cols,most", [("MXFP4", 512, 260), ("MXFP4", 512, 128), ("MXFP4", 384, 260), ("Q5_1", 384, 260), ("Q5_1", 640, 100),
+                                            ("Q4_0", 640, 260), ("Q8_0", 384, 200), ("Q4_K", 512, 260), ("IQ1_M", 256, 128)])
+def test_group_of_mixed_counts(lib, dev, name, cols, most):
+    """an expert tensor's matrices, four row tiles each, some 150 entries of no tokens to `most`: tiles of one accumulator and of both
+    in turn in a block, a token slot whose size changes from tile to tile, and units of one step or (up to 128 tokens) two; by the
+    pointers and by the tensor: the bits mm_run gives"""
+    tid, rows, n_mat, n_w = TYPES[name], 400, 150, 6
+    rng = synth.rng_for(69, tid * 10000 + cols + most)
+    nb = synth.tensor_bytes(tid, rows, cols)
+    wd = to_dev(np.concatenate([synth.random_tensor(tid, rows, cols, rng).reshape(-1).view(np.uint8) for _ in range(n_w)]), dev)
+    cnt = rng.choice(np.array([0, 1, 5, 16, 17, 48, 100, 128, 129, 144, 200, 255, 256, 260]), n_mat).astype(np.int32)
+    cnt = np.where(cnt > most, cnt % most, cnt).astype(np.int32)
+    cnt[:3] = most, 1, most
+    which = rng.integers(0, n_w, n_mat)
+    slots = (cnt + 15) // 16 * 16
+    xoff = (np.cumsum(slots) - slots) * cols
+    yoff = (np.cumsum(cnt) - cnt) * rows
+    total = int(slots.sum())
+    gen = torch.Generator(device=dev)
+    gen.manual_seed(69)
+    x = torch.randn((total, cols), generator=gen, device=dev)  # (a slot a row; the slots past an entry's tokens hold something too)
+    x16, flag = torch.empty(total * cols, dtype=torch.float16, device=dev), torch.zeros(1, dtype=torch.int32, device=dev)
+    assert lib.mm_x16_rows(ptr(x), cols, ptr(to_dev(np.arange(total, dtype=np.int32), dev)), total, cols, ptr(x16), ptr(flag), None)
+    want = torch.empty((int(cnt.sum()), rows), dtype=torch.float32, device=dev)
+    lib.mm_status()
+    for m in range(n_mat):
+        if cnt[m]:
+            assert lib.mm_run(tid, wd.data_ptr() + int(which[m]) * nb, rows, cols, ptr(x16) + 2 * int(xoff[m]), int(cnt[m]), ptr(want) + 4 * int(yoff[m]),
+                              rows, None)
+    table = torch.tensor([wd.data_ptr() + int(i) * nb for i in which], dtype=torch.int64, device=dev)
+    args = [to_dev(a.astype(t), dev) for a, t in ((cnt, np.int32), (xoff, np.uint32), (yoff, np.uint32))]
+    y = torch.empty_like(want)
+    for base in ((0, 0, 0), (wd.data_ptr(), nb, n_w)):
+        for _ in range(3):
+            y.fill_(float("nan"))
+            assert lib.mm_group_of(tid, *base, ptr(table), ptr(args[0]), n_mat, most, rows, cols, ptr(x16), ptr(args[1]), cols, ptr(y), ptr(args[2]), rows, None)
+            sync()
+            assert torch.equal(y.view(torch.int32), want.view(torch.int32))
+    assert lib.mm_status() == 0
