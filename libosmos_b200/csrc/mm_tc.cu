@@ -298,6 +298,123 @@ __device__ __forceinline__ void q6_step(uint32_t at, uint32_t sub, float d, cons
   }
 }
 
+// The other types (all but NVFP4 and MXFP8, whose codes are no integers): a step's bytes as words in registers, taken apart by
+// decode.cuh's field readers - a sub-block's fields once, not once a chunk - and the codes to F16 as above, eight of them (c) to four
+// pairs. Chunk by chunk out of shared memory these were bound by its passes (every byte, half and word of 32 rows meets four to a bank)
+// and by the integers' conversions, and a tile's weights decode once a 256 tokens: 17408 x 5120 at 2048 tokens Q3_K 936 -> 400 us, Q5_1
+// 655 -> 378, NVFP4 (its own way below) 625 -> 359, IQ4_XS 612 -> 456, IQ3_XXS 580 -> 457, IQ2_XXS 580 -> 431, Q2_K 563 -> 384, IQ1_M 542
+// -> 403 (decoded into shared memory once a 512 tokens they took 488 to 534); 4096 x 4096 at 64 tokens 37-71 -> 23-35.
+template <uint32_t T>
+__device__ __forceinline__ void chunk_halves(const Chunk& c, uint32_t* r) {
+  uint32_t lo = (uint32_t) c.lo, hi = (uint32_t) c.hi;
+  float scale = c.d, plus;
+  if constexpr (T == QTYPE_Q5_1) {
+    plus = c.e;
+  } else if constexpr (T == QTYPE_Q2_K) {
+    scale = mul_rn(c.d, (float) c.s), plus = -mul_rn(c.e, (float) c.m);
+  } else if constexpr (T == QTYPE_IQ1_S || T == QTYPE_IQ1_M) {  // -1, 0, 1 as 0, 1, 2; (d (2 s + 1)) (grid +- 1/8), exact
+    scale = mul_rn(c.d, (float) (2 * c.s + 1)), plus = mul_rn(scale, c.m < 0 ? -1.125f : -0.875f);
+    lo = (lo ^ kTops) - 0x7F7F7F7Fu, hi = (hi ^ kTops) - 0x7F7F7F7Fu;
+  } else {  // a signed byte as it and 128
+    if constexpr (T == QTYPE_Q3_K || T == QTYPE_IQ4_XS) scale = mul_rn(c.d, (float) c.s);
+    else if constexpr (T == QTYPE_IQ3_XXS) scale = mul_rn(mul_rn(c.d, 0.5f + (float) c.s), 0.5f);
+    else if constexpr (T == QTYPE_IQ2_XXS || T == QTYPE_IQ2_XS || T == QTYPE_IQ2_S) scale = mul_rn(mul_rn(c.d, 0.5f + (float) c.s), 0.25f);
+    plus = mul_rn(scale, -128.0f), lo ^= kTops, hi ^= kTops;
+  }
+  const Affine a(scale, plus);
+  a.bytes(lo, r[0], r[1]), a.bytes(hi, r[2], r[3]);
+}
+// The words of a row's block that hold step `sub`'s fields, each field where step 0's lies, so that the readers' offsets are known
+// when compiled whatever the step is. (Four copies of the code, a step each - the four teams are on the four steps at once, and their
+// instructions do not fit: IQ3_XXS 829 us where this takes 457.)
+template <uint32_t T> constexpr int kFieldWords = (Fmt<T>::values == 32 ? 2 * Fmt<T>::bytes : Fmt<T>::bytes) / 4 + 2;
+template <uint32_t T>
+__device__ __forceinline__ void load_fields(const uint8_t* p, uint32_t sub, WordWindow<kFieldWords<T>, 0>& rd) {
+  const uint32_t at = smem_addr(p);
+  auto words = [&](int first, int n, uint32_t from, uint32_t shift) {  // words first .. first + n - 1, `from` bytes on
+    const uint8_t* const src = p + from;
+    const uint32_t lead = (at + from) & 3u;
+    const uint32_t* const al = (const uint32_t*) (src - lead);
+#pragma unroll
+    for (int i = first; i < first + n; i++) rd.w[i] = __funnelshift_r(al[i], al[i + 1], 8u * lead) >> shift;
+  };
+  auto scale = [&]() { rd.w[0] = (rd.w[0] & 0xFFFF0000u) | lds_half(at); };
+  if constexpr (T == QTYPE_IQ2_XXS) {
+    words(0, 5, 16u * sub, 0), scale();
+  } else if constexpr (T == QTYPE_IQ2_XS) {
+    words(0, 5, 16u * sub, 0), scale(), rd.w[16] = lds_half(at + 66u + 2u * sub) << 16;
+  } else if constexpr (T == QTYPE_IQ3_XXS) {
+    words(0, 5, 16u * sub, 0), scale(), words(16, 3, 8u * sub, 0);
+  } else if constexpr (T == QTYPE_IQ2_S) {
+    words(0, 3, 8u * sub, 0), scale(), words(8, 3, 8u * sub, 0), rd.w[16] = lds_half(at + 66u + 2u * sub) << 16, rd.w[18] = lds_half(at + 74u + 2u * sub) << 16;
+  } else if constexpr (T == QTYPE_IQ1_S) {
+    words(0, 3, 8u * sub, 0), scale(), words(8, 2, 4u * sub, 0);
+  } else if constexpr (T == QTYPE_IQ1_M) {
+    words(0, 2, 8u * sub, 0), words(8, 1, 4u * sub, 0), words(12, 2, 0, 0);
+  } else if constexpr (T == QTYPE_IQ4_XS) {
+    rd.w[0] = lds_half(at) | (lds_half(at + 2u) >> (4u * sub)) << 16, rd.w[1] = lds8(at + 4u + sub), words(2, 8, 32u * sub, 0);
+  } else if constexpr (T == QTYPE_Q2_K) {
+    words(0, 1, 4u * sub, 0), words(4, 8, 32u * (sub >> 1), 4u * (sub & 1u)), words(20, 1, 0, 0);
+  } else if constexpr (T == QTYPE_Q3_K) {
+    words(0, 8, 0, 2u * sub), words(8, 8, 32u * (sub >> 1), 4u * (sub & 1u));
+    words(24, 1, 4u * (sub & 1u), 4u * (sub >> 1)), words(26, 1, 0, 2u * sub), words(27, 1, 0, 0);
+  } else {  // a block or two of the step's own
+    words(0, kFieldWords<T> - 1, sub * (kStep / Fmt<T>::values) * Fmt<T>::bytes, 0);
+  }
+}
+template <class Put>
+__device__ __forceinline__ void nvfp4_step(const uint8_t* p, uint32_t sub, const Put& put) {
+  WordWindow<kFieldWords<QTYPE_NVFP4>, 0> rd;
+  load_fields<QTYPE_NVFP4>(p, sub, rd);
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    // a UE4M3 byte's magnitude in an F16's exponent and mantissa is it times 2^-8, and the byte 0x7F is zero; an E2M1 code by an
+    // F16 scale: at most six bits from 2^-10 to 2880, so every product here is exact
+    const uint32_t c = rd.u8(q), h = c == 0x7Fu ? 0u : (c & 0x7Fu) << 7, h2 = h | h << 16;
+    const __half2 f = __hmul2_rn(*(const __half2*) &h2, __float2half2_rn(256.0f)), one = __float2half2_rn(16384.0f);
+    uint32_t r[8];
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      const uint32_t w = rd.u32(4 + 8 * q + 4 * k);
+      e2m1_halves(((w << 1) & 0x0E0E0E0Eu) | ((w << 4) & kTops), one, r[2 * k], r[2 * k + 1]);
+      e2m1_halves(((w >> 3) & 0x0E0E0E0Eu) | (w & kTops), one, r[4 + 2 * k], r[5 + 2 * k]);
+    }
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      const __half2 v = __hmul2_rn(*(const __half2*) &r[k], f);
+      r[k] = *(const uint32_t*) &v;
+    }
+    put((uint32_t) q, r);
+  }
+}
+// false: an odd scale, nothing put
+template <uint32_t T, class Put>
+__device__ __forceinline__ bool fields_step(const uint8_t* p, uint32_t sub, const Grids& g, const Put& put) {
+  WordWindow<kFieldWords<T>, 0> rd;
+  load_fields<T>(p, sub, rd);
+  constexpr bool kTwo = Fmt<T>::values == 32;  // (the step is two blocks; else two sub-blocks of one)
+  const PlainLuts lut{g};
+  Sub sb[2];
+  bool odd = false;
+#pragma unroll
+  for (int b = 0; b < 2; b++) {
+    sb[b] = sub_of<T>(rd, kTwo ? b * Fmt<T>::bytes : 0, kTwo ? 0 : b);
+    odd = odd || !(fabsf(sb[b].d) < __uint_as_float(0x7F800000u));
+    if constexpr (T == QTYPE_IQ1_M) sb[b].a = ((sub & 2u) ? sb[b].b : sb[b].a) >> (16u * (sub & 1u));  // (the step's scale word)
+  }
+  if (__any_sync(0xFFFFFFFFu, odd)) return false;
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    const int b = q >> 1;
+    uint32_t r[8];
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+      chunk_halves<T>(chunk_of<T>(rd, kTwo ? b * Fmt<T>::bytes : 0, kTwo ? 0 : b, 2 * (q & 1) + i, sb[b], lut), r + 4 * i);
+    put((uint32_t) q, r);
+  }
+  return true;
+}
+
 template <uint32_t T, class Put>
 __device__ __forceinline__ void decode_step(uint32_t at, const uint8_t* p, uint32_t sub, const Grids& g, const Put& put) {
   if constexpr (T == QTYPE_Q4_K || T == QTYPE_Q5_K) {
@@ -360,8 +477,12 @@ __device__ __forceinline__ void decode_step(uint32_t at, const uint8_t* p, uint3
     if (__any_sync(0xFFFFFFFFu, inf_or_nan(h))) return decode_step_any<T>(p, sub, g, put);
     if (sub & 1u) q6_step<true>(at, sub, half_value(h), put);
     else q6_step<false>(at, sub, half_value(h), put);
-  } else {
+  } else if constexpr (T == QTYPE_NVFP4) {
+    nvfp4_step(p, sub, put);
+  } else if constexpr (T == QTYPE_MXFP8) {
     decode_step_any<T>(p, sub, g, put);
+  } else {
+    if (!fields_step<T>(p, sub, g, put)) decode_step_any<T>(p, sub, g, put);
   }
 }
 

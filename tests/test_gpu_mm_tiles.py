@@ -10,7 +10,7 @@ import torch
 from helpers import ptr, same_bits, sync, to_dev
 from libosmos_b200 import synth
 from oracle.oracle import TYPES
-from test_gpu_mm import _exact, _within, _x16
+from test_gpu_mm import _exact, _f16_weights, _one_hot_product, _within, _x16
 
 pytestmark = pytest.mark.gpu
 
@@ -279,3 +279,42 @@ def test_group_of_mixed_counts(lib, dev, name, cols, most):
             sync()
             assert torch.equal(y.view(torch.int32), want.view(torch.int32))
     assert lib.mm_status() == 0
+
+
+# where the other types keep their F16 scales (IQ1_M's lies in four nibbles; NVFP4 and MXFP8 have none)
+_OTHER_SCALES = {"Q2_K": (80, 82), "Q3_K": (108,), "Q5_1": (0, 2), "IQ4_NL": (0,), "IQ4_XS": (0,), "IQ2_XXS": (0,), "IQ2_XS": (0,), "IQ2_S": (0,), "IQ3_XXS": (0,),
+                 "IQ1_S": (0,), "Q2_0": (0,), "IQ1_M": (), "NVFP4": (), "MXFP8": ()}
+
+
+@pytest.mark.parametrize("name", sorted(_OTHER_SCALES))
+@pytest.mark.parametrize("blocks", [1, 3])
+@pytest.mark.parametrize("off", [0, 2, 4, 14])
+def test_other_types_decoded(lib, dev, oracle, name, blocks, off):
+    """every weight as the product sees it, of the types that go through the field readers: every step of a 256-value block, a matrix
+    anywhere in a 16-byte piece (a row's blocks then start at any even place), scales of either sign, zero, subnormal and large -
+    and in two rows an infinite one, whose warps take the decoder chunk by chunk"""
+    tid, rows = TYPES[name], 144
+    values, nbytes = synth.BLOCK[tid]
+    cols = blocks * max(values, 128)
+    rng = synth.rng_for(70, tid, cols, off)
+    w = synth.random_tensor(tid, rows, cols, rng).reshape(rows, cols // values, nbytes).copy()
+    special = np.array([0x8000, 0x0000, 0x8001, 0x0001, 0x83FF, 0x03FF, 0xA000, 0xBC00, 0x3C00, 0x4B80, 0xCB80], np.uint16)  # (helpers.special_scales')
+    for at in _OTHER_SCALES[name]:
+        v = rng.choice(special, w.shape[:2])
+        pick = rng.random(w.shape[:2]) < 0.5
+        w[..., at], w[..., at + 1] = np.where(pick, v & 0xFF, w[..., at]), np.where(pick, v >> 8, w[..., at + 1])
+    if name == "NVFP4":
+        w[..., :4] = rng.integers(0, 256, w.shape[:2] + (4,))  # (every UE4M3 byte)
+    infinite = np.zeros(rows, bool)
+    if _OTHER_SCALES[name]:
+        infinite[[5, 100]] = True
+        w[infinite, -1, _OTHER_SCALES[name][0] + 1] = 0x7C
+        w[infinite, -1, _OTHER_SCALES[name][0]] = 0
+    w = w.reshape(-1)
+    with np.errstate(over="ignore", invalid="ignore"):
+        want = _f16_weights(oracle, tid, w, rows, cols)
+    assert np.isfinite(want[~infinite]).all()
+    pool = np.zeros(w.size + 32, np.uint8)
+    pool[off:off + w.size] = w
+    got = _one_hot_product(lib, dev, tid, ptr(to_dev(pool, dev)) + off, rows, cols)
+    assert np.array_equal(got[~infinite], want[~infinite])
