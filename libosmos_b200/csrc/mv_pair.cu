@@ -16,7 +16,7 @@
 // of the launch before the first slot and after the last) - and from three tokens on by x's reads. Measured, against a lane a
 // thread (mv_staged.cu): 49152 x 2048 at one token Q6_K 41.1 -> 29.5 us (2.8 TB/s), Q5_K 45.1 -> 33.4, Q4_K 39.6 -> 29.9, IQ4_XS
 // 42.1 -> 27.7; at eight tokens 80-85 -> 64-69; Q4_K 2048 x 7168 at five 22.6 -> 12.0; 1536 x 4096 MXFP4 matrices of 64 experts
-// at 64 picks 239 -> 111 us; without MXFP4's table of pairs 128 experts top-4, 32 tokens, 677 -> 626 us the layer.
+// at 64 picks 239 -> 111 us; without MXFP4's table of pairs 128 experts top-4, 32 tokens, 620 -> 510 us the layer.
 //
 // A warp owns a ring of slots; a slot holds the same run of up to 8 256-value stretches of its 2 RT rows, a bulk copy a
 // row of the 16-byte pieces around the row's bytes - so a row may start anywhere (Q6_K's 210-byte blocks: rows are
@@ -141,24 +141,25 @@ template <> struct Pair<QTYPE_MXFP4> {
   // An E2M1 code's bits as an F16's sign, exponent's low two bits and mantissa's top one are its value times 2^-14 (a subnormal
   // code is a subnormal F16); to F32 exactly, times 2^(e - 113): one rounding, of the value itself, as decode8's product. Past
   // e = 240 that factor is no F32: half the scale times the doubled code, as there. (Against a table of 256 pairs in shared memory, a copy
-  // a lane, which took most of its passes.)
+  // a lane, which took most of its passes; the scale has to be one addition and a shift for it: with its ranges told apart long rows were
+  // slower than the table, 8192 x 4096 at one token 11.2 -> 11.7 us, now 10.2; 49152 x 7168 92.5 -> 95.5, now 82.7.)
   __device__ __forceinline__ void values(uint32_t at, const Table&, uint64_t* v) const {
     const uint2 q = lds_8_bytes(at + off, sh);
     const uint32_t e = lds8(at + eoff);
     const bool large = e > 240u;
-    const float d = e8m0_value(e, large ? 128 : 113), one = large ? 32768.0f : 1.0f;
+    const float d = __uint_as_float((e + (large ? 0xFFFFFFFFu : 14u)) << 23);  // (either is a normal F32, whatever e)
 #pragma unroll
     for (int i = 0; i < 2; i++) {
       const uint32_t w = i ? q.y : q.x;
       const uint32_t lo = ((w << 1) & 0x0E0E0E0Eu) | ((w << 4) & kTops), hi = ((w >> 3) & 0x0E0E0E0Eu) | (w & kTops);
-      const uint32_t le = (lo << 8) & 0xFF00FF00u, lp = lo & 0xFF00FF00u, he = (hi << 8) & 0xFF00FF00u, hp = hi & 0xFF00FF00u;
+      const uint32_t le = __byte_perm(lo, 0, 0x2404), lp = lo & 0xFF00FF00u, he = __byte_perm(hi, 0, 0x2404), hp = hi & 0xFF00FF00u;
       v[4 * i] = pack2(low_half(le), low_half(he)), v[4 * i + 1] = pack2(low_half(lp), low_half(hp));
       v[4 * i + 2] = pack2(high_half(le), high_half(he)), v[4 * i + 3] = pack2(high_half(lp), high_half(hp));
     }
     const uint64_t dd = pack2(d, d);
     if (large) {
 #pragma unroll
-      for (int j = 0; j < kChunk; j++) v[j] = mul2(v[j], pack2(one, one));
+      for (int j = 0; j < kChunk; j++) v[j] = mul2(v[j], pack2(32768.0f, 32768.0f));
     }
 #pragma unroll
     for (int j = 0; j < kChunk; j++) v[j] = mul2(dd, v[j]);

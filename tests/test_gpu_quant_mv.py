@@ -197,6 +197,43 @@ def test_mv_special_scales(lib, dev, oracle, name, cols, rows, infinite):
     assert lib.mv_status() == 0
 
 
+def test_mv_mxfp4_every_exponent(lib, dev, oracle):
+    """every exponent (0 to 255: subnormal values, the largest F32s and past them) with every code, a value a row at every place of
+    the row in turn, by rows and grouped: the oracle's bits"""
+    tid, rows, cols = TYPES["MXFP4"], 256 * 16, 256
+    blocks = np.zeros((rows, cols // 32, 17), np.uint8)
+    blocks[:, :, 0] = 120
+    r = np.arange(rows)
+    at = (r * 37 + r // 256) % cols
+    blk, j = at // 32, at % 32
+    blocks[r, blk, 0] = r // 16
+    blocks[r, blk, 1 + j % 16] = np.where(j < 16, r % 16, (r % 16) << 4)
+    w = blocks.reshape(-1)
+    x = (synth.rng_for(71).uniform(0.5, 1.0, (8, cols)) * 2.0 ** -3).astype(np.float32)
+    want = oracle.mv_rows(tid, w, rows, cols, x)
+    finite = want[np.isfinite(want)]
+    assert np.isinf(want).any() and not np.isnan(want).any() and np.abs(finite).max() > 2.0 ** 124 and np.abs(finite[finite != 0]).min() < 2.0 ** -126
+    wd, xd = to_dev(w, dev), to_dev(x, dev)
+    lib.mv_status()
+    for n in (1, 2, 3, 5, 8):
+        y = torch.full((n, rows), -3.0, dtype=torch.float32, device=dev)
+        assert lib.mv_run(tid, ptr(wd), rows, cols, ptr(xd), n, ptr(y), None)
+        sync()
+        assert same_bits(y.cpu().numpy(), want[:n])
+    few = 512  # (the same rows as eight matrices, one to eight tokens each)
+    table = pointer_table(wd, [m * (w.size // 8) for m in range(8)], dev)
+    cnt = np.arange(1, 9, dtype=np.int32)
+    y = torch.full((int(cnt.sum()), few), -3.0, dtype=torch.float32, device=dev)
+    first = np.cumsum(cnt) - cnt
+    xs = np.concatenate([x[:c] for c in cnt])
+    assert lib.mv_group_tok(tid, ptr(table), ptr(to_dev(cnt, dev)), ptr(to_dev(first.astype(np.int32), dev)), 8, 8, few, cols, ptr(to_dev(xs, dev)), cols,
+                            ptr(y), few, None)
+    sync()
+    for m, (c, f) in enumerate(zip(cnt, first)):
+        assert same_bits(y[f:f + c].cpu().numpy(), want[:c, m * few:(m + 1) * few])
+    assert lib.mv_status() == 0
+
+
 @pytest.mark.parametrize("name", PAIRED)
 @pytest.mark.parametrize("cols,rows", [(768, 37), (2560, 130)])
 def test_mv_paired_lanes_grouped(lib, dev, oracle, name, cols, rows):
