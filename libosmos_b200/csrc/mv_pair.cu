@@ -595,9 +595,9 @@ int launch(const Request& r, const Device* dev, cudaStream_t s) {
   if constexpr (GROUP) {
     // an entry's rows over a few blocks, about four units a warp each and at most eight - more, down to a unit a warp, where
     // the entries are too few for three blocks an SM (one token's four MXFP4 experts of 1536 x 4096, the
-    // layer: 154 us with the first rule alone, 70 with this one; the staged kernel 162), but a quarter fewer or less where their warps
-    // take no more units each for it (68 experts top-3 of that shape, six tokens: 197 us a layer with 23 blocks an entry, whose
-    // warps take one unit or two, 173 with 12; staged 172)
+    // layer: 123 us with the first rule alone, 57 with this one; the staged kernel 162), but a quarter fewer or less where their warps
+    // take no more units each for it (128 experts top-4 of that shape, six tokens: 177 us a layer without this, whose
+    // warps take one unit or two, 163 with it; 68 experts top-3 159 and 155, staged 172)
     const uint32_t sms = (uint32_t) dev->sms;
     const uint32_t some = units / (4u * kWarps) > 8u ? 8u : units / (4u * kWarps), most = units / kWarps;
     const uint32_t want = (3u * sms + r.n_entries - 1) / r.n_entries, more = want < most ? want : most;
@@ -627,11 +627,13 @@ int by_shape(const Request& r, cudaStream_t s) {
   // tokens that kernel's packed row pairs use half the instructions (49152 x 2048: 27.1 us against 34.0, two tokens 37.4
   // against 39.4; three 72.8 against 45.7). A matrix of few rows leaves most warps here without any - two rows a warp, not
   // one - which at the token counts that kernel has an instance for is felt in the types that unpack little (1024 x 8192, one
-  // token: Q4_0 4.5 against 5.6, IQ4_XS 6.1 against 6.4, MXFP4 5.5 against 7.7, and with MXFP4's table to build 2048 x 2048 3.9
-  // against 4.1; Q4_K, Q5_K and Q6_K are faster here at every size).
+  // token: Q4_0 4.5 against 5.6, IQ4_XS 6.1 against 6.4, MXFP4 4.9 against 6.6; Q4_K, Q5_K and Q6_K are faster here at every
+  // size). MXFP4's line, that kernel against this: at one token 2048 x 4096 4.8 / 5.1, 2368 x 4096 5.1 / 5.1; at two and more 1536
+  // x 4096 5.2 / 5.7 (two), 7.1 / 7.4 (four), 10.9 / 10.9 (eight), 2048 x 4096 6.1 / 5.7, 8.4 / 7.5, 13.3 / 11.0, 2048 x 2048 4.0 / 4.0,
+  // 5.3 / 4.8, 7.9 / 6.7.
   if (T == QTYPE_Q4_0 || T == QTYPE_Q8_0 || T == QTYPE_IQ4_XS || T == QTYPE_MXFP4) {
     const bool whole = (r.n_tok & (r.n_tok - 1)) == 0;
-    const uint64_t few = (T == QTYPE_MXFP4 || T == QTYPE_Q8_0 ? 16ull : 8ull) * dev->sms;
+    const uint64_t few = (T == QTYPE_Q8_0 ? 16ull : T == QTYPE_MXFP4 ? (r.n_tok == 1 ? 16ull : 12ull) : 8ull) * dev->sms;
     if ((T == QTYPE_Q8_0 && r.n_tok <= 2) || (whole && r.rows <= few))
       if (const int st = mvs::try_launch(T, r, s)) return st;
   }

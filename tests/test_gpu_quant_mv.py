@@ -197,6 +197,24 @@ def test_mv_special_scales(lib, dev, oracle, name, cols, rows, infinite):
     assert lib.mv_status() == 0
 
 
+@pytest.mark.parametrize("off", [-1, 0, 1])
+@pytest.mark.parametrize("an_sm", [12, 16])
+def test_mv_mxfp4_either_side_of_its_line(lib, dev, oracle, an_sm, off):
+    """rows about the counts up to which the kernel with a lane a thread takes MXFP4 (12 an SM, one token 16): the oracle's bits on both"""
+    tid, cols = TYPES["MXFP4"], 512
+    rows = an_sm * torch.cuda.get_device_properties(dev).multi_processor_count + off
+    w, x = _mv_case(tid, rows, cols, 8, 22)
+    want = oracle.mv_rows(tid, w, rows, cols, x)
+    wd, xd = to_dev(w, dev), to_dev(x, dev)
+    lib.mv_status()
+    for n in (1, 2, 3, 4, 8):
+        y = torch.full((n, rows), -3.0, dtype=torch.float32, device=dev)
+        assert lib.mv_run(tid, ptr(wd), rows, cols, ptr(xd), n, ptr(y), None)
+        sync()
+        assert same_bits(y.cpu().numpy(), want[:n])
+    assert lib.mv_status() == 0
+
+
 def test_mv_mxfp4_every_exponent(lib, dev, oracle):
     """every exponent (0 to 255: subnormal values, the largest F32s and past them) with every code, a value a row at every place of
     the row in turn, by rows and grouped: the oracle's bits"""
