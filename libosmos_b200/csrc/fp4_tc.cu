@@ -98,7 +98,7 @@ struct Args {
 };
 
 struct Shared {
-  uint64_t full[kStages], empty[kStages], raw_full[kRawStages], raw_empty[kRawStages], acc_full;
+  uint64_t full[kStages], empty[kStages], raw_full[kRawStages], raw_empty[kRawStages], acc_full, drain;
   uint32_t tmem_base;
   int fail;
 };
@@ -118,13 +118,12 @@ __global__ void __launch_bounds__(kThreads, 1) fp4_tc_kernel(const Args a, const
   constexpr uint32_t kSfChunks = MX ? 2 : 4;  // chunks of 4 factors a stage: 256 values / (4 x 32) or / (4 x 16)
 
   if (tid == 0) {
-    // a stage is full when every producer has stored its part of A (an arrival each), every producer's scale-byte copies
-    // have landed (an arrival each, made by the copy engine) and the loader's tensor-map copy has delivered its bytes
-    // (the producers arrive a warp at a time: an arrival is an atomic on shared memory, and hundreds a stage would be the
-    // slowest thing in the kernel)
+    // a stage is full when every producer of its team has stored its part of A and of the scale factors, and the loader's
+    // tensor-map copy has delivered its bytes (the producers arrive a warp at a time: an arrival is an atomic on shared memory,
+    // and hundreds a stage would be the slowest thing in the kernel)
     for (int i = 0; i < kStages; i++) bar_init(&sh.full[i], kProdWarps + 1), bar_init(&sh.empty[i], 1);
     for (int i = 0; i < kRawStages; i++) bar_init(&sh.raw_full[i], 1), bar_init(&sh.raw_empty[i], kProdWarps);
-    bar_init(&sh.acc_full, 1);
+    bar_init(&sh.acc_full, 1), bar_init(&sh.drain, 1);
     sh.fail = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -159,6 +158,10 @@ __global__ void __launch_bounds__(kThreads, 1) fp4_tc_kernel(const Args a, const
     if (sf_t < n_mma && team < steps) read_sf(team);
     for (uint32_t it = team; it < steps; it += kTeams) {
       const uint32_t stage = it % kStages, use = it / kStages;
+      // (A wait names its phase by a parity, and a team has every second step, so it has not seen the phase before by itself. Here
+      // that one, step it - 6's products, is over: the team has waited for those of step it - 5, and they end in order. And of the
+      // raw slot below it is step it - 3's, whose products this wait is for.)
+      static_assert(kTeams == 2 && kStages == 3 && kRawStages == kStages, "the phases before a team's waits");
       if (use > 0 && !bar_wait_soon(&sh.empty[stage], (use - 1) & 1u)) {
         sh.fail = 1;
         break;
@@ -239,7 +242,8 @@ __global__ void __launch_bounds__(kThreads, 1) fp4_tc_kernel(const Args a, const
       for (uint32_t it = 0; it < steps; it++) {
         const uint32_t rs = it % kRawStages, use = it / kRawStages;
         if (use > 0 && !bar_wait(&sh.raw_empty[rs], (use - 1) & 1u)) {
-          sh.fail = 1;
+          sh.fail = 1;  // (the copies in flight land before the block's shared memory is another's)
+          for (uint32_t i = it - kRawStages; i < it; i++) bar_wait(&sh.raw_full[i % kRawStages], (i / kRawStages) & 1u);
           break;
         }
         const uint32_t bar = smem_addr(&sh.raw_full[rs]);
@@ -257,7 +261,8 @@ __global__ void __launch_bounds__(kThreads, 1) fp4_tc_kernel(const Args a, const
       for (uint32_t it = 0; it < steps; it++) {
         const uint32_t stage = it % kStages, use = it / kStages;
         if (use > 0 && !bar_wait(&sh.empty[stage], (use - 1) & 1u)) {
-          sh.fail = 1;
+          sh.fail = 1;  // (as above; a stage that the producers have left never fills, and the wait is the time its copy has)
+          for (uint32_t i = it - kStages; i < it; i++) bar_wait(&sh.full[i % kStages], (i / kStages) & 1u);
           break;
         }
         const uint32_t bar = smem_addr(&sh.full[stage]);
@@ -278,7 +283,9 @@ __global__ void __launch_bounds__(kThreads, 1) fp4_tc_kernel(const Args a, const
     for (uint32_t it = 0; it < steps; it++) {
       const uint32_t stage = it % kStages, use = it / kStages;
       if (!bar_wait_soon(&sh.full[stage], use & 1u)) {
-        sh.fail = 1;
+        sh.fail = 1;  // (what has been issued ends before tensor memory is released)
+        mma_commit(issuer, &sh.drain);
+        bar_wait_warp(&sh.drain, 0);
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -331,7 +338,7 @@ __global__ void __launch_bounds__(kThreads, 1) fp4_tc_kernel(const Args a, const
   }
   // ================= epilogue =================
   // Every warp, once its own role is done: a warp reads the tensor-memory lanes of its quarter (its index mod 4: the hardware's
-  // rule), so the three or four warps of a quarter share its rows' 32-token chunks.
+  // rule), so the four or five warps of a quarter share its rows' 32-token chunks.
   __syncwarp();
   {
     const uint32_t quarter = warp % 4u, part = warp / 4u, parts = ((uint32_t) (kThreads / kWarp) - quarter + 3u) / 4u;
