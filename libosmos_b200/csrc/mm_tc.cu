@@ -1093,8 +1093,9 @@ bool launch(Args a, uint32_t n_mat, uint32_t max_cnt, cudaStream_t s) {
   // tokens a tile: the split with the least estimated time - rounds of tiles over the SMs times a K step's cycles, which are
   // the decoders' or the products' (2 a token, and reading their operands), whichever is more
   uint64_t best = 0;
-  constexpr uint32_t kMost = EPI == kGatedMean ? 192u : kMaxSpan;  // (two slots of the token ring)
-  for (uint32_t cols = parts_of(a.n, kMost); cols <= parts_of(a.n, MM_TILE); cols++) {
+  // (of the gated mean too, although its ring has three slots of 256 tokens, not four: up to 192 a tile Q8_0 4 x 2560 x 512, 200 tokens,
+  // took 74.7 us and 2 x 4096 x 2048, 500 tokens, 138.4, against 67.8 and 128.3; 4 x 7168 x 1536 at 2048 2117 and 2124)
+  for (uint32_t cols = parts_of(a.n, kMaxSpan); cols <= parts_of(a.n, MM_TILE); cols++) {
     const uint32_t tok = whole16(parts_of(a.n, cols)), step = 60u + 9u * tok / 4u;
     const uint64_t rounds = (row_tiles * parts_of(a.n, tok) + (uint32_t) sms - 1u) / (uint32_t) sms;
     const uint64_t cost = rounds * (step > 320u ? step : 320u);

@@ -11,6 +11,7 @@ from helpers import ptr, same_bits, sync, to_dev
 from libosmos_b200 import synth
 from oracle.oracle import TYPES
 from test_gpu_mm import _exact, _f16_weights, _one_hot_product, _within, _x16
+from test_gpu_mm import test_mm_run_gated_mean as _gated_mean
 
 pytestmark = pytest.mark.gpu
 
@@ -318,3 +319,9 @@ def test_other_types_decoded(lib, dev, oracle, name, blocks, off):
     pool[off:off + w.size] = w
     got = _one_hot_product(lib, dev, tid, ptr(to_dev(pool, dev)) + off, rows, cols)
     assert np.array_equal(got[~infinite], want[~infinite])
+
+
+@pytest.mark.parametrize("hc,dim,counts", [(2, 4096, (500, 512, 1000)), (4, 2560, (200, 250, 256, 257))])
+def test_gated_mean_of_large_tiles(lib, dev, oracle, hc, dim, counts):
+    """the gated mean over row tiles enough that a tile takes up to 256 tokens: three slots of its token ring, both accumulators"""
+    _gated_mean(lib, dev, oracle, hc, dim, 384, counts)
