@@ -83,6 +83,9 @@ __device__ __forceinline__ uint64_t tile_desc_sw64(uint32_t addr) {
 // instruction descriptor: D F32, A and B f16, both K-major, M = 128, N = n
 __device__ __forceinline__ uint32_t idesc(uint32_t n) { return (1u << 4) | (n >> 3) << 17 | (uint32_t) (kM >> 4) << 24; }
 
+__device__ __forceinline__ void bar_arrive_n(uint64_t* bar, uint32_t n) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(n) : "memory");
+}
 __device__ __forceinline__ void arrive_when_copied(uint64_t* bar) {
   asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_addr(bar)) : "memory");
 }
@@ -90,7 +93,7 @@ __device__ __forceinline__ void arrive_when_copied(uint64_t* bar) {
 // ---- the rows' raw bytes in shared memory ---------------------------------------------------------------------------
 // This many values of K at a time (a whole number of blocks), in slots of an odd number of 16-byte pieces a row: the 16-byte
 // reads of a warp - 32 rows - then take no more passes than their bytes need.
-template <uint32_t T> constexpr uint32_t kRawK = (T == QTYPE_Q8_0 || T == QTYPE_MXFP8) ? 128u : 256u;
+template <uint32_t T> constexpr uint32_t kRawK = (T == QTYPE_Q8_0 || T == QTYPE_MXFP8 || T == QTYPE_Q5_1) ? 128u : 256u;
 template <uint32_t T> constexpr uint32_t kRawBytes = kRawK<T> / Fmt<T>::values * Fmt<T>::bytes;
 template <uint32_t T> constexpr uint32_t kRawSlot = ((kRawBytes<T> + 30u + 15u) & ~15u) | 16u;
 // a matrix whose rows all start on 16 bytes comes by tensor-map copies: a window of each row that starts on 16 bytes and holds the
@@ -536,21 +539,33 @@ struct Shared {
 __host__ __device__ constexpr uint32_t whole16(uint32_t n) { return (n + 15u) & ~15u; }
 __host__ __device__ constexpr uint32_t parts_of(uint32_t n, uint32_t of) { return (n + of - 1u) / of; }
 
-// The steps a producer team walks of a tile of `steps`: those of its whole raw blocks. A row of an odd multiple of 128 values
-// ends in half a block of 256, which has a step for two of the four teams; the other two wait for it and hand it back all the
-// same. A wait on a raw slot names its phase by a parity, and so holds only for a team that has seen the phase before: a team
-// that left a block out could, three slots deep, take the phase before it for its own and decode bytes that had not landed.
-__host__ __device__ constexpr uint32_t walked(uint32_t steps, uint32_t steps_raw) { return parts_of(steps, steps_raw) * steps_raw; }
-// whether each team meets every phase, from the first, of every slot it uses: over rows of all lengths mod a block and enough tiles
-constexpr bool every_phase_seen(uint32_t slots, uint32_t steps_raw) {
-  for (uint32_t steps = 2; steps <= 4 * steps_raw; steps += 2) {
+// A wait on a raw slot names its phase by a parity, so it is right only where the phase before is known to be over. A producer team
+// sees every phase of its slots but where a row of an odd multiple of 128 values ends in half a block of 256: that block has a step
+// for two of the four teams, and the other two go past it. Whether, wherever a team waits for block b, block b - slots has landed by what
+// the team has waited for before: that block itself; or block b' of its own, for which the loader had seen b' - slots and those before used up; or
+// the products of step s - 8, s its last step (they end in order, and each step's block had landed). Rows of 2 .. 40 steps, `whole`
+// at a time, tiles enough to repeat. (Three slots of 256 values do not hold - a team could take the phase before for its own and
+// decode bytes that had not landed - so Q5_1, whose 256 values leave room for three, has blocks of 128.)
+constexpr bool phases_known(uint32_t slots, uint32_t steps_raw, uint32_t whole) {
+  for (uint32_t steps = whole; steps <= 40; steps += whole) {
+    const uint32_t blocks = parts_of(steps, steps_raw);
     for (uint32_t team = 0; team < (uint32_t) kTeams; team++) {
-      uint32_t next[8] = {}, s0 = 0, rb0 = 0;  // next[slot]: the phase to be met next
-      for (uint32_t tile = 0; tile < 4 * slots; tile++, s0 += steps, rb0 += parts_of(steps, steps_raw)) {
-        for (uint32_t it = (team - s0) % (uint32_t) kTeams; it < walked(steps, steps_raw); it += (uint32_t) kTeams) {
-          const uint32_t rb = rb0 + it / steps_raw, slot = rb % slots, phase = rb / slots;
-          if (phase != next[slot]) return false;
-          next[slot] = phase + 1;
+      uint32_t own[64] = {}, n = 0, most = 0, last = 0;  // its blocks so far, less 1 the greatest; its last step
+      for (uint32_t tile = 0; tile * blocks < 12 * slots; tile++) {
+        const uint32_t s0 = tile * steps;
+        for (uint32_t it = (team - s0) % (uint32_t) kTeams; it < steps; it += (uint32_t) kTeams) {
+          const uint32_t b = tile * blocks + it / steps_raw;
+          if (b >= slots) {
+            const uint32_t before = b - slots;
+            bool known = most > slots && before <= most - 1 - slots;
+            for (uint32_t i = 0; i < n && i < 64; i++) known = known || own[i] == before + 1;
+            if (last >= kSteps) {
+              const uint32_t s = last - kSteps;
+              known = known || before <= s / steps * blocks + s % steps / steps_raw;
+            }
+            if (!known) return false;
+          }
+          own[n++ % 64] = b + 1, most = b + 1, last = s0 + it;
         }
       }
     }
@@ -678,17 +693,12 @@ __global__ void __launch_bounds__(kThreads, 1) mm_tc_kernel(const Args a, const 
         row = min(tl.rt * kM + r, rows - 1u);
       }
       const uint32_t base15 = (uint32_t) ((uintptr_t) (w + (uint64_t) row * row_bytes) & 15u);
-      for (uint32_t it = (team - s0) % kTeams; it < walked(steps, kStepsRaw); it += kTeams) {
+      for (uint32_t it = (team - s0) % kTeams; it < steps; it += kTeams) {
         const uint32_t s = s0 + it, stage = s % kSteps, unit = stage >> two, kb = it / kStepsRaw, sub = it % kStepsRaw, rb = rb0 + kb, slot = rb % kRawStages<T>;
-        const bool past = it >= steps;  // (no step of the row's: the block is waited for and handed back)
-        if (!bar_wait_soon(&sh.full_raw[slot], (rb / kRawStages<T>) & 1u) ||
-            (!past && s >= kSteps && !bar_wait_soon(&sh.empty[unit], (s / kSteps - 1u) & 1u))) {
+        if (!bar_wait_soon(&sh.full_raw[slot], (rb / kRawStages<T>) & 1u) ||  // (its parity: phases_known)
+            (s >= kSteps && !bar_wait_soon(&sh.empty[unit], (s / kSteps - 1u) & 1u))) {
           ok = false;
           break;
-        }
-        if (past) {
-          if (lane == 0) bar_arrive(&sh.empty_raw[slot]);
-          break;  // (the tile's last block)
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t off = slot * (kM * kSlot) + r * pitch + ((base15 + kb * kRawBytes<T>) & 15u);
@@ -703,7 +713,8 @@ __global__ void __launch_bounds__(kThreads, 1) mm_tc_kernel(const Args a, const 
         __syncwarp();
         if (lane == 0) {
           bar_arrive(&sh.full_a[unit]);
-          bar_arrive(&sh.empty_raw[slot]);
+          // (the raw block's last step arrives for those a row's end leaves out)
+          bar_arrive_n(&sh.empty_raw[slot], it == steps - 1u ? kStepsRaw - sub : 1u);
         }
       }
     }
@@ -1055,7 +1066,7 @@ template <uint32_t T, uint32_t EPI = kStore>
 bool launch(Args a, uint32_t n_mat, uint32_t max_cnt, cudaStream_t s) {
   constexpr int kBytes = (int) kSmem<T, EPI>;
   static_assert(kBytes + grid_smem_bytes<T>() + (int) sizeof(Shared) + 64 <= 227 * 1024, "a block's shared memory");
-  static_assert(every_phase_seen(kRawStages<T>, kRawK<T> / kStep), "a producer's wait on a raw slot");
+  static_assert(phases_known(kRawStages<T>, kRawK<T> / kStep, Fmt<T>::values > 128 ? Fmt<T>::values / kStep : 2), "a producer's wait on a raw slot");
   a.status = status_word();
   if (!a.status) return false;
   int sms = 0, dev = 0;
