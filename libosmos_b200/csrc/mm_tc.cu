@@ -641,6 +641,11 @@ __global__ void __launch_bounds__(kThreads, 1) mm_tc_kernel(const Args a, const 
   {
     const uint32_t n = tid < n_mat ? (a.wt ? (uint32_t) max(a.cnt[tid], 0) : a.n) : 0u, cols = parts_of(n, a.span);
     const uint32_t mine = cols * (a.row_tiles + a.row_tiles1), most = __reduce_max_sync(0xFFFFFFFFu, n ? whole16(parts_of(n, cols)) : 0u);
+    // (the pointers are the device's: one that is no matrix of the tensor comes through the map as another's rows, or as zeros)
+    if (n && a.wt && a.raw_map) {
+      const uint64_t at = (uint64_t) (a.wt[tid] - a.base), index = at / a.bytes;
+      if (index >= a.n_base || index * a.bytes != at) atomicOr(a.status, kNotOfTensor);
+    }
     uint32_t sum = mine;
 #pragma unroll
     for (int o = 1; o < kWarp; o <<= 1) {
@@ -740,13 +745,7 @@ __global__ void __launch_bounds__(kThreads, 1) mm_tc_kernel(const Args a, const 
     if (a.raw_map) {  // a copy a block: the second warp has nothing to do
       for (uint32_t t = blockIdx.x; t < tiles && ok && warp == (uint32_t) kFirstRaw; t += gridDim.x) {
         const Tile tl = tile_at(a, first, t, m_at, lane);
-        uint32_t mat = 0;
-        if (a.wt) {
-          // (the pointers are the device's: one that is no matrix of the tensor would be another's rows, or rows of zeros)
-          const uint64_t at = (uint64_t) (a.wt[tl.m] - a.base), index = at / a.bytes;
-          if (index < a.n_base && index * a.bytes == at) mat = (uint32_t) index;
-          else if (lane == 0) atomicOr(a.status, kNotOfTensor);
-        }
+        const uint32_t mat = a.wt ? (uint32_t) ((uint64_t) (a.wt[tl.m] - a.base) / a.bytes) : 0u;
         for (uint32_t kb = 0; kb < kblocks; kb++, rb++) {
           const uint32_t slot = rb % kRawStages<T>;
           if (rb >= kRawStages<T> && !bar_wait_soon(&sh.empty_raw[slot], (rb / kRawStages<T> - 1u) & 1u)) {
