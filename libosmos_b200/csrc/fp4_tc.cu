@@ -23,9 +23,10 @@
 //                        onto the accumulator's barrier after the last. The whole warp runs this, one elected lane issues.
 //   epilogue (all warps, their roles done) thread = one weight row (its TMEM lane): tcgen05.ld the sums, times the tensors'
 //                        scale, stored.
-// 17408 x 5120, 2048 tokens, with the tokens' quantization: 183 -> 164 us with the teams, the elected issuer, the shorter
-// repacking and the shared epilogue. What is left: a stage brings 54 KB to the SM in about 1,100 cycles (over 11 TB/s in all),
-// the tensor pipe needs 700 of them; 3,000 cycles of a tile's 34,000 are its start, 4,300 its stores.
+// 17408 x 5120, 2048 tokens, with the teams, the elected issuer, the shorter repacking and the shared epilogue: a graph of launches
+// over four weight copies 160 -> 143 us the product alone, 180 -> 163 with the tokens' quantization (as two calls a pass 196 -> 184).
+// What is left: a stage brings 54 KB to the SM in about 1,100 cycles (over 11 TB/s in all), the tensor pipe needs 700 of them; 3,000
+// cycles of a tile's 34,000 are its start, 4,300 its stores.
 // The descriptors follow the layouts CUTLASS documents in cute/arch/mma_sm100_desc.hpp (InstrDescriptorBlockScaled),
 // cute/atom/mma_traits_sm100.hpp (the scale factors' tensor-memory fragment) and cutlass/detail/sm100_blockscaled_layout.hpp
 // (the chunk layout); tests/test_fp4_desc.py holds the instruction descriptor to CUTLASS's own encoder.

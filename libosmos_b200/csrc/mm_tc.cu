@@ -28,11 +28,11 @@
 //                        tensor-map copy where rows start on 16 bytes, else 16-byte cp.async pieces
 //   token loader (1 warp) the tokens' x16, a K step a tensor-map copy; grouped tokens that start inside a tile of x16 by 16-byte
 //                        cp.async pieces
-// Bound by the decoders' integer and F32 pipes up to about 128 tokens a tile (a 64-value step of 128 rows is some 330 instructions
-// a thread, 300 to 400 cycles; its products are 128 cycles at 64 tokens), past that by the tokens' copies, 32 KB a step at 256 tokens
-// where the products take 512 cycles. Measured, against decoded tiles in shared memory, a tile a block (with the tokens' rounding):
-// Q4_K 4096 x 4096 at 777 / 2048 tokens 62.8 / 106 us -> 40.7 / 71; 128 MXFP4 experts of 1536 x 4096 over 2048 tokens, the
-// layer, 1827 -> 769.
+// Bound by the decoders' integer and F32 pipes up to about 128 tokens a tile (a 64-value step of 128 Q4_K rows is 1,460 warp
+// instructions, all roles together, of IQ3_XXS 2,260, at two thirds of the issue slots; its products are 128 cycles at 64 tokens), past
+// that by the tokens' copies, 32 KB a step at 256 tokens where the products take 512 cycles (the tensor pipe is active 64 %). Measured,
+// against decoded tiles in shared memory, a tile a block (with the tokens' rounding, passes of mm_tokens): Q4_K 4096 x 4096 at 777 /
+// 2048 tokens 62.8 / 106 us -> 40.7 / 71; 128 MXFP4 experts of 1536 x 4096 over 2048 tokens, the layer, 1827 -> 769.
 // Every mbarrier wait is bounded (%globaltimer) with one outcome a warp; a wait that runs out raises the status word, every
 // role falls through to the common exit and tensor memory is released.
 #include <cuda.h>
@@ -631,8 +631,8 @@ __global__ void __launch_bounds__(kThreads, 1) mm_tc_kernel(const Args a, const 
   }
   // (a dependent launch: the counts, x16 and the readers of y may be the kernel ahead's. Where that kernel is this call's own
   // conversion - launched the ordinary way, so that whatever wrote the weights is over - the weights' loads and their
-  // decoding need not wait for it, only the tokens' loads and the stores. Q4_K 4096 x 4096, 777 tokens: 37.1 -> 34.5 us; MXFP4
-  // 2560 x 1536, 126 tokens: 16.4 -> 14.4.)
+  // decoding need not wait for it, only the tokens' loads and the stores. Passes of mm_tokens back to back, Q4_K 4096 x 2048 at
+  // 2048 tokens: 41.4 -> 39.9 us; MXFP4 2560 x 1536, 126 tokens: 13.8 -> 12.7; elsewhere 0 to 4 %.)
   if (!a.early) pdl_wait();
   pdl_launch_next();
   // the matrices' first tiles, a thread each, and the most tokens a tile has
