@@ -24,7 +24,7 @@
 //                        first of a tile overwrite, the rest accumulate), then tcgen05.commit onto the unit's "empty" mbarrier; after
 //                        a tile's last step a commit onto its accumulators' "full" ones. The whole warp runs this, one elected
 //                        lane issues.
-//   raw loaders (2 warps) the rows' bytes, 256 values of K at a time (128 of the widest types), a ring of three or four: one
+//   raw loaders (2 warps) the rows' bytes, 256 values of K at a time (128 of Q8_0, MXFP8 and Q5_1), a ring of three or four: one
 //                        tensor-map copy where rows start on 16 bytes, else 16-byte cp.async pieces
 //   token loader (1 warp) the tokens' x16, a K step a tensor-map copy; grouped tokens that start inside a tile of x16 by 16-byte
 //                        cp.async pieces
